@@ -11,6 +11,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <initializer_list>
 #include <memory>
 #include <vector>
 
@@ -232,6 +233,111 @@ __global__ void __launch_bounds__(256, K >= 10 ? 5 : 6) spmv_kernel(const long l
     }
 }
 
+// Short rows (fewer than ten entries on average): a CTA takes 256 consecutive
+// rows at a time, streams their entries as 16-byte loads (whatever row they
+// belong to), multiplies each by its x into shared memory, and then every
+// thread adds up its own row there. Four gathers per load are
+// in flight and no lane idles over a row's end, where a group of lanes per row
+// spends most of its instructions on predicates and waits for the row pointers,
+// the columns and the gathers one after another for 28 bytes of values. A tile
+// with more entries than fit in shared memory is summed a warp per row.
+// 7 entries per row on a 256^3 grid, 72 bytes per row: 600 us a product with
+// four lanes per row, 250 us so (a copy of the bytes takes 178).
+constexpr int SR_ROWS = 256;
+constexpr int SR_CAP = 2816;  // entries of a tile (11 per row): 11 KB, eight CTAs per SM
+__global__ void __launch_bounds__(SR_ROWS, 8) spmv_rows_kernel(const long long* __restrict__ rp, const int* __restrict__ col,
+                                                              const float* __restrict__ val,
+                                                              const float* __restrict__ x, float* __restrict__ y,
+                                                              long long rows, long long nnz,
+                                                              const float* __restrict__ add, float add_scale,
+                                                              const float* __restrict__ pdot,
+                                                              double* __restrict__ dot_acc,
+                                                              const int* __restrict__ done) {
+    if (done && *done) return;
+    __shared__ __align__(16) float prod[SR_CAP + 8];
+    __shared__ double red[8];
+    const int tid = threadIdx.x;
+    double local = 0.0;
+    for (long long r0 = (long long)blockIdx.x * SR_ROWS; r0 < rows; r0 += (long long)gridDim.x * SR_ROWS) {
+        const long long row = r0 + tid;
+        const bool active = row < rows;
+        const long long rlast = min(r0 + SR_ROWS, rows);
+        const long long e0 = rp[r0], e1 = rp[rlast];
+        const long long base = e0 & ~3ll;  // 16-byte aligned start of the tile's entries
+        const long long a = active ? rp[row] : 0, b = active ? rp[row + 1] : 0;
+        float sum = 0.0f;
+        if (e1 - base <= SR_CAP) {
+            for (long long e = base + 4 * tid; e < e1; e += 4 * SR_ROWS) {
+                float4 o = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (e >= e0 && e + 4 <= e1) {
+                    const int4 c = __ldg(reinterpret_cast<const int4*>(col + e));
+                    const float4 v = __ldg(reinterpret_cast<const float4*>(val + e));
+                    o = make_float4(v.x * __ldg(x + c.x), v.y * __ldg(x + c.y), v.z * __ldg(x + c.z),
+                                    v.w * __ldg(x + c.w));
+                } else {
+                    float* of = &o.x;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        if (e + k >= e0 && e + k < e1) of[k] = __ldg(val + e + k) * __ldg(x + __ldg(col + e + k));
+                }
+                *reinterpret_cast<float4*>(prod + (e - base)) = o;
+            }
+            __syncthreads();
+            // four strided partial sums, as four lanes per row would hold
+            float t0 = 0.0f, t1 = 0.0f, t2 = 0.0f, t3 = 0.0f;
+            const int kb = (int)(b - base);
+            int k = (int)(a - base);
+            for (; k + 4 <= kb; k += 4) {
+                t0 += prod[k];
+                t1 += prod[k + 1];
+                t2 += prod[k + 2];
+                t3 += prod[k + 3];
+            }
+            if (k < kb) t0 += prod[k];
+            if (k + 1 < kb) t1 += prod[k + 1];
+            if (k + 2 < kb) t2 += prod[k + 2];
+            sum = (t0 + t2) + (t1 + t3);
+            __syncthreads();
+        } else {
+            const int lane = tid & 31;
+            for (int w = 0; w < 32; ++w) {  // the warp's 32 rows, one after another
+                const long long ra = __shfl_sync(FULL, a, w), rb = __shfl_sync(FULL, b, w);
+                float s = 0.0f;
+                for (long long e = ra + lane; e < rb; e += 32) s = fmaf(__ldg(val + e), __ldg(x + __ldg(col + e)), s);
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(FULL, s, o);
+                if (lane == w) sum = s;
+            }
+        }
+        if (active) {
+            if (add) sum = fmaf(add_scale, add[row], sum);
+            y[row] = sum;
+            if (pdot) local += (double)pdot[row] * (double)sum;
+        }
+    }
+    if (dot_acc) {
+        for (int o = 16; o > 0; o >>= 1) local += __shfl_xor_sync(FULL, local, o);
+        if ((tid & 31) == 0) red[tid >> 5] = local;
+        __syncthreads();
+        if (tid == 0) {
+            double t = 0.0;
+            for (int w = 0; w < SR_ROWS / 32; ++w) t += red[w];
+            atomicAdd(dot_acc + blockIdx.x % CG_SLOTS, t);
+        }
+    }
+}
+
+int launch_spmv_rows(const DevCsr& A, const float* x, float* y, const float* add, float add_scale, const float* pdot,
+                     double* dot_acc, const int* done, cudaStream_t st) {
+    const long long tiles = (A.rows + SR_ROWS - 1) / SR_ROWS;
+    const unsigned blocks = (unsigned)std::max<long long>(1, std::min<long long>(tiles, grid_cap() / 2));  // 8 per SM
+    spmv_rows_kernel<<<blocks, SR_ROWS, 0, st>>>(A.row_ptr, A.col, A.val, x, y, A.rows, A.nnz, add, add_scale, pdot,
+                                                 dot_acc, done);
+    count_launch();
+    ST_CUDA(cudaGetLastError());
+    return ST_OK;
+}
+
 template <int G, int K, bool PF>
 int launch_spmv_g(const DevCsr& A, const float* x, float* y, const float* add, float add_scale, const float* pdot,
                   double* dot_acc, const int* done, cudaStream_t st) {
@@ -298,13 +404,24 @@ __global__ void cg_init_kernel(const float* __restrict__ b, const float* __restr
     block_add2(a, c, rz, bb, CG_SLOTS);
 }
 
+// Whether every given pointer (null ones aside) may be read as 16-byte quads.
+inline bool quads_ok(std::initializer_list<const void*> ps) {
+    for (const void* p : ps)
+        if (reinterpret_cast<uintptr_t>(p) & 15) return false;
+    return true;
+}
+
 // x += alpha p, r -= alpha q, z = M r; acc rz_new = <r,z>, rr = <r,r>.
+// Bound by memory (8 words per unknown) beside the FP64 sums: read and written
+// four unknowns at a time where the caller's x allows it (quads), so that a
+// thread has five 16-byte loads in flight (one word at a time: 169 us at 16.8M
+// unknowns, 3.2 TB/s).
 // alpha = rz_old / pq; |pq| < 1e-30 stops the solve (sparse_ops.cpp:37,88).
 // The scalars are formed once per block (FP64 is a slow pipe on this GPU).
 // skip_rz: <r, z> comes from the stencil preconditioner's kernel instead.
 __global__ void cg_update_kernel(long long n, float* __restrict__ x, float* __restrict__ r, float* __restrict__ z,
                                  const float* __restrict__ p, const float* __restrict__ q,
-                                 const float* __restrict__ dinv, CgScalars* sc, int k, int skip_rz) {
+                                 const float* __restrict__ dinv, CgScalars* sc, int k, int skip_rz, int quads) {
     __shared__ float s_alpha;
     __shared__ int s_stop;
     if (threadIdx.x == 0) {
@@ -329,7 +446,31 @@ __global__ void cg_update_kernel(long long n, float* __restrict__ x, float* __re
     if (s_stop) return;
     const float alpha = s_alpha;
     double a = 0.0, c = 0.0;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    const long long n4 = quads ? n >> 2 : 0;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
+        const float4 p4 = reinterpret_cast<const float4*>(p)[i], q4 = reinterpret_cast<const float4*>(q)[i];
+        float4 x4 = reinterpret_cast<float4*>(x)[i], r4 = reinterpret_cast<float4*>(r)[i];
+        float4 d4 = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+        if (dinv) d4 = reinterpret_cast<const float4*>(dinv)[i];
+        x4 = make_float4(fmaf(alpha, p4.x, x4.x), fmaf(alpha, p4.y, x4.y), fmaf(alpha, p4.z, x4.z), fmaf(alpha, p4.w, x4.w));
+        r4 = make_float4(fmaf(-alpha, q4.x, r4.x), fmaf(-alpha, q4.y, r4.y), fmaf(-alpha, q4.z, r4.z),
+                         fmaf(-alpha, q4.w, r4.w));
+        const float4 z4 = make_float4(d4.x * r4.x, d4.y * r4.y, d4.z * r4.z, d4.w * r4.w);
+        reinterpret_cast<float4*>(x)[i] = x4;
+        reinterpret_cast<float4*>(r)[i] = r4;
+        if (z) reinterpret_cast<float4*>(z)[i] = z4;
+        const double r0 = r4.x, r1 = r4.y, r2 = r4.z, r3 = r4.w;
+        a += r0 * (double)z4.x;
+        a += r1 * (double)z4.y;
+        a += r2 * (double)z4.z;
+        a += r3 * (double)z4.w;
+        c += r0 * r0;
+        c += r1 * r1;
+        c += r2 * r2;
+        c += r3 * r3;
+    }
+    for (long long i = 4 * n4 + blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
+         i += (long long)gridDim.x * blockDim.x) {
         x[i] = fmaf(alpha, p[i], x[i]);
         const float ri = fmaf(-alpha, q[i], r[i]);
         r[i] = ri;
@@ -400,8 +541,15 @@ __global__ void cg_pupdate_kernel(long long n, float* __restrict__ p, const floa
     __syncthreads();
     if (s_stop) return;
     const float beta = s_beta;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        p[i] = fmaf(beta, p[i], z[i]);
+    const long long n4 = n >> 2;  // p, z and r are the solver's own vectors: 16-byte aligned
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
+        const float4 z4 = reinterpret_cast<const float4*>(z)[i];
+        const float4 p4 = reinterpret_cast<float4*>(p)[i];
+        reinterpret_cast<float4*>(p)[i] = make_float4(fmaf(beta, p4.x, z4.x), fmaf(beta, p4.y, z4.y),
+                                                      fmaf(beta, p4.z, z4.z), fmaf(beta, p4.w, z4.w));
+    }
+    const long long i = 4 * n4 + blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (i < n) p[i] = fmaf(beta, p[i], z[i]);
 }
 
 // Jacobi diagonal of sparse_ops.cpp:60-73: 1/A_ii from the first entry with
@@ -420,12 +568,26 @@ __global__ void jacobi_kernel(const long long* __restrict__ rp, const int* __res
 }
 
 // diag of A^T A + lam I from the rows of A^T: 1 / (sum_k AT[j,k]^2 + lam).
+// G lanes per row (coalesced), the squares exact and their sums in FP64.
+template <int G>
 __global__ void normal_jacobi_kernel(const long long* __restrict__ rp, const float* __restrict__ val, long long rows,
                                      double lam, float* __restrict__ dinv) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < rows; i += (long long)gridDim.x * blockDim.x) {
+    const int lane = threadIdx.x % G;
+    const long long stride = (long long)gridDim.x * blockDim.x / G;
+    const long long first = (blockIdx.x * (long long)blockDim.x + (threadIdx.x & ~31u)) / G;  // of the warp: uniform trips
+    const long long gid = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / G;
+    for (long long it = 0; first + it * stride < rows; ++it) {
+        const long long i = gid + it * stride;
+        const long long a = i < rows ? rp[i] : 0, b = i < rows ? rp[i + 1] : 0;
         double s = 0.0;
-        for (long long p = rp[i]; p < rp[i + 1]; ++p) s += (double)val[p] * (double)val[p];
-        dinv[i] = (float)(1.0 / (s + lam));
+#pragma unroll 4
+        for (long long p = a + lane; p < b; p += G) {
+            const double v = (double)__ldg(val + p);
+            s = fma(v, v, s);
+        }
+#pragma unroll
+        for (int o = G / 2; o > 0; o >>= 1) s += __shfl_xor_sync(FULL, s, o, G);
+        if (lane == 0 && i < rows) dinv[i] = (float)(1.0 / (s + lam));
     }
 }
 
@@ -629,7 +791,7 @@ int build_transpose(const DevCsr& A, DevCsr* T, cudaStream_t st) {
 int launch_spmv(const DevCsr& A, const float* x, float* y, const float* add, float add_scale, const float* pdot,
                 double* dot_acc, const int* done, cudaStream_t st) {
     const double avg = A.rows > 0 ? (double)A.nnz / (double)A.rows : 0.0;
-    // tuning override: SEISMIC_GB300_SPMV_G=<2|4|8|16|32> threads per row
+    // tuning override: SEISMIC_GB300_SPMV_G=<1|8|16|32> threads per row
     static const int forced = [] {
         const char* e = std::getenv("SEISMIC_GB300_SPMV_G");
         return e ? std::atoi(e) : 0;
@@ -638,7 +800,7 @@ int launch_spmv(const DevCsr& A, const float* x, float* y, const float* add, flo
         case 32: return launch_spmv_g<32, 6, false>(A, x, y, add, add_scale, pdot, dot_acc, done, st);
         case 16: return launch_spmv_g<16, 10, true>(A, x, y, add, add_scale, pdot, dot_acc, done, st);
         case 8: return launch_spmv_g<8, 4, true>(A, x, y, add, add_scale, pdot, dot_acc, done, st);
-        case 4: return launch_spmv_g<4, 4, false>(A, x, y, add, add_scale, pdot, dot_acc, done, st);
+        case 1: return launch_spmv_rows(A, x, y, add, add_scale, pdot, dot_acc, done, st);
         default: break;
     }
     // measured on the 2M-ray matrix (180 entries per row) and its transpose (360): 16 threads per
@@ -647,8 +809,7 @@ int launch_spmv(const DevCsr& A, const float* x, float* y, const float* add, flo
     if (avg >= 256) return launch_spmv_g<32, 6, false>(A, x, y, add, add_scale, pdot, dot_acc, done, st);
     if (avg >= 24) return launch_spmv_g<16, 10, true>(A, x, y, add, add_scale, pdot, dot_acc, done, st);
     if (avg >= 10) return launch_spmv_g<8, 4, true>(A, x, y, add, add_scale, pdot, dot_acc, done, st);
-    if (avg >= 5) return launch_spmv_g<4, 4, false>(A, x, y, add, add_scale, pdot, dot_acc, done, st);
-    return launch_spmv_g<2, 4, false>(A, x, y, add, add_scale, pdot, dot_acc, done, st);
+    return launch_spmv_rows(A, x, y, add, add_scale, pdot, dot_acc, done, st);
 }
 
 int launch_f64_to_f32(const double* a, float* b, long long n, cudaStream_t st) {
@@ -670,7 +831,12 @@ int launch_jacobi(const DevCsr& A, float* dinv, cudaStream_t st) {
     return ST_OK;
 }
 int launch_normal_jacobi(const DevCsr& AT, double lam, float* dinv, cudaStream_t st) {
-    normal_jacobi_kernel<<<blocks_for(AT.rows), 256, 0, st>>>(AT.row_ptr, AT.val, AT.rows, lam, dinv);
+    // coalesced, a warp per row (1M rows of 361 entries: 2.2 ms, bound by the FP64 pipe, against 4.19
+    // with a thread per row); 4 lanes where a row would leave most of a warp idle
+    if (AT.nnz >= 24 * AT.rows)
+        normal_jacobi_kernel<32><<<blocks_for(AT.rows * 32), 256, 0, st>>>(AT.row_ptr, AT.val, AT.rows, lam, dinv);
+    else
+        normal_jacobi_kernel<4><<<blocks_for(AT.rows * 4), 256, 0, st>>>(AT.row_ptr, AT.val, AT.rows, lam, dinv);
     count_launch();
     ST_CUDA(cudaGetLastError());
     return ST_OK;
@@ -779,6 +945,7 @@ int cg_loop(const CgProblem& P, CgWork& W, int k0, int max_iter, double tol, int
     const long long n = P.n;
     CgScalars h{};
     const float* zp = P.dinv ? W.z : W.r;
+    const int quads = quads_ok({P.x, W.r, W.z, W.p, W.q, P.dinv});
     int k = k0;
     while (k < max_iter) {
         const int batch = std::min(check_every, max_iter - k);
@@ -790,7 +957,8 @@ int cg_loop(const CgProblem& P, CgWork& W, int k0, int max_iter, double tol, int
                 ST_TRY(launch_spmv(*P.A, W.p, W.q, nullptr, 0.0f, W.p, W.sc->acc[k % 3].pq, &W.sc->done, st));
             }
             cg_update_kernel<<<cg_blocks(n), 256, 0, st>>>(n, P.x, W.r, P.dinv && !P.sq ? W.z : nullptr, W.p,
-                                                             W.q, P.sq ? nullptr : P.dinv, W.sc, k, P.sq != nullptr);
+                                                             W.q, P.sq ? nullptr : P.dinv, W.sc, k, P.sq != nullptr,
+                                                             quads);
             count_launch();
             if (P.sq) {
                 stencil_prec_kernel<<<cg_blocks(n), 256, 0, st>>>(n, W.r, P.dinv, P.sq, P.gx, P.gy, P.gz, P.w[0],
