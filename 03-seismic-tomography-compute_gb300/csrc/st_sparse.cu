@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(256, K >= 10 ? 5 : 6) spmv_kernel(const long l
 // the columns and the gathers one after another for 28 bytes of values. A tile
 // with more entries than fit in shared memory is summed a warp per row.
 // 7 entries per row on a 256^3 grid, 72 bytes per row: 600 us a product with
-// four lanes per row, 250 us so (a copy of the bytes takes 178).
+// four lanes per row, 242 us so (a copy of the bytes takes 178).
 constexpr int SR_ROWS = 256;
 constexpr int SR_CAP = 2816;  // entries of a tile (11 per row): 11 KB, eight CTAs per SM
 __global__ void __launch_bounds__(SR_ROWS, 8) spmv_rows_kernel(const long long* __restrict__ rp, const int* __restrict__ col,
@@ -769,24 +769,6 @@ template int build_csr<long long, double>(long long, long long, long long, const
                                           const double*, bool, DevCsr*, cudaStream_t);
 template int build_csr<int, float>(long long, long long, long long, const int*, const int*, const float*, bool,
                                    DevCsr*, cudaStream_t);
-
-// Transpose: rebuild from (col, row) keys of the existing entries.
-__global__ void expand_rows_kernel(const long long* __restrict__ rp, long long rows, int* __restrict__ rowidx) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < rows; i += (long long)gridDim.x * blockDim.x)
-        for (long long p = rp[i]; p < rp[i + 1]; ++p) rowidx[p] = (int)i;
-}
-
-int build_transpose(const DevCsr& A, DevCsr* T, cudaStream_t st) {
-    ST_CHECK(A.rows < (1ll << 31), ST_ERR_ARG, "rows must fit int32 to transpose");
-    int* rowidx = nullptr;
-    ST_CUDA(cudaMalloc(&rowidx, (size_t)std::max<long long>(A.nnz, 1) * sizeof(int)));
-    expand_rows_kernel<<<blocks_for(A.rows), 256, 0, st>>>(A.row_ptr, A.rows, rowidx);
-    count_launch();
-    ST_CUDA(cudaGetLastError());
-    int rc = build_csr<int, float>(A.cols, A.rows, A.nnz, A.col, rowidx, A.val, false, T, st);
-    cudaFree(rowidx);
-    return rc;
-}
 
 int launch_spmv(const DevCsr& A, const float* x, float* y, const float* add, float add_scale, const float* pdot,
                 double* dot_acc, const int* done, cudaStream_t st) {
