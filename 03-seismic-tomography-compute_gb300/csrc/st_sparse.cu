@@ -152,17 +152,46 @@ __global__ void pad_scatter_kernel(const long long* __restrict__ rp, const int* 
 
 __global__ void fill_last_kernel(long long* rp, long long R, const long long* total) { rp[R] = *total; }
 
+// A sum of a few products held as an unevaluated pair of FP32 values (Dot2 of
+// Ogita, Rump and Oishi, "Accurate sum and dot product", 2005): the products are
+// split exactly by FMA and the rounding error of every addition is kept, so eight
+// products lose at most (8 * 2^-24)^2 of their magnitude, typically 2^-49. The FP64
+// pipe takes a warp's operation in 16 cycles here (conversions too), the
+// FP32 one in a quarter of a cycle: a kernel adds up to eight products so and
+// then folds the pair into its FP64 sum. Only for factors that pair_safe admits:
+// zero or 2^-50 .. 2^60, so that no product or error term over- or underflows; the
+// callers take FP64 products otherwise (tiny gradients, infinities, NaN).
+__device__ __forceinline__ bool pair_safe(float a) {
+    const unsigned m = __float_as_uint(a) & 0x7fffffffu;
+    return (m - 0x26800000u <= 0x5d800000u - 0x26800000u) | (m == 0u);
+}
+struct PairSum {
+    float h = 0.0f, l = 0.0f;
+    __device__ __forceinline__ void add(float a, float b) {
+        const float p = __fmul_rn(a, b);
+        const float e = __fmaf_rn(a, b, -p);
+        const float t = __fadd_rn(h, p);
+        const float z = __fsub_rn(t, h);
+        const float err = __fadd_rn(__fsub_rn(h, __fsub_rn(t, z)), __fsub_rn(p, z));
+        h = t;
+        l = __fadd_rn(l, __fadd_rn(e, err));
+    }
+    __device__ __forceinline__ double value() const { return (double)h + (double)l; }
+};
+
 // ---------------------------------------------------------------- SpMV
 // y[row] = sum val*x[col] with G threads per row (FP32 accumulation, a
 // G-way strided partial sum per row reduced by shuffles), optional
 // y += add_scale * add and FP64 accumulation of dot(pdot, y).
-// Each lane first loads the column and value of up to K of its row's entries
-// (coalesced), then issues all K gathers of x before it sums: the gathers,
-// which wait on L2, are all in flight at once (the rest of a longer row
-// follows in a loop). PF: the group pulls the columns and values of the row
+// Each lane loads the column and value of up to K of its row's entries at a
+// time (coalesced), then issues all K gathers of x before it sums: the gathers,
+// which wait on L2, are all in flight at once. The rest of a longer row follows
+// in more such turns (TURNS: rows of 256 entries and more on average, some of
+// thousands) or one entry at a time (shorter rows: a second turn, mostly empty,
+// measured 0.655 ms against 0.561 with 16 lanes on rows of 180). PF: the group pulls the columns and values of the row
 // it takes two rows on into L2. Resident CTAs per SM are pinned (six at 40
 // registers, five at 48 for the 10-entry variant): the gathers need the warps.
-template <int G, int K, bool PF>
+template <int G, int K, bool PF, bool TURNS>
 __global__ void __launch_bounds__(256, K >= 10 ? 5 : 6) spmv_kernel(const long long* __restrict__ rp, const int* __restrict__ col,
                                                    const float* __restrict__ val, const float* __restrict__ x,
                                                    float* __restrict__ y, long long rows, const float* __restrict__ add,
@@ -192,23 +221,31 @@ __global__ void __launch_bounds__(256, K >= 10 ? 5 : 6) spmv_kernel(const long l
                 asm volatile("prefetch.global.L2 [%0];" ::"l"(val + e));
             }
         }
-        int cs[K];
-        float vs[K], xs[K];
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-            const long long e = a + lane + (long long)k * G;
-            cs[k] = e < b ? __ldg(col + e) : 0;
-            vs[k] = e < b ? __ldg(val + e) : 0.0f;
-        }
-#pragma unroll
-        for (int k = 0; k < K; ++k) xs[k] = (a + lane + (long long)k * G < b) ? __ldg(x + cs[k]) : 0.0f;
         float s0 = 0.0f, s1 = 0.0f;
+        auto turn = [&](long long q) {
+            int cs[K];
+            float vs[K], xs[K];
 #pragma unroll
-        for (int k = 0; k < K; k += 2) {
-            s0 = fmaf(vs[k], xs[k], s0);
-            if (k + 1 < K) s1 = fmaf(vs[k + 1], xs[k + 1], s1);
+            for (int k = 0; k < K; ++k) {
+                const long long e = q + lane + (long long)k * G;
+                cs[k] = e < b ? __ldg(col + e) : 0;
+                vs[k] = e < b ? __ldg(val + e) : 0.0f;
+            }
+#pragma unroll
+            for (int k = 0; k < K; ++k) xs[k] = (q + lane + (long long)k * G < b) ? __ldg(x + cs[k]) : 0.0f;
+#pragma unroll
+            for (int k = 0; k < K; k += 2) {
+                s0 = fmaf(vs[k], xs[k], s0);
+                if (k + 1 < K) s1 = fmaf(vs[k + 1], xs[k + 1], s1);
+            }
+        };
+        if (TURNS) {
+            for (long long q = a; q < b; q += (long long)K * G) turn(q);
+        } else {
+            turn(a);
+            for (long long p = a + lane + (long long)K * G; p < b; p += G)
+                s0 = fmaf(__ldg(val + p), __ldg(x + __ldg(col + p)), s0);
         }
-        for (long long p = a + lane + (long long)K * G; p < b; p += G) s0 = fmaf(__ldg(val + p), __ldg(x + __ldg(col + p)), s0);
         float sum = s0 + s1;
 #pragma unroll
         for (int o = G / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(FULL, sum, o, G);
@@ -338,14 +375,14 @@ int launch_spmv_rows(const DevCsr& A, const float* x, float* y, const float* add
     return ST_OK;
 }
 
-template <int G, int K, bool PF>
+template <int G, int K, bool PF, bool TURNS>
 int launch_spmv_g(const DevCsr& A, const float* x, float* y, const float* add, float add_scale, const float* pdot,
                   double* dot_acc, const int* done, cudaStream_t st) {
     // up to 64 CTAs of 256 threads per SM, the rest by the grid-stride loop
     // (measured on the 2M-ray matrix: 16 per SM 0.58 ms, 32 0.56, 64 0.54 for A x)
     const long long b = (A.rows * G + 255) / 256;
     const unsigned blocks = (unsigned)std::max<long long>(1, std::min<long long>(b, (long long)grid_cap() * 4));
-    spmv_kernel<G, K, PF><<<blocks, 256, 0, st>>>(A.row_ptr, A.col, A.val, x, y, A.rows, add, add_scale, pdot, dot_acc,
+    spmv_kernel<G, K, PF, TURNS><<<blocks, 256, 0, st>>>(A.row_ptr, A.col, A.val, x, y, A.rows, add, add_scale, pdot, dot_acc,
                                                   done);
     count_launch();
     ST_CUDA(cudaGetLastError());
@@ -412,10 +449,11 @@ inline bool quads_ok(std::initializer_list<const void*> ps) {
 }
 
 // x += alpha p, r -= alpha q, z = M r; acc rz_new = <r,z>, rr = <r,r>.
-// Bound by memory (8 words per unknown) beside the FP64 sums: read and written
+// Bound by memory (8 words per unknown): read and written
 // four unknowns at a time where the caller's x allows it (quads), so that a
-// thread has five 16-byte loads in flight (one word at a time: 169 us at 16.8M
-// unknowns, 3.2 TB/s).
+// thread has five 16-byte loads in flight, with the inner products carried in
+// pairs of FP32 values within a quad. 16.8M unknowns: 85 us (a copy of the bytes
+// takes 79), 146 with FP64 products, 169 with single words as well.
 // alpha = rz_old / pq; |pq| < 1e-30 stops the solve (sparse_ops.cpp:37,88).
 // The scalars are formed once per block (FP64 is a slow pipe on this GPU).
 // skip_rz: <r, z> comes from the stencil preconditioner's kernel instead.
@@ -459,15 +497,25 @@ __global__ void cg_update_kernel(long long n, float* __restrict__ x, float* __re
         reinterpret_cast<float4*>(x)[i] = x4;
         reinterpret_cast<float4*>(r)[i] = r4;
         if (z) reinterpret_cast<float4*>(z)[i] = z4;
-        const double r0 = r4.x, r1 = r4.y, r2 = r4.z, r3 = r4.w;
-        a += r0 * (double)z4.x;
-        a += r1 * (double)z4.y;
-        a += r2 * (double)z4.z;
-        a += r3 * (double)z4.w;
-        c += r0 * r0;
-        c += r1 * r1;
-        c += r2 * r2;
-        c += r3 * r3;
+        const bool safe = pair_safe(r4.x) & pair_safe(r4.y) & pair_safe(r4.z) & pair_safe(r4.w) & pair_safe(z4.x) &
+                          pair_safe(z4.y) & pair_safe(z4.z) & pair_safe(z4.w);
+        if (!safe) {
+            const double r0 = r4.x, r1 = r4.y, r2 = r4.z, r3 = r4.w;
+            a += (r0 * (double)z4.x + r1 * (double)z4.y) + (r2 * (double)z4.z + r3 * (double)z4.w);
+            c += (r0 * r0 + r1 * r1) + (r2 * r2 + r3 * r3);
+            continue;
+        }
+        PairSum rz, rr;
+        rz.add(r4.x, z4.x);
+        rz.add(r4.y, z4.y);
+        rz.add(r4.z, z4.z);
+        rz.add(r4.w, z4.w);
+        rr.add(r4.x, r4.x);
+        rr.add(r4.y, r4.y);
+        rr.add(r4.z, r4.z);
+        rr.add(r4.w, r4.w);
+        a += rz.value();
+        c += rr.value();
     }
     for (long long i = 4 * n4 + blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
          i += (long long)gridDim.x * blockDim.x) {
@@ -567,27 +615,90 @@ __global__ void jacobi_kernel(const long long* __restrict__ rp, const int* __res
     }
 }
 
-// diag of A^T A + lam I from the rows of A^T: 1 / (sum_k AT[j,k]^2 + lam).
-// G lanes per row (coalesced), the squares exact and their sums in FP64.
-template <int G>
+// diag of A^T A + lam I from the rows of A^T: 1 / (sum_k AT[j,k]^2 + lam). A warp
+// per row, its lanes over the entries (coalesced). The rows of a warp lie a grid
+// apart (neighbouring cells are heavy together: where rays meet, a row holds
+// thousands of entries), and each group of 32 keeps row w's sum on lane w, so
+// that the FP64 division runs on full warps; pairs of FP32 values carry the
+// squares until then. 1M rows of 361 entries: 0.48 ms (2.15 with FP64 sums and a
+// warp per row, 4.19 with a thread per row). Short rows (less than 24 entries) are staged through
+// shared memory instead, a thread per row.
 __global__ void normal_jacobi_kernel(const long long* __restrict__ rp, const float* __restrict__ val, long long rows,
                                      double lam, float* __restrict__ dinv) {
-    const int lane = threadIdx.x % G;
-    const long long stride = (long long)gridDim.x * blockDim.x / G;
-    const long long first = (blockIdx.x * (long long)blockDim.x + (threadIdx.x & ~31u)) / G;  // of the warp: uniform trips
-    const long long gid = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / G;
-    for (long long it = 0; first + it * stride < rows; ++it) {
-        const long long i = gid + it * stride;
-        const long long a = i < rows ? rp[i] : 0, b = i < rows ? rp[i + 1] : 0;
-        double s = 0.0;
-#pragma unroll 4
-        for (long long p = a + lane; p < b; p += G) {
-            const double v = (double)__ldg(val + p);
-            s = fma(v, v, s);
-        }
+    const int lane = threadIdx.x & 31;
+    const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
+    const long long first = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
+    for (long long r0 = first; r0 < rows; r0 += 32 * warps) {
+        float mh = 0.0f, ml = 0.0f;
+        double wide = -1.0;  // the sum where the pairs cannot hold it
+        for (int w = 0; w < 32; ++w) {
+            const long long r = r0 + w * warps;
+            if (r >= rows) break;
+            const long long ra = rp[r], rb = rp[r + 1];
+            PairSum s;
+            unsigned odd = 0;
+            for (long long q = ra + lane; q - lane < rb; q += 8 * 32) {
+                float v[8];
 #pragma unroll
-        for (int o = G / 2; o > 0; o >>= 1) s += __shfl_xor_sync(FULL, s, o, G);
-        if (lane == 0 && i < rows) dinv[i] = (float)(1.0 / (s + lam));
+                for (int k = 0; k < 8; ++k) v[k] = q + 32 * k < rb ? __ldg(val + q + 32 * k) : 0.0f;
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    odd |= pair_safe(v[k]) ? 0u : 1u;
+                    s.add(v[k], v[k]);
+                }
+            }
+            if (!__any_sync(FULL, odd)) {
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    const float h = __shfl_xor_sync(FULL, s.h, o), l = __shfl_xor_sync(FULL, s.l, o);
+                    s.add(h, 1.0f);
+                    s.l += l;
+                }
+                if (lane == w) {
+                    mh = s.h;
+                    ml = s.l;
+                }
+            } else {
+                double t = 0.0;
+                for (long long e = ra + lane; e < rb; e += 32) t += (double)val[e] * (double)val[e];
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(FULL, t, o);
+                if (lane == w) wide = t;
+            }
+        }
+        const double mine = wide >= 0.0 || wide != wide ? wide : (double)mh + (double)ml;
+        const long long i = r0 + lane * warps;
+        if (i < rows) dinv[i] = (float)(1.0 / (mine + lam));
+    }
+}
+
+__global__ void __launch_bounds__(SR_ROWS) normal_jacobi_rows_kernel(const long long* __restrict__ rp,
+                                                                     const float* __restrict__ val, long long rows,
+                                                                     double lam, float* __restrict__ dinv) {
+    constexpr int CAP = 24 * SR_ROWS;
+    __shared__ float v[CAP];
+    for (long long r0 = (long long)blockIdx.x * SR_ROWS; r0 < rows; r0 += (long long)gridDim.x * SR_ROWS) {
+        const long long i = r0 + threadIdx.x;
+        const long long e0 = rp[r0], e1 = rp[min(r0 + SR_ROWS, rows)];
+        const long long a = i < rows ? rp[i] : 0, b = i < rows ? rp[i + 1] : 0;
+        const bool staged = e1 - e0 <= CAP;
+        if (staged)
+            for (long long e = e0 + threadIdx.x; e < e1; e += SR_ROWS) v[e - e0] = __ldg(val + e);
+        __syncthreads();
+        PairSum s;
+        bool safe = staged;
+        if (staged)
+            for (int k = (int)(a - e0); k < (int)(b - e0); ++k) {
+                safe = safe & pair_safe(v[k]);
+                s.add(v[k], v[k]);
+            }
+        double t = s.value();
+        if (!safe) {
+            t = 0.0;
+            for (long long e = a; e < b; ++e) t += (double)val[e] * (double)val[e];
+        }
+        if (i < rows) dinv[i] = (float)(1.0 / (t + lam));
+        __syncthreads();
     }
 }
 
@@ -779,18 +890,18 @@ int launch_spmv(const DevCsr& A, const float* x, float* y, const float* add, flo
         return e ? std::atoi(e) : 0;
     }();
     switch (forced) {
-        case 32: return launch_spmv_g<32, 6, false>(A, x, y, add, add_scale, pdot, dot_acc, done, st);
-        case 16: return launch_spmv_g<16, 10, true>(A, x, y, add, add_scale, pdot, dot_acc, done, st);
-        case 8: return launch_spmv_g<8, 4, true>(A, x, y, add, add_scale, pdot, dot_acc, done, st);
+        case 32: return launch_spmv_g<32, 6, false, true>(A, x, y, add, add_scale, pdot, dot_acc, done, st);
+        case 16: return launch_spmv_g<16, 10, true, false>(A, x, y, add, add_scale, pdot, dot_acc, done, st);
+        case 8: return launch_spmv_g<8, 4, true, false>(A, x, y, add, add_scale, pdot, dot_acc, done, st);
         case 1: return launch_spmv_rows(A, x, y, add, add_scale, pdot, dot_acc, done, st);
         default: break;
     }
     // measured on the 2M-ray matrix (180 entries per row) and its transpose (360): 16 threads per
     // row with 10 entries held per lane and the L2 prefetch 0.545 ms; the transpose with 32
-    // threads, 6 entries per lane and no prefetch 0.599 ms (before the held entries: 0.66 / 0.80)
-    if (avg >= 256) return launch_spmv_g<32, 6, false>(A, x, y, add, add_scale, pdot, dot_acc, done, st);
-    if (avg >= 24) return launch_spmv_g<16, 10, true>(A, x, y, add, add_scale, pdot, dot_acc, done, st);
-    if (avg >= 10) return launch_spmv_g<8, 4, true>(A, x, y, add, add_scale, pdot, dot_acc, done, st);
+    // threads, 6 entries per lane, no prefetch and the rest in turns 0.570 ms (0.640 with the rest one by one)
+    if (avg >= 256) return launch_spmv_g<32, 6, false, true>(A, x, y, add, add_scale, pdot, dot_acc, done, st);
+    if (avg >= 24) return launch_spmv_g<16, 10, true, false>(A, x, y, add, add_scale, pdot, dot_acc, done, st);
+    if (avg >= 10) return launch_spmv_g<8, 4, true, false>(A, x, y, add, add_scale, pdot, dot_acc, done, st);
     return launch_spmv_rows(A, x, y, add, add_scale, pdot, dot_acc, done, st);
 }
 
@@ -813,12 +924,10 @@ int launch_jacobi(const DevCsr& A, float* dinv, cudaStream_t st) {
     return ST_OK;
 }
 int launch_normal_jacobi(const DevCsr& AT, double lam, float* dinv, cudaStream_t st) {
-    // coalesced, a warp per row (1M rows of 361 entries: 2.2 ms, bound by the FP64 pipe, against 4.19
-    // with a thread per row); 4 lanes where a row would leave most of a warp idle
     if (AT.nnz >= 24 * AT.rows)
-        normal_jacobi_kernel<32><<<blocks_for(AT.rows * 32), 256, 0, st>>>(AT.row_ptr, AT.val, AT.rows, lam, dinv);
+        normal_jacobi_kernel<<<blocks_for(AT.rows * 32) / 2 + 1, 256, 0, st>>>(AT.row_ptr, AT.val, AT.rows, lam, dinv);
     else
-        normal_jacobi_kernel<4><<<blocks_for(AT.rows * 4), 256, 0, st>>>(AT.row_ptr, AT.val, AT.rows, lam, dinv);
+        normal_jacobi_rows_kernel<<<blocks_for(AT.rows), SR_ROWS, 0, st>>>(AT.row_ptr, AT.val, AT.rows, lam, dinv);
     count_launch();
     ST_CUDA(cudaGetLastError());
     return ST_OK;

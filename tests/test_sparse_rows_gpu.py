@@ -54,15 +54,45 @@ def test_short_rows(kind, rows):
     assert np.all(np.abs(y.cpu().numpy() - want) <= (lengths + 1) * EPS * mag)
 
 
-@pytest.mark.parametrize("rows,m", [(3, 1), (700, 6), (130, 40), (1000, 300)])
-def test_normal_diagonal(rows, m):
+@pytest.mark.parametrize("scale", [1.0, 1e-22, 1e22])  # 1e-22, 1e22: the squares leave the FP32 range
+@pytest.mark.parametrize("rows,m", [(3, 1), (700, 6), (130, 40), (1000, 300), (40_000, 300)])
+def test_normal_diagonal(rows, m, scale):
     A, rp, col, val = _matrix(np.full(rows, m), 500, m)
+    A.scale(scale)
+    val = val * np.float32(scale)
     d = torch.zeros(500, device="cuda")
     torch.cuda.synchronize()
-    call("st_csr_normal_jacobi", A.handle, 0.25, d.data_ptr())
+    lam = 0.25 * scale * scale
+    call("st_csr_normal_jacobi", A.handle, lam, d.data_ptr())
     torch.cuda.synchronize()
-    want = 1.0 / (np.bincount(col, val.astype(np.float64) ** 2, minlength=500) + 0.25)
-    np.testing.assert_allclose(d.cpu().numpy(), want, rtol=2 * EPS)
+    want = 1.0 / (np.bincount(col, val.astype(np.float64) ** 2, minlength=500) + lam)
+    got = d.cpu().numpy()
+    fits = want < 3.4e38
+    # the reference as the output's type holds it (at 1e22 the inverses are subnormal)
+    np.testing.assert_allclose(got[fits], want[fits].astype(np.float32), rtol=2 * EPS)
+    assert np.isinf(got[~fits]).all()
+
+
+@pytest.mark.parametrize("scale", [1.0, 1e-15, 1e25, 1e-25])
+def test_cg_scales_with_its_right_hand_side(scale):
+    """Residuals at and beyond the range of the FP32 pairs: the iterates follow the right-hand side's scale, down to
+    the solver's own stop at |p.q| < 1e-30."""
+    n = 4100
+    idx = np.arange(n)
+    diag = 2.0 + np.random.default_rng(n).random(n)
+    A = se.CSRMatrix().build_from_triplets(n, n, np.concatenate([idx, idx[1:]]), np.concatenate([idx, idx[:-1]]),
+                                           np.concatenate([diag, np.full(n - 1, -0.5)]))
+    b = torch.from_numpy(np.random.default_rng(n + 1).standard_normal(n).astype(np.float32)).cuda()
+    x, xs = torch.zeros(n, device="cuda"), torch.zeros(n, device="cuda")
+    se.normal_cg_device(A, None, 0.1, x, 3, 1e-30, True, rhs=b)
+    it, rel, _ = se.normal_cg_device(A, None, 0.1, xs, 3, 1e-30, True, rhs=b * scale)
+    if scale == 1e-25:
+        assert it == 0 and not xs.any()
+        return
+    assert it == 3 and 0.0 < rel < 1.0
+    # b * scale rounds once per value, then the iterations' own rounding
+    np.testing.assert_allclose(xs.double().cpu().numpy() / scale, x.double().cpu().numpy(), rtol=0,
+                               atol=64 * EPS * float(x.abs().max()))
 
 
 @pytest.mark.parametrize("n", [1, 5, 1026, 70001])
