@@ -90,18 +90,59 @@ void set_receivers_args(StepArgs& a, const st_receiver_grid& R) {
     a.rny = (int)R.ny;
 }
 
+// FP64 model in the reference layout (edge-replicated halo) from an interior
+// FP32 velocity, and the bits of the largest finite velocity (0 when none is
+// positive).
+__global__ void vel_interior_to_model_kernel(const float* __restrict__ v, double* __restrict__ model, Layout L,
+                                             unsigned* vmax_bits) {
+    const long long nx = L.nx, ny = L.ny, nz = L.nz, NZh = nz + 2, n = L.NXh * L.NYh * NZh;
+    float m = 0.0f;
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
+        const long long xd = e / (L.NYh * NZh), r = e % (L.NYh * NZh), yd = r / NZh, zr = r % NZh;
+        const long long ix = min(max(xd - 1, 0ll), nx - 1), iy = min(max(yd - 1, 0ll), ny - 1),
+                        iz = min(max(zr - 1, 0ll), nz - 1);
+        const float x = v[(ix * ny + iy) * nz + iz];
+        model[e] = (double)x;
+        if (isfinite(x) && x > m) m = x;
+    }
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0 && m > 0.0f) atomicMax(vmax_bits, __float_as_uint(m));
+}
+
 double cfl_damp(st_solver* s) {
     // the coefficient array already carries damp^2; recover damp from it is
-    // not possible per point, so recompute the reference rule on the host copy
-    if (ensure_vel_host(s) != ST_OK) return 1.0;  // (a failed download reports through the next CUDA call)
+    // not possible per point, so recompute the reference rule from the model
     double vmax = 0.0;
-    for (double v : s->vel_host)
-        if (std::isfinite(v) && v > vmax) vmax = v;
+    if (model_vmax(s, &vmax) != ST_OK) return 1.0;  // (a failed download reports through the next CUDA call)
     const double dt = s->cfg.dt;
     const double cfl = std::max({vmax * dt / s->grid.dx, vmax * dt / s->grid.dy, vmax * dt / s->grid.dz});
     if (cfl <= 1.0) return 1.0;
     const double ratio = vmax * dt / std::min({s->grid.dx, s->grid.dy, s->grid.dz});
     return std::min(1.0, s->cfl_safety / ratio);
+}
+
+// The host copy of the model from an interior device velocity, for a device
+// without room for a copy of its own there.
+int model_to_host(st_solver* s, const float* vel) {
+    const Layout& L = s->L;
+    const long long n = L.nx * L.ny * L.nz;
+    std::vector<float> h((size_t)n);
+    ST_CUDA(cudaMemcpyAsync(h.data(), vel, (size_t)n * 4, cudaMemcpyDeviceToHost, s->stream));
+    ST_CUDA(cudaStreamSynchronize(s->stream));
+    const long long NXh = L.NXh, NYh = L.NYh, NZh = L.nz + 2, nx = L.nx, ny = L.ny, nz = L.nz;
+    auto clampi = [](long long v, long long hi) { return v < 0 ? 0 : (v > hi ? hi : v); };
+    for (long long xd = 0; xd < NXh; ++xd) {
+        const long long ix = clampi(xd - 1, nx - 1);
+        for (long long yd = 0; yd < NYh; ++yd) {
+            const long long iy = clampi(yd - 1, ny - 1);
+            double* row = s->vel_host.data() + (xd * NYh + yd) * NZh;
+            const float* src = h.data() + (ix * ny + iy) * nz;
+            for (long long zr = 0; zr < NZh; ++zr) row[zr] = src[clampi(zr - 1, nz - 1)];
+        }
+    }
+    s->vel_host_valid = true;
+    s->vmax = -1.0;
+    return ST_OK;
 }
 
 }  // namespace
@@ -215,23 +256,29 @@ int st_solver_set_velocity_device(st_solver* s, const float* vel) {
     ST_CHECK(s && vel, ST_ERR_ARG, "null argument");
     ST_CUDA(cudaSetDevice(s->device));
     const Layout& L = s->L;
-    const long long n = L.nx * L.ny * L.nz;
-    // host copy of the model (reference layout, edge-replicated halo) for field().velocity and the CFL rule
-    std::vector<float> h((size_t)n);
-    ST_CUDA(cudaMemcpyAsync(h.data(), vel, (size_t)n * 4, cudaMemcpyDeviceToHost, s->stream));
-    ST_CUDA(cudaStreamSynchronize(s->stream));
-    const long long NXh = L.NXh, NYh = L.NYh, NZh = L.nz + 2, nx = L.nx, ny = L.ny, nz = L.nz;
-    auto clampi = [](long long v, long long hi) { return v < 0 ? 0 : (v > hi ? hi : v); };
-    for (long long xd = 0; xd < NXh; ++xd) {
-        const long long ix = clampi(xd - 1, nx - 1);
-        for (long long yd = 0; yd < NYh; ++yd) {
-            const long long iy = clampi(yd - 1, ny - 1);
-            double* row = s->vel_host.data() + (xd * NYh + yd) * NZh;
-            const float* src = h.data() + (ix * ny + iy) * nz;
-            for (long long zr = 0; zr < NZh; ++zr) row[zr] = src[clampi(zr - 1, nz - 1)];
-        }
+    // The model for field().velocity and the CFL rule stays on the device (the
+    // host copy is refreshed only when read) and its maximum is found there: a
+    // 192^3 model took 12 ms through the host, and two of these calls and a
+    // scan of the host copy per shot stood beside 20 ms of propagation.
+    const size_t bytes = (size_t)ref_elems(s) * sizeof(double);
+    if (!s->vel_dev && cudaMalloc(&s->vel_dev, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        s->vel_dev = nullptr;
+        ST_TRY(model_to_host(s, vel));
+    } else {
+        ST_CUDA(cudaMemsetAsync(s->counter, 0, sizeof(unsigned long long), s->stream));
+        vel_interior_to_model_kernel<<<nblocks(ref_elems(s)), 256, 0, s->stream>>>(
+            vel, s->vel_dev, L, reinterpret_cast<unsigned*>(s->counter));
+        count_launch();
+        ST_CUDA(cudaGetLastError());
+        unsigned bits = 0;
+        ST_CUDA(cudaMemcpyAsync(&bits, s->counter, sizeof(bits), cudaMemcpyDeviceToHost, s->stream));
+        ST_CUDA(cudaStreamSynchronize(s->stream));
+        float m;
+        std::memcpy(&m, &bits, sizeof(m));
+        s->vmax = (double)m;
+        s->vel_host_valid = false;
     }
-    s->vel_host_valid = true;
     const double damp = cfl_damp(s);
     vel_interior_to_coeff_kernel<<<nblocks(L.elems), 256, 0, s->stream>>>(vel, s->c, L,
                                                                            s->cfg.dt * s->cfg.dt * damp * damp);

@@ -155,11 +155,18 @@ int ensure_vel_host(st_solver* s) {
 }
 
 // Largest finite velocity (compute_local_max_velocity, wave_equation.cpp:435-443).
-double host_vmax(const st_solver* s) {
-    double vmax = 0.0;
-    for (double v : s->vel_host)
-        if (std::isfinite(v) && v > vmax) vmax = v;
-    return vmax;
+// A scan of the host copy takes 2 ms per 10^6 cells, so it runs once per model and
+// not where a device-side upload has found the maximum already.
+int model_vmax(st_solver* s, double* out) {
+    if (s->vmax < 0.0) {
+        ST_TRY(ensure_vel_host(s));
+        double vmax = 0.0;
+        for (double v : s->vel_host)
+            if (std::isfinite(v) && v > vmax) vmax = v;
+        s->vmax = vmax;
+    }
+    *out = s->vmax;
+    return ST_OK;
 }
 
 // Square of the reference's CFL damping factor (wave_equation.cpp:316-387):
@@ -179,11 +186,9 @@ double cfl_damp2_of(st_solver* s, double vmax) {
     return f * f;
 }
 
-double cfl_damp2(st_solver* s) { return cfl_damp2_of(s, host_vmax(s)); }
-
 // Largest finite velocity of a device FP64 array, as the bits of a
 // non-negative double (monotonic as unsigned integers); 0 when none is
-// positive, as host_vmax.
+// positive, as model_vmax.
 __global__ void vmax_finite_kernel(const double* __restrict__ v, long long n, unsigned long long* out) {
     double m = 0.0;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -212,16 +217,19 @@ int upload_velocity(st_solver* s, const double* vp) {
     std::memcpy(&vmax, &bits, sizeof(vmax));
     ST_TRY(launch_vel_to_coeff(s->vel_dev, s->c, s->L, s->cfg.dt * s->cfg.dt * cfl_damp2_of(s, vmax), s->stream));
     s->vel_host_valid = false;
+    s->vmax = vmax;
     s->coeff_dirty = false;
     return ST_OK;
 }
 
 int refresh_coeff(st_solver* s) {
     if (!s->coeff_dirty) return ST_OK;
+    double vmax = 0.0;
+    ST_TRY(model_vmax(s, &vmax));
     ST_TRY(ensure_staging(s));
     ST_CUDA(cudaMemcpyAsync(s->staging, s->vel_host.data(), (size_t)ref_elems(s) * sizeof(double),
                             cudaMemcpyHostToDevice, s->stream));
-    ST_TRY(launch_vel_to_coeff(s->staging, s->c, s->L, s->cfg.dt * s->cfg.dt * cfl_damp2(s), s->stream));
+    ST_TRY(launch_vel_to_coeff(s->staging, s->c, s->L, s->cfg.dt * s->cfg.dt * cfl_damp2_of(s, vmax), s->stream));
     ST_CUDA(cudaStreamSynchronize(s->stream));
     s->coeff_dirty = false;
     return ST_OK;
@@ -547,6 +555,7 @@ int st_solver_initialize_velocity(st_solver* s, double vp0) {
     ST_CHECK(s, ST_ERR_ARG, "null solver");
     std::fill(s->vel_host.begin(), s->vel_host.end(), vp0);
     s->vel_host_valid = true;
+    s->vmax = -1.0;
     s->coeff_dirty = true;
     return ST_OK;
 }
@@ -556,6 +565,7 @@ int st_solver_set_velocity_field(st_solver* s, const double* vp, int64_t count) 
     const int64_t n = std::min<int64_t>(count, (int64_t)s->vel_host.size());
     ST_TRY(ensure_vel_host(s));
     if (n > 0) std::memcpy(s->vel_host.data(), vp, (size_t)n * sizeof(double));
+    s->vmax = -1.0;
     s->coeff_dirty = true;
     return ST_OK;
 }
@@ -736,7 +746,9 @@ int st_solver_compute_energy(st_solver* s, double* out) {
 int st_solver_verify_cfl(st_solver* s, int* ok) {
     // FaultTolerance::verify_cfl_condition (core/fault_tolerance.cpp:49-70)
     ST_CHECK(s && ok, ST_ERR_ARG, "null argument");
-    const double vmax = host_vmax(s), dt = s->cfg.dt;
+    double vmax = 0.0;
+    ST_TRY(model_vmax(s, &vmax));
+    const double dt = s->cfg.dt;
     const double cfl = std::max({vmax * dt / s->grid.dx, vmax * dt / s->grid.dy, vmax * dt / s->grid.dz});
     *ok = cfl <= s->cfl_safety ? 1 : 0;
     return ST_OK;
