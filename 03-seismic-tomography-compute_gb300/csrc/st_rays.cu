@@ -31,6 +31,7 @@
 // outruns its bound sends the call to the triplet builder. 500k rays on 50^3 cells
 // (45M entries): build, transpose and two products 6.3 ms, 16.8 with two plain
 // walks and the sort of the triplets.
+#include "st_fp64.cuh"
 #include "st_sort.cuh"
 #include "st_sparse.cuh"
 
@@ -119,23 +120,17 @@ __device__ __forceinline__ long long time_key(double t) {
     return b < 0 ? (long long)0x8000000000000000ull - b : b;
 }
 
-// x / d, correctly rounded, from y = 1 / d correctly rounded: two steps of
-// Markstein's correction ("Computation of elementary functions on the IBM RISC
-// System/6000 processor", 1990): the first leaves the quotient within one unit in
-// the last place, so the second's remainder is exact and its rounding correct. For
-// |d| in 2^-300 .. 2^300; x below 2^-400 goes to the division.
+// x / d through the axis's reciprocal y; an x below 2^-400 goes to the division.
 __device__ __forceinline__ double quotient(double x, double d, double y) {
     const unsigned hx = (unsigned)__double2hiint(x) & 0x7fffffffu;
-    if (hx < (623u << 20) && x != 0.0) return __ddiv_rn(x, d);
-    double q = __dmul_rn(x, y);
-    q = __fma_rn(__fma_rn(-q, d, x), y, q);
-    return __fma_rn(__fma_rn(-q, d, x), y, q);
+    if (hx < (623u << 20) && (hx | (unsigned)__double2loint(x))) return __ddiv_rn(x, d);
+    return quotient_of(x, d, y);
 }
 
 // Whether the fast walk takes an axis: finite, and d zero or of moderate size.
 __device__ __forceinline__ bool fast_axis(double p, double d) {
-    const unsigned hp = (unsigned)__double2hiint(p) & 0x7fffffffu, hd = (unsigned)__double2hiint(d) & 0x7fffffffu;
-    return hp < (1323u << 20) && hd < (1323u << 20) && (hd >= (723u << 20) || d == 0.0);
+    const unsigned hp = (unsigned)__double2hiint(p) & 0x7fffffffu;
+    return hp < (1323u << 20) && (moderate(d) || d == 0.0);
 }
 
 // The most iterations of walk(): one and, per axis, the faces between the start

@@ -18,10 +18,15 @@
 // sorted order. Both kernels are bound by the FP64 pipe (one correctly
 // rounded division per sample); threads take picks and cells in order of
 // their sample counts, so the lanes of a warp run loops of similar length
-// and the FP64 pipe is not spent on masked-off lanes. All FP64 arithmetic is written with explicitly rounded
-// intrinsics (no contraction into FMA), so each value is the reference's
-// expression evaluated in IEEE double: the results match it bit for bit
-// given the same source-station distances.
+// and the FP64 pipe is not spent on masked-off lanes. The divisor belongs to
+// the cell (v, or v * v), so its reciprocal is formed once per cell and call and
+// the sample's quotient takes five operations (quotient_of, correctly rounded)
+// where the division takes about ten; values out of its range are divided. All
+// FP64 arithmetic is written with explicitly rounded intrinsics (no contraction
+// into FMA), so each value is the reference's expression evaluated in IEEE
+// double: the results match it bit for bit given the same source-station
+// distances.
+#include "st_fp64.cuh"
 #include "st_sort.cuh"
 #include "st_sparse.cuh"
 
@@ -43,6 +48,9 @@ struct st_ray_picks {
     int* t_pick = nullptr;        // [n_samples] pick of each sample, cell-major
     int* pick_order = nullptr;    // [n_picks] picks by descending sample count
     int* cell_order = nullptr;    // [n_cells] cells by descending sample count
+    double2* table = nullptr;     // [n_cells] (velocity used, its reciprocal or 0) of the current call
+    double* trial_times = nullptr;  // line-search trials: [n_picks], on first use
+    double* partial = nullptr;      // and the misfit's partial sums
     double* stage_vp = nullptr;   // host-call staging: [n_cells]
     double* stage_res = nullptr;  // [n_picks]
     double* stage_out = nullptr;  // [max(n_cells, n_picks)]
@@ -56,6 +64,9 @@ struct st_ray_picks {
         cudaFree(t_pick);
         cudaFree(pick_order);
         cudaFree(cell_order);
+        cudaFree(table);
+        cudaFree(trial_times);
+        cudaFree(partial);
         cudaFree(stage_vp);
         cudaFree(stage_res);
         cudaFree(stage_out);
@@ -180,54 +191,126 @@ __global__ void gather_pick_kernel(const unsigned* __restrict__ order, const uns
         t_pick[k] = (int)spick[order[k]];
 }
 
-__device__ inline bool valid_velocity(double v) { return isfinite(v) && v > 0.0; }
+__device__ inline bool valid_velocity(double v) { return finite_bits(v) && v > 0.0; }
+
+// The velocity a cell's samples are divided by (invalid -> 1500) and its
+// reciprocal, 0 where quotient_of does not take it.
+__device__ __forceinline__ double2 table_entry(double v) {
+    if (!valid_velocity(v)) v = 1500.0;
+    return make_double2(v, moderate(v) ? __drcp_rn(v) : 0.0);
+}
+
+__global__ void table_kernel(const double* __restrict__ vp, long long nc, double2* __restrict__ table) {
+    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < nc;
+         c += (long long)gridDim.x * blockDim.x)
+        table[c] = table_entry(vp[c]);
+}
+
+struct TrialClamp {
+    double lo, hi;   // the model's range
+    double plo, phi; // the fault policy's, applied first when set
+    int policy;
+};
+
+__device__ __forceinline__ double clamp_finite(double v, double lo, double hi) {
+    if (!finite_bits(v)) v = lo;
+    return v < lo ? lo : (v > hi ? hi : v);
+}
+
+// The table of the trial model clamp(vp - step g).
+__global__ void trial_table_kernel(const double* __restrict__ vp, const double* __restrict__ g, double step,
+                                   TrialClamp C, long long nc, double2* __restrict__ table) {
+    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < nc;
+         c += (long long)gridDim.x * blockDim.x) {
+        double v = __dsub_rn(vp[c], __dmul_rn(step, g[c]));
+        if (C.policy) v = clamp_finite(v, C.plo, C.phi);
+        table[c] = table_entry(clamp_finite(v, C.lo, C.hi));
+    }
+}
+
+// ds / v of one sample.
+__device__ __forceinline__ double sample_time(double d, double2 e, bool fast) {
+    return fast && e.y != 0.0 ? quotient_of(d, e.x, e.y) : __ddiv_rn(d, e.x);
+}
 
 // _forward_model (inversion.py:329-381), one thread per pick, the samples
-// added in order. The loads and divisions of four samples are issued
+// added in order. The loads and quotients of four samples are issued
 // together (they are independent); only the additions keep the reference's
 // order.
 __global__ void ray_forward_kernel(long long np, const int* __restrict__ order, const long long* __restrict__ off,
                                    const int* __restrict__ cell, const double* __restrict__ ds,
-                                   const double* __restrict__ dist, const double* __restrict__ vp,
+                                   const double* __restrict__ dist, const double2* __restrict__ table,
                                    double* __restrict__ times) {
     for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < np;
          j += (long long)gridDim.x * blockDim.x) {
         const long long i = order[j];
         const long long b = off[i], e = off[i + 1];
         const double d = ds[i];
+        const bool fast = moderate(d) || d == 0.0;
         double t = 0.0;
         long long k = b;
         for (; k + 4 <= e; k += 4) {
+            double2 v[4];
             double term[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                double v = __ldg(vp + __ldg(cell + k + j));
-                if (!valid_velocity(v)) v = 1500.0;
-                term[j] = __ddiv_rn(d, v);
-            }
+            for (int j = 0; j < 4; ++j) v[j] = __ldg(table + __ldg(cell + k + j));
+#pragma unroll
+            for (int j = 0; j < 4; ++j) term[j] = sample_time(d, v[j], fast);
 #pragma unroll
             for (int j = 0; j < 4; ++j)
-                if (isfinite(term[j])) t = __dadd_rn(t, term[j]);
+                if (finite_bits(term[j])) t = __dadd_rn(t, term[j]);
         }
         for (; k < e; ++k) {
-            double v = __ldg(vp + __ldg(cell + k));
-            if (!valid_velocity(v)) v = 1500.0;
-            const double term = __ddiv_rn(d, v);
-            if (isfinite(term)) t = __dadd_rn(t, term);
+            const double term = sample_time(d, __ldg(table + __ldg(cell + k)), fast);
+            if (finite_bits(term)) t = __dadd_rn(t, term);
         }
-        if (b < e && (!isfinite(t) || t < 0.0)) t = __ddiv_rn(dist[i], 6000.0);
+        if (b < e && (!finite_bits(t) || t < 0.0)) t = __ddiv_rn(dist[i], 6000.0);
         times[i] = t;
     }
+}
+
+// Misfit of the traveltimes (obs_data.py:116-129): sum of w r^2 (halved by the
+// caller) or of w |r|, in an order that depends only on the pick count, so equal
+// times give equal misfits.
+constexpr int MISFIT_BLOCKS = 608;
+__device__ __forceinline__ double block_total(double s) {
+    __shared__ double part[8];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+    __syncthreads();
+    s = 0.0;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += part[w];
+    return s;
+}
+
+__global__ void misfit_kernel(const double* __restrict__ times, const double* __restrict__ obs,
+                              const double* __restrict__ weight, long long np, int l1, double* __restrict__ partial) {
+    double s = 0.0;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < np;
+         i += (long long)gridDim.x * blockDim.x) {
+        const double r = __dsub_rn(obs[i], times[i]);
+        s = __dadd_rn(s, __dmul_rn(weight[i], l1 ? fabs(r) : __dmul_rn(r, r)));
+    }
+    s = block_total(s);
+    if (threadIdx.x == 0) partial[blockIdx.x] = s;
+}
+
+__global__ void misfit_total_kernel(double* __restrict__ partial) {
+    double s = 0.0;
+    for (int b = threadIdx.x; b < MISFIT_BLOCKS; b += blockDim.x) s += partial[b];
+    s = block_total(s);
+    if (threadIdx.x == 0) partial[MISFIT_BLOCKS] = s;
 }
 
 // _compute_gradient (inversion.py:383-433), one thread per cell, its samples
 // in (pick, sample) order: g += (r * (-ds / (v * v))) * w. Terms of four
 // samples are formed together; the additions keep the order.
-__device__ inline double grad_term(int i, double vv, const double* __restrict__ ds, const double* __restrict__ weight,
-                                   const double* __restrict__ res, bool* ok) {
+__device__ inline double grad_term(int i, double vv, double y, const double* __restrict__ ds,
+                                   const double* __restrict__ weight, const double* __restrict__ res, bool* ok) {
     const double r = __ldg(res + i);
-    const double f = __ddiv_rn(-__ldg(ds + i), vv);
-    *ok = isfinite(r) && isfinite(f);
+    const double d = -__ldg(ds + i);
+    const double f = y != 0.0 && (moderate(d) || d == 0.0) ? quotient_of(d, vv, y) : __ddiv_rn(d, vv);
+    *ok = finite_bits(r) && finite_bits(f);
     return __dmul_rn(__dmul_rn(r, f), __ldg(weight + i));
 }
 
@@ -244,19 +327,20 @@ __global__ void ray_gradient_kernel(long long nc, const int* __restrict__ order,
         double acc = 0.0;
         if (b < e && valid_velocity(v)) {
             const double vv = __dmul_rn(v, v);
+            const double y = moderate(vv) ? __drcp_rn(vv) : 0.0;
             long long k = b;
             for (; k + 4 <= e; k += 4) {
                 double term[4];
                 bool ok[4];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) term[j] = grad_term(__ldg(t_pick + k + j), vv, ds, weight, res, ok + j);
+                for (int j = 0; j < 4; ++j) term[j] = grad_term(__ldg(t_pick + k + j), vv, y, ds, weight, res, ok + j);
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
                     if (ok[j]) acc = __dadd_rn(acc, term[j]);
             }
             for (; k < e; ++k) {
                 bool ok;
-                const double term = grad_term(__ldg(t_pick + k), vv, ds, weight, res, &ok);
+                const double term = grad_term(__ldg(t_pick + k), vv, y, ds, weight, res, &ok);
                 if (ok) acc = __dadd_rn(acc, term);
             }
         }
@@ -464,6 +548,7 @@ int st_ray_picks_create(int device, const st_ray_model* model, int64_t n_picks, 
     ST_CUDA(cudaMalloc(&p->ds, (size_t)npp * 8));
     ST_CUDA(cudaMalloc(&p->dist, (size_t)npp * 8));
     ST_CUDA(cudaMalloc(&p->weight, (size_t)npp * 8));
+    ST_CUDA(cudaMalloc(&p->table, (size_t)p->n_cells * sizeof(double2)));
     ST_CUDA(cudaMalloc(&p->stage_vp, (size_t)p->n_cells * 8));
     ST_CUDA(cudaMalloc(&p->stage_res, (size_t)npp * 8));
     ST_CUDA(cudaMalloc(&p->stage_out, (size_t)std::max(npp, p->n_cells) * 8));
@@ -508,8 +593,10 @@ int st_ray_picks_forward_model(st_ray_picks* p, const double* vp, int on_device,
         dt = p->stage_out;
     }
     if (p->n_picks > 0) {
+        table_kernel<<<blocks_for(p->n_cells, 256), 256, 0, st>>>(dvp, p->n_cells, p->table);
+        count_launch();
         ray_forward_kernel<<<blocks_for(p->n_picks, 128), 128, 0, st>>>(p->n_picks, p->pick_order, p->off, p->cell,
-                                                                        p->ds, p->dist, dvp, dt);
+                                                                        p->ds, p->dist, p->table, dt);
         count_launch();
         ST_CUDA(cudaGetLastError());
     }
@@ -546,6 +633,55 @@ int st_ray_picks_compute_gradient(st_ray_picks* p, const double* vp, const doubl
         ST_CUDA(cudaStreamSynchronize(st));
     }
     return ST_OK;
+}
+
+// Scratch of the misfit entry points, on first use.
+static int ensure_misfit(st_ray_picks* p, bool times) {
+    if (!p->partial) ST_CUDA(cudaMalloc(&p->partial, (MISFIT_BLOCKS + 1) * sizeof(double)));
+    if (times && !p->trial_times)
+        ST_CUDA(cudaMalloc(&p->trial_times, (size_t)std::max<long long>(p->n_picks, 1) * sizeof(double)));
+    return ST_OK;
+}
+
+static int misfit_of(st_ray_picks* p, const double* times, const double* obs, const double* weight, int l1,
+                     double* out) {
+    misfit_kernel<<<MISFIT_BLOCKS, 256, 0, p->stream>>>(times, obs, weight, p->n_picks, l1, p->partial);
+    count_launch();
+    misfit_total_kernel<<<1, 256, 0, p->stream>>>(p->partial);
+    count_launch();
+    ST_CUDA(cudaGetLastError());
+    double s = 0.0;
+    ST_CUDA(cudaMemcpyAsync(&s, p->partial + MISFIT_BLOCKS, sizeof(s), cudaMemcpyDeviceToHost, p->stream));
+    ST_CUDA(cudaStreamSynchronize(p->stream));
+    *out = l1 ? s : 0.5 * s;
+    return ST_OK;
+}
+
+int st_ray_picks_misfit(st_ray_picks* p, const double* times, const double* obs, const double* weight, int l1,
+                        double* misfit) {
+    ST_CHECK(p && misfit && (p->n_picks == 0 || (times && obs && weight)), ST_ERR_ARG, "null argument");
+    ST_CUDA(cudaSetDevice(p->device));
+    ST_TRY(ensure_misfit(p, false));
+    return misfit_of(p, times, obs, weight, l1, misfit);
+}
+
+int st_ray_picks_trial_misfit(st_ray_picks* p, const double* vp, const double* gradient, double step,
+                              const double* policy_range, double vp_min, double vp_max, const double* obs,
+                              const double* weight, int l1, double* misfit) {
+    ST_CHECK(p && vp && gradient && misfit && (p->n_picks == 0 || (obs && weight)), ST_ERR_ARG, "null argument");
+    ST_CUDA(cudaSetDevice(p->device));
+    ST_TRY(ensure_misfit(p, true));
+    const TrialClamp C{vp_min, vp_max, policy_range ? policy_range[0] : 0.0, policy_range ? policy_range[1] : 0.0,
+                       policy_range != nullptr};
+    trial_table_kernel<<<blocks_for(p->n_cells, 256), 256, 0, p->stream>>>(vp, gradient, step, C, p->n_cells, p->table);
+    count_launch();
+    if (p->n_picks > 0) {
+        ray_forward_kernel<<<blocks_for(p->n_picks, 128), 128, 0, p->stream>>>(
+            p->n_picks, p->pick_order, p->off, p->cell, p->ds, p->dist, p->table, p->trial_times);
+        count_launch();
+    }
+    ST_CUDA(cudaGetLastError());
+    return misfit_of(p, p->trial_times, obs, weight, l1, misfit);
 }
 
 }  // extern "C"

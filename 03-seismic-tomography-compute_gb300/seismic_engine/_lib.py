@@ -205,6 +205,8 @@ SIGNATURES = {
     "st_ray_picks_stream": [_vp, C.POINTER(_vp)],
     "st_ray_picks_forward_model": [_vp, _vp, C.c_int, _vp],
     "st_ray_picks_compute_gradient": [_vp, _vp, _vp, C.c_int, _vp],
+    "st_ray_picks_misfit": [_vp, _vp, _vp, _vp, C.c_int, _d],
+    "st_ray_picks_trial_misfit": [_vp, _vp, _vp, C.c_double, _d, C.c_double, C.c_double, _vp, _vp, C.c_int, _d],
     "st_csr_shape": [_vp, _i64],
     "st_mmap_writer_open": [C.c_char_p, C.c_int64, C.POINTER(_vp)],
     "st_mmap_writer_write_frame": [_vp, _vp, C.c_int64],

@@ -148,12 +148,12 @@ class AdjointStateInversion:
 
     def _misfit(self, times) -> float:
         """OBSDataCoordinator.compute_misfit (obs_data.py:116-129)."""
-        r = self.observed - times
-        if self.misfit_type in ("l2", "cross_correlation"):
-            return float(0.5 * (self.weights * (r * r)).sum())
-        if self.misfit_type == "l1":
-            return float((self.weights * r.abs()).sum())
-        raise ValueError(f"Unknown misfit type: {self.misfit_type}")
+        return self.rays.misfit(times, self.observed, self.weights, self._l1())
+
+    def _l1(self) -> bool:
+        if self.misfit_type not in ("l2", "cross_correlation", "l1"):
+            raise ValueError(f"Unknown misfit type: {self.misfit_type}")
+        return self.misfit_type == "l1"
 
     def _smooth(self, g):
         """SparseOps.smooth_gradient on the device (FP64)."""
@@ -198,16 +198,26 @@ class AdjointStateInversion:
         return vp
 
     def _line_search(self, vp, gradient, current_misfit: float) -> float:
-        """inversion.py:436-453."""
+        """inversion.py:436-453. A trial is the table of its model, its
+        traveltimes and their misfit in four launches and one read; a subclass
+        or policy with its own clamp, forward model or misfit takes them."""
         step = self.step_length
+        lo, hi = self.model.vp_min, self.model.vp_max  # update_from_flat's clamp, model left unchanged
+        cls, ref = type(self), AdjointStateInversion
+        fused = (cls._forward is ref._forward and cls._misfit is ref._misfit and
+                 type(self.fault_policy).clamp_velocity is FaultRecoveryPolicy.clamp_velocity)
         for _ in range(self.line_search_max):
-            trial = vp - step * gradient
-            if self.enable_fault_tolerance:
-                trial = self.fault_policy.clamp_velocity(trial)
-            lo, hi = self.model.vp_min, self.model.vp_max  # update_from_flat's clamp, model left unchanged
-            import torch
-            trial = torch.where(torch.isfinite(trial), trial, torch.full_like(trial, lo)).clamp(lo, hi)
-            trial_misfit = self._misfit(self._forward(trial))
+            if fused:
+                trial_misfit = self.rays.trial_misfit(
+                    vp, gradient, step, self.fault_policy.velocity_clamp_range if self.enable_fault_tolerance else None,
+                    lo, hi, self.observed, self.weights, self._l1())
+            else:
+                import torch
+                trial = vp - step * gradient
+                if self.enable_fault_tolerance:
+                    trial = self.fault_policy.clamp_velocity(trial)
+                trial = torch.where(torch.isfinite(trial), trial, torch.full_like(trial, lo)).clamp(lo, hi)
+                trial_misfit = self._misfit(self._forward(trial))
             if not math.isfinite(trial_misfit):
                 step *= self.fault_policy.step_reduction_factor
                 continue

@@ -177,6 +177,34 @@ class SampledRays:
         call("st_ray_picks_compute_gradient", self._h, v.ctypes.data, r.ctypes.data, 0, g.ctypes.data)
         return g
 
+    # ---- the line search's misfits (device tensors)
+    def misfit(self, times, observed, weights, l1: bool = False) -> float:
+        """OBSDataCoordinator.compute_misfit (obs_data.py:116-129) of CUDA
+        float64 traveltimes: 1/2 sum w r^2, or sum w |r| with l1."""
+        for a, name in ((times, "times"), (observed, "observed"), (weights, "weights")):
+            self._check_tensor(a, self.n_picks, name)
+        out = C.c_double()
+        self._enter()
+        call("st_ray_picks_misfit", self._h, times.data_ptr(), observed.data_ptr(), weights.data_ptr(), int(l1),
+             C.byref(out))
+        return out.value
+
+    def trial_misfit(self, vp, gradient, step: float, policy_range, vp_min: float, vp_max: float, observed, weights,
+                     l1: bool = False) -> float:
+        """Misfit of the model vp - step * gradient clamped to policy_range
+        (None: not) and to vp_min .. vp_max: one trial of the line search
+        (inversion.py:436-453) without a model or traveltimes of its own."""
+        self._check_tensor(vp, self.n_cells, "vp")
+        self._check_tensor(gradient, self.n_cells, "gradient")
+        for a, name in ((observed, "observed"), (weights, "weights")):
+            self._check_tensor(a, self.n_picks, name)
+        out = C.c_double()
+        pr = None if policy_range is None else (C.c_double * 2)(*(float(v) for v in policy_range))
+        self._enter()
+        call("st_ray_picks_trial_misfit", self._h, vp.data_ptr(), gradient.data_ptr(), float(step), pr, float(vp_min),
+             float(vp_max), observed.data_ptr(), weights.data_ptr(), int(l1), C.byref(out))
+        return out.value
+
     def matrix(self) -> CSRMatrix:
         """The sampled-ray matrix (rows = picks, columns = cells, FP32 values
         ds * samples in the cell): A (1 / vp) = traveltimes where every

@@ -666,6 +666,18 @@ int st_ray_picks_forward_model(st_ray_picks* p, const double* vp, int on_device,
  * the reference's pick, then sample order (bit-exact as above). */
 int st_ray_picks_compute_gradient(st_ray_picks* p, const double* vp, const double* residuals, int on_device,
                                   double* gradient);
+/* Misfit of traveltimes (obs_data.py:116-129) on device arrays of n_picks
+ * values: 1/2 sum w (obs - t)^2, or with l1 sum w |obs - t|; the order of the
+ * sum depends on n_picks alone. Runs on the handle's stream and waits for it. */
+int st_ray_picks_misfit(st_ray_picks* p, const double* times, const double* obs, const double* weight, int l1,
+                        double* misfit);
+/* Misfit of the line search's trial model (inversion.py:436-453): vp - step *
+ * gradient (device, n_cells), clamped to policy_range[0..1] when given (not
+ * finite -> the lower bound) and then to vp_min .. vp_max, its traveltimes and
+ * st_ray_picks_misfit of them. Waits for the handle's stream. */
+int st_ray_picks_trial_misfit(st_ray_picks* p, const double* vp, const double* gradient, double step,
+                              const double* policy_range, double vp_min, double vp_max, const double* obs,
+                              const double* weight, int l1, double* misfit);
 /* The sampled-ray matrix of the picks as a CSR (rows = picks, columns =
  * cells, A[i, c] = ds_i * the number of samples of pick i in cell c, FP32),
  * so that A (1 / vp) gives the forward model wherever every velocity is
