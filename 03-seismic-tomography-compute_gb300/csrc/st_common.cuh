@@ -193,9 +193,10 @@ using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t
 int get_encode_tiled(EncodeTiledFn* out);
 
 // 4-D tensor map over a snapshot store of nt compact interior fields
-// [t][x][y][z] of `kind` with box {bz, by, 1, 1}; needs nz * element size to
-// be a multiple of 16 bytes (TMA stride rule).
-int make_snap_map(CUtensorMap* map, const void* base, int kind, const Layout& L, long long nt, int bz, int by);
+// [t][x][y][z] of `kind` with box {bz, by, 1, 1}; rows lie cz elements apart (0: nz),
+// cz * element size a multiple of 16 bytes (TMA stride rule).
+int make_snap_map(CUtensorMap* map, const void* base, int kind, const Layout& L, long long nt, int bz, int by,
+                  long long cz = 0);
 
 // Builds a 3-D FP32 tensor map over a device field of layout L with box
 // {bz, by, 1} (innermost first).

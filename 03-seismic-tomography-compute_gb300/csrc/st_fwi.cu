@@ -23,7 +23,7 @@
 namespace stg {
 
 int shot_forward_impl(st_solver* s, const st_shot* shot, float* seis, int snap_kind, void* snaps, unsigned* amax,
-                      bool slices = false);
+                      bool slices = false, int64_t cz = 0);
 
 namespace {
 

@@ -10,6 +10,7 @@ namespace stg {
 struct StepArgs {
     float* out;              // field written: the update at every interior point
     int nx, ny, nz, NZP;
+    int cz;                  // row pitch of the compact volumes (snapshots, image, illumination, gradient); 0: nz
     long long plane;
     int x_chunk;             // x-planes marched by one CTA
     float ax, ay, az;        // 1/dx^2, 1/dy^2, 1/dz^2
@@ -90,10 +91,11 @@ int fd_step_grid_chunks(const Layout& L, int tyv, int minb, int min_waves, int h
 struct ImageMaps {
     CUtensorMap snap, image, illum;
 };
-bool image_maps_supported(int kind, const Layout& L);
+// cz: the volumes' row pitch (0: nz).
+bool image_maps_supported(int kind, const Layout& L, long long cz = 0);
 int build_image_maps(ImageMaps* m, const void* snaps, int kind, long long nt, const float* image,
-                     const float* illum, const Layout& L);
-int make_compact_map(CUtensorMap* map, const float* base, const Layout& L, int bz, int by);
+                     const float* illum, const Layout& L, long long cz = 0);
+int make_compact_map(CUtensorMap* map, const float* base, const Layout& L, int bz, int by, long long cz = 0);
 
 // Launch one fused step. snap_out / snap_in are SnapKind values; epi: 0 = none,
 // 1 = imaging (operands staged by TMA when imaps is given, StepArgs::snap_t
@@ -107,7 +109,7 @@ int launch_fd_step(const Layout& L, const FieldMaps& mcur, const FieldMaps& mpre
 // output of step t) and a.out2 = the output of step t-1, from snapshots
 // a.snap_t and a.snap_t - 1 (scales a.amax_in, a.amax_in2) and the receiver
 // forcing rows a.force_row (step t) and a.force_row2 (step t-1). Needs
-// staged image maps (nz % 4 == 0).
+// staged image maps (image_maps_supported for a.cz).
 int launch_fd_step2_image(const Layout& L, const FieldMaps& mcur, const FieldMaps& mprev, const FieldMaps& mc,
                           StepArgs a, int snap_in, const ImageMaps& imaps, cudaStream_t st);
 // Launch two adjoint steps with the gradient epilogue (fd_step2_kernel,
@@ -122,7 +124,8 @@ int launch_fd_step2_grad(const Layout& L, const FieldMaps& mcur, const FieldMaps
 // samples a.seis_row / a.seis_row2; injects per a.inj_steps; with snapshots
 // stores u_t to a.snap_out (scale a.amax_cur) and u_{t-1} to a.snap_out2
 // (scale a.amax_cur2, when not null) and max-reduces |u_{t+1}|, |u_{t+2}|
-// into a.amax_next, a.amax_next2. Needs nz % 4 == 0.
+// into a.amax_next, a.amax_next2. With snapshots, needs a row pitch of a
+// multiple of 4.
 int launch_fd_step2_forward(const Layout& L, const FieldMaps& mcur, const FieldMaps& mprev, const FieldMaps& mc,
                             StepArgs a, int snap_out, cudaStream_t st);
 // 4-D map over a snapshot store for the gradient step's halo tile.
@@ -142,9 +145,11 @@ int launch_vel_to_coeff(const double* vel_ref, float* c, const Layout& L, double
 int launch_count_nonfinite(const float* f, long long n, unsigned long long* out, cudaStream_t st);
 int launch_sumsq_finite(const float* f, long long n, double* out, cudaStream_t st);
 int launch_interior_copy(const float* f, const Layout& L, float* out, cudaStream_t st);
-// Snapshot of field f (device layout) with scale amax, as the stepping kernels store it.
+// Snapshot of field f (device layout) with scale amax, as the stepping kernels store it (row pitch cz; 0: nz).
 int launch_snapshot_of_field(const float* f, const Layout& L, void* snap, int kind, const unsigned* amax,
-                             cudaStream_t st);
+                             cudaStream_t st, long long cz = 0);
+// dst [rows][nz] = the first nz values of every row of src [rows][cz].
+int launch_unpad_rows(const float* src, float* dst, long long rows, long long cz, long long nz, cudaStream_t st);
 int launch_finalize_image(const float* image, const float* illum, float* refl, long long n, cudaStream_t st);
 int launch_scatter_scaled(float* f, const long long* idx, int n, const float* val, const float* c,
                           cudaStream_t st);

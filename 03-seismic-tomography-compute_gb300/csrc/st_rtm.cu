@@ -91,9 +91,11 @@ int launch_rec_force(st_solver* s, const st_receiver_grid& R, const float* row) 
 
 // Forward shot (shared by st_shot_forward and the RTM / gradient drivers).
 // seis may be null (no sampling); snap_kind != NONE needs snaps and amax.
+// cz: the snapshot store's row pitch (0: nz).
 int shot_forward_impl(st_solver* s, const st_shot* shot, float* seis, int snap_kind, void* snaps, unsigned* amax,
-                      bool slices = false) {
+                      bool slices = false, int64_t cz = 0) {
     const Layout& L = s->L;
+    if (cz == 0) cz = L.nz;
     ST_CHECK(shot->src_ix >= 0 && shot->src_ix < L.nx && shot->src_iy >= 0 && shot->src_iy < L.ny &&
                  shot->src_iz >= 0 && shot->src_iz < L.nz,
              ST_ERR_ARG, "source outside the interior");
@@ -104,7 +106,7 @@ int shot_forward_impl(st_solver* s, const st_shot* shot, float* seis, int snap_k
     ST_TRY(refresh_coeff(s));
     ST_TRY(zero_fields(s));
     const int nt = shot->nt;
-    const size_t per = (size_t)(L.nx * L.ny * L.nz) * (size_t)snap_bytes(snap_kind);
+    const size_t per = (size_t)(L.nx * L.ny * cz) * (size_t)snap_bytes(snap_kind);
     if (snap_kind != SNAP_NONE) ST_CUDA(cudaMemsetAsync(amax, 0, sizeof(unsigned) * (size_t)(nt + 1), s->stream));
     const long long src = dev_index(s, shot->src_ix, shot->src_iy, shot->src_iz);
     float w = 0.0f;
@@ -114,17 +116,19 @@ int shot_forward_impl(st_solver* s, const st_shot* shot, float* seis, int snap_k
     // own (slice capture) or a terrain is attached; a pair leaves the snapshot
     // of its first output pending: the next pair stores it from its previous
     // field, a single step or the end of the pass stores it here
-    const bool pairs = s->fused_steps == 2 && !s->zlim && !(slices && s->slices) && L.nz % 4 == 0;
+    const bool pairs = s->fused_steps == 2 && !s->zlim && !(slices && s->slices) &&
+                       (snap_kind == SNAP_NONE || cz % 4 == 0);
     bool pending = false;
     auto store_pending = [&](int t) -> int {
         if (!pending) return ST_OK;
         pending = false;
         return launch_snapshot_of_field(s->f[s->ip], L, static_cast<char*>(snaps) + (size_t)(t - 1) * per,
-                                        snap_kind, amax + t - 1, s->stream);
+                                        snap_kind, amax + t - 1, s->stream, cz);
     };
     for (int t = 0; t < nt; ++t) {
         if (pairs && t + 1 < nt) {
             StepArgs a = base_args(s, nullptr);
+            a.cz = (int)cz;
             float w1 = 0.0f, w2 = 0.0f;
             const bool i1 = finite_sample(shot->wavelet, shot->wavelet_len, t + 1, &w1);
             const bool i2 = t + 2 < nt && finite_sample(shot->wavelet, shot->wavelet_len, t + 2, &w2);
@@ -155,6 +159,7 @@ int shot_forward_impl(st_solver* s, const st_shot* shot, float* seis, int snap_k
         }
         if (snap_kind != SNAP_NONE) ST_TRY(store_pending(t));
         StepArgs a = base_args(s, nullptr);
+        a.cz = (int)cz;
         float wn = 0.0f;
         if (t + 1 < nt && finite_sample(shot->wavelet, shot->wavelet_len, t + 1, &wn))
             set_injection(a, shot->src_ix, shot->src_iy, shot->src_iz, wn);
@@ -189,18 +194,20 @@ long long receiver_at(const st_receiver_grid& R, int64_t ix, int64_t iy, int64_t
 // epilogue runs (image/illum); with src_trace != null lambda at the source
 // is sampled after every step (the transpose of the wavelet -> data map).
 int rtm_backward_impl(st_solver* s, const st_shot* shot, const float* data, int snap_kind, const void* snaps,
-                      const unsigned* amax, float* image, float* illum, float* src_trace = nullptr) {
+                      const unsigned* amax, float* image, float* illum, float* src_trace = nullptr,
+                      int64_t cz = 0) {
     const Layout& L = s->L;
+    if (cz == 0) cz = L.nz;  // row pitch of the store, the image and the illumination
     const st_receiver_grid& R = shot->rec;
     const int64_t nrec = R.nx * R.ny;
     const int nt = shot->nt;
-    const size_t npts = (size_t)(L.nx * L.ny * L.nz);
+    const size_t npts = (size_t)(L.nx * L.ny * cz);
     const size_t per = npts * (size_t)snap_bytes(snap_kind);
     const bool imaging = snaps != nullptr;
     // the imaging operands ride the TMA ring when the store's rows allow it
     ImageMaps imaps;
-    const bool staged = imaging && image_maps_supported(snap_kind, L);
-    if (staged) ST_TRY(build_image_maps(&imaps, snaps, snap_kind, std::max(nt, 1), image, illum, L));
+    const bool staged = imaging && image_maps_supported(snap_kind, L, cz);
+    if (staged) ST_TRY(build_image_maps(&imaps, snaps, snap_kind, std::max(nt, 1), image, illum, L, cz));
     ST_TRY(zero_fields(s));
     if (imaging) {
         ST_CUDA(cudaMemsetAsync(image, 0, npts * sizeof(float), s->stream));
@@ -218,6 +225,7 @@ int rtm_backward_impl(st_solver* s, const st_shot* shot, const float* data, int 
     for (int t = nt - 1; t >= 0; --t) {
         if (pairs && t >= 1) {
             StepArgs a = base_args(s, nullptr);
+            a.cz = (int)cz;
             if (nrec > 0) {
                 set_receivers(a, R);
                 a.force_row = data + (size_t)(t - 1) * nrec;
@@ -233,6 +241,7 @@ int rtm_backward_impl(st_solver* s, const st_shot* shot, const float* data, int 
             continue;
         }
         StepArgs a = base_args(s, nullptr);
+        a.cz = (int)cz;
         if (nrec > 0 && t >= 1) {
             set_receivers(a, R);
             a.force_row = data + (size_t)(t - 1) * nrec;
@@ -309,11 +318,32 @@ static int rtm_shot_impl(st_solver* s, const st_shot* shot, const float* data, i
     const int64_t nrec = shot->rec.nx * shot->rec.ny;
     ST_CHECK(nrec == 0 || data, ST_ERR_ARG, "receiver data missing");
     ST_CUDA(cudaSetDevice(s->device));
-    const size_t npts = (size_t)(s->L.nx * s->L.ny * s->L.nz);
-    const size_t snap_total = npts * (size_t)snap_bytes(snap_kind) * (size_t)std::max(shot->nt, 1);
+    const size_t rows = (size_t)(s->L.nx * s->L.ny), npts = rows * (size_t)s->L.nz;
+    const size_t es = (size_t)snap_bytes(snap_kind), nsnap = (size_t)std::max(shot->nt, 1);
     unsigned* amax = snap_amax;
+    // A store of the library's own pads its rows to a multiple of 8 values where nz
+    // is none, and images into padded volumes beside it: the TMA can then stage
+    // every operand and two steps share a launch, where rows that are not multiples
+    // of 16 bytes leave one step per launch with its operands loaded at use
+    // (150 x 203 x 171, FP16: 89 us per adjoint step and 30 per forward step). A
+    // caller's store keeps its rows; so does a pass that captures slices of it, and
+    // one for which the padding does not fit.
+    int64_t cz = s->L.nz;
+    float *im = image, *il = illum;
     if (!snaps) {
-        ST_TRY(ensure_buffer(s, &s->snap_buf, &s->snap_cap, snap_total));
+        if (!image_maps_supported(snap_kind, s->L) && s->fused_steps == 2 && !s->slices) {
+            const int64_t pz = (s->L.nz + 7) / 8 * 8;
+            const size_t store = (rows * (size_t)pz * es * nsnap + 255) / 256 * 256;
+            const size_t vol = (rows * (size_t)pz * sizeof(float) + 255) / 256 * 256;
+            if (ensure_buffer(s, &s->snap_buf, &s->snap_cap, store + 2 * vol) == ST_OK) {
+                cz = pz;
+                im = reinterpret_cast<float*>(static_cast<char*>(s->snap_buf) + store);
+                il = reinterpret_cast<float*>(static_cast<char*>(s->snap_buf) + store + vol);
+            } else {
+                cudaGetLastError();
+            }
+        }
+        if (cz == s->L.nz) ST_TRY(ensure_buffer(s, &s->snap_buf, &s->snap_cap, npts * es * nsnap));
         snaps = s->snap_buf;
     }
     if (!amax) {
@@ -321,10 +351,14 @@ static int rtm_shot_impl(st_solver* s, const st_shot* shot, const float* data, i
         amax = static_cast<unsigned*>(s->aux_buf);
     }
     ST_CUDA(cudaEventRecord(s->ev[0], s->stream));
-    ST_TRY(shot_forward_impl(s, shot, nullptr, snap_kind, snaps, amax));
+    ST_TRY(shot_forward_impl(s, shot, nullptr, snap_kind, snaps, amax, false, cz));
     ST_CUDA(cudaEventRecord(s->ev[1], s->stream));
     if (data_ready) ST_CUDA(cudaStreamWaitEvent(s->stream, data_ready, 0));
-    ST_TRY(rtm_backward_impl(s, shot, data, snap_kind, snaps, amax, image, illum));
+    ST_TRY(rtm_backward_impl(s, shot, data, snap_kind, snaps, amax, im, il, nullptr, cz));
+    if (im != image) {
+        ST_TRY(launch_unpad_rows(im, image, (long long)rows, cz, s->L.nz, s->stream));
+        ST_TRY(launch_unpad_rows(il, illum, (long long)rows, cz, s->L.nz, s->stream));
+    }
     ST_CUDA(cudaEventRecord(s->ev[2], s->stream));
     s->phases_recorded = 1;
     if (refl) ST_TRY(launch_finalize_image(image, illum, refl, (long long)npts, s->stream));
@@ -347,7 +381,6 @@ int st_rtm_shot_host(st_solver* s, const double* vp, int64_t vp_count, const st_
     const int64_t nrec = shot->rec.nx * shot->rec.ny;
     const size_t npts = (size_t)(s->L.nx * s->L.ny * s->L.nz);
     const size_t dbytes = (size_t)nrec * (size_t)std::max(shot->nt, 0) * sizeof(float);
-    const size_t snap_total = npts * (size_t)snap_bytes(snap_kind) * (size_t)std::max(shot->nt, 1);
     // aux layout: amax[nt+1] | image | illum | refl | fp64 out
     const size_t amax_bytes = ((sizeof(unsigned) * (size_t)(shot->nt + 1) + 255) / 256) * 256;
     const size_t img_bytes = ((npts * sizeof(float) + 255) / 256) * 256;
@@ -358,7 +391,6 @@ int st_rtm_shot_host(st_solver* s, const double* vp, int64_t vp_count, const st_
     float* illum = reinterpret_cast<float*>(aux + amax_bytes + img_bytes);
     float* refl = reinterpret_cast<float*>(aux + amax_bytes + 2 * img_bytes);
     double* out64 = reinterpret_cast<double*>(aux + amax_bytes + 3 * img_bytes);
-    ST_TRY(ensure_buffer(s, &s->snap_buf, &s->snap_cap, snap_total));
     float* data = nullptr;
     cudaEvent_t data_ready = nullptr;
     if (dbytes > 0) {
@@ -376,7 +408,7 @@ int st_rtm_shot_host(st_solver* s, const double* vp, int64_t vp_count, const st_
         ST_CUDA(cudaEventRecord(s->ev_copy, s->copy_stream));
         data_ready = s->ev_copy;
     }
-    int rc = rtm_shot_impl(s, shot, data, snap_kind, s->snap_buf, amax, image, illum, refl, data_ready);
+    int rc = rtm_shot_impl(s, shot, data, snap_kind, nullptr, amax, image, illum, refl, data_ready);
     if (rc < 0 && s->copy_stream) cudaStreamSynchronize(s->copy_stream);
     if (rc < 0) return rc;
     const float* srcs[3] = {image, illum, refl};

@@ -296,7 +296,7 @@ __device__ __forceinline__ void process_row(const StepArgs& a, const RowCtx& R, 
     }
     if constexpr (EPI == EPI_MASK) {  // terrain masks: the column's points above its z limit hold 0
         const long long col = (long long)x * a.ny + R.iy;
-        const int zl = a.zlim[col] - (int)(cbase - col * a.nz);
+        const int zl = a.zlim[col] - (int)(cbase - col * a.cz);
 #pragma unroll
         for (int k = 0; k < 4; ++k)
             if (k < zl) res[k] = 0.0f;
@@ -321,7 +321,7 @@ __device__ __forceinline__ void process_row(const StepArgs& a, const RowCtx& R, 
         float q[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) q[k] = u0[k] * snap_inv;
-        if (zvalid == 4 && (a.nz & 3) == 0) {
+        if (zvalid == 4 && (a.cz & 3) == 0) {
             snap_store4<SNAP_OUT>(a.snap_out, cbase, q);
         } else {
             for (int k = 0; k < zvalid; ++k) snap_store<SNAP_OUT>(a.snap_out, cbase + k, q[k]);
@@ -431,7 +431,7 @@ __global__ void __launch_bounds__(NTHREADS, (Geo<EPI, SNAP_IN>::MINB))
         snap_inv = m > 0.0f ? SNAP_QMAX / m : 0.0f;
     }
     float snap_scale = 1.0f;
-    const bool vec_acc = !is_forward(EPI) && (a.nz & 3) == 0 && zvalid == 4;
+    const bool vec_acc = !is_forward(EPI) && (a.cz & 3) == 0 && zvalid == 4;
     if constexpr (!is_forward(EPI)) snap_scale = __uint_as_float(*a.amax_in) / SNAP_QMAX;
 
     const bool tab_smem = a.sw <= DTAB_MAX;
@@ -507,8 +507,8 @@ __global__ void __launch_bounds__(NTHREADS, (Geo<EPI, SNAP_IN>::MINB))
     auto prefetch = [&](int x) {
         if constexpr (EPI == EPI_IMAGE || EPI == EPI_GRAD) {
             if (!vec_acc || x >= xb) return;
-            const long long ca = ((long long)x * a.ny + RA.iy) * a.nz + iz0;
-            const long long cb = ca + a.nz;
+            const long long ca = ((long long)x * a.ny + RA.iy) * a.cz + iz0;
+            const long long cb = ca + a.cz;
             if constexpr (EPI == EPI_IMAGE) {
                 if (RA.active) {
                     snA = snap_raw4<SNAP_IN>(a.snap_in, ca);
@@ -579,7 +579,7 @@ __global__ void __launch_bounds__(NTHREADS, (Geo<EPI, SNAP_IN>::MINB))
                 if (xx >= 0 && xx % a.rsx == 0 && xx / a.rsx < a.rnx) irx = xx / a.rsx;
             }
             const long long obA = (long long)(x + 1) * a.plane + (long long)(RA.iy + 1) * a.NZP + iz0 + Layout::ZOFF;
-            const long long cbA = ((long long)x * a.ny + RA.iy) * a.nz + iz0;
+            const long long cbA = ((long long)x * a.ny + RA.iy) * a.cz + iz0;
             float finA[4] = {0, 0, 0, 0}, finB[4] = {0, 0, 0, 0};
             if constexpr (!kPrefetch) prefetch(x);  // operands of this plane, at use
             if constexpr (EPI == EPI_IMAGE_T) {
@@ -630,7 +630,7 @@ __global__ void __launch_bounds__(NTHREADS, (Geo<EPI, SNAP_IN>::MINB))
             if constexpr (RPT == 2)
                 process_row<SNAP_OUT, SNAP_IN, EPI>(a, RB, x, zvalid, dz, zfar, dxx, dtab, umB, u0B, upB, u0A, ypB,
                                                     zmB, zpB, pvB, cvB, rk, irx, inj_k, snap_inv, amax_local, &fired,
-                                                    obA + a.NZP, cbA + a.nz, finB, a0B0, a1B0, vec_acc);
+                                                    obA + a.NZP, cbA + a.cz, finB, a0B0, a1B0, vec_acc);
         } else if constexpr (EPI == EPI_GRAD) {
             if (i == 1) {
                 // snapshot centres of plane xa-1 (zero outside the domain)
@@ -878,7 +878,11 @@ struct PlaneKind {
     static constexpr int PA = PA_, PB = PB_;
 };
 
-template <int MODE, int SK>
+// RAG: nz is not a multiple of 4, so the last group of a row reaches past the
+// grid; the points beyond it hold 0 (they are stored, into the field's zero halo
+// and the compact rows' padding). A variant of its own: the masks tested at run
+// time cost the aligned grids 1-10%.
+template <int MODE, int SK, bool RAG>
 __global__ void __launch_bounds__(NTHREADS, (Geo2<MODE, SK>::MINB))
     fd_step2_kernel(const __grid_constant__ CUtensorMap map_cur, const __grid_constant__ CUtensorMap map_prev,
                     const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_snap,
@@ -921,6 +925,8 @@ __global__ void __launch_bounds__(NTHREADS, (Geo2<MODE, SK>::MINB))
     const int zc = z0 + 4 * tz4;
     const int yc = y0 + yr;
     const bool cin = yc < a.ny && zc < a.nz;
+    const int zin = a.nz - zc;
+    (void)zin;
     constexpr int NRING = 2 * TZ + 2 * G::TYV;
     static_assert(NRING <= NTHREADS, "one ring point per thread");
     const bool has_ring = tid < NRING;
@@ -1066,8 +1072,9 @@ __global__ void __launch_bounds__(NTHREADS, (Geo2<MODE, SK>::MINB))
     int s = 0, sp = STAGES - 1;
     unsigned parity = 0;
     long long ob = (long long)(xa + 1) * a.plane + (long long)(yc + 1) * a.NZP + zc + Layout::ZOFF;
-    long long cb = ((long long)xa * a.ny + yc) * a.nz + zc;
-    const long long cplane = (long long)a.ny * a.nz;
+    const int cz = RAG ? a.cz : a.nz;  // an aligned grid's rows are never padded
+    long long cb = ((long long)xa * a.ny + yc) * cz + zc;
+    const long long cplane = (long long)a.ny * cz;
     int i = 0;
     // one plane; q0 / q1 / q2 are the queue slots of planes i-2 / i-1 / i
     // (for the u' queue: i-3 / i-2 / i-1); returns true when a wait gave up
@@ -1150,6 +1157,13 @@ __global__ void __launch_bounds__(NTHREADS, (Geo2<MODE, SK>::MINB))
                                 if (k == inj_kc) lp[k] += a.inj_val;
                         }
                     }
+                }
+                if constexpr (RAG) {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        if (k >= zin) lp[k] = 0.0f;
+                }
+                if constexpr (FWD) {
                     if constexpr (SNAPS) {
                         if (own) {
                             // plane x = xa - 3 + i: one plane past sub-step B's (cb),
@@ -1226,6 +1240,13 @@ __global__ void __launch_bounds__(NTHREADS, (Geo2<MODE, SK>::MINB))
                             if (k == inj_kc) res[k] += a.inj_val2;
                     }
                 }
+            }
+            if constexpr (RAG) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (k >= zin) res[k] = 0.0f;
+            }
+            if constexpr (FWD) {
                 if constexpr (SNAPS) {
 #pragma unroll
                     for (int k = 0; k < 4; ++k) amax2 = fmaxf(amax2, fabsf(res[k]));
@@ -1408,8 +1429,8 @@ __global__ void __launch_bounds__(NTHREADS, (Geo2<MODE, SK>::MINB))
     }
 }
 
-template <int MODE, int SK>
-int launch_step2_variant(const Layout& L, const FieldMaps& mcur, const FieldMaps& mprev, const FieldMaps& mc,
+template <int MODE, int SK, bool RAG>
+int launch_step2_rows(const Layout& L, const FieldMaps& mcur, const FieldMaps& mprev, const FieldMaps& mc,
                          const ImageMaps* im, StepArgs a, cudaStream_t st) {
     using G = Geo2<MODE, SK>;
     static bool configured = false;
@@ -1417,7 +1438,7 @@ int launch_step2_variant(const Layout& L, const FieldMaps& mcur, const FieldMaps
     {
         std::lock_guard<std::mutex> lk(mu);
         if (!configured) {
-            ST_CUDA(cudaFuncSetAttribute(fd_step2_kernel<MODE, SK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            ST_CUDA(cudaFuncSetAttribute(fd_step2_kernel<MODE, SK, RAG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          G::SMEM));
             configured = true;
         }
@@ -1430,10 +1451,19 @@ int launch_step2_variant(const Layout& L, const FieldMaps& mcur, const FieldMaps
     const CUtensorMap& ms = im ? im->snap : mc.cur[0];
     const CUtensorMap& mi = im ? im->image : mc.cur[0];
     const CUtensorMap& ml = im ? im->illum : mc.cur[0];
-    fd_step2_kernel<MODE, SK><<<grid, NTHREADS, G::SMEM, st>>>(mcur.cur2, mprev.cur[0], mc.cur[0], ms, mi, ml, a);
+    fd_step2_kernel<MODE, SK, RAG><<<grid, NTHREADS, G::SMEM, st>>>(mcur.cur2, mprev.cur[0], mc.cur[0], ms, mi, ml, a);
     ::stg::count_launch();
     ST_CUDA(cudaGetLastError());
     return ST_OK;
+}
+
+template <int MODE, int SK>
+int launch_step2_variant(const Layout& L, const FieldMaps& mcur, const FieldMaps& mprev, const FieldMaps& mc,
+                         const ImageMaps* im, StepArgs a, cudaStream_t st) {
+    if constexpr (MODE != MODE_GRAD)  // gradients take aligned rows only
+        if (a.cz != a.nz || a.nz % 4 != 0)
+            return launch_step2_rows<MODE, SK, true>(L, mcur, mprev, mc, im, a, st);
+    return launch_step2_rows<MODE, SK, false>(L, mcur, mprev, mc, im, a, st);
 }
 
 int num_sms() {
@@ -1580,7 +1610,7 @@ __global__ void sumsq_finite_kernel(const float* __restrict__ f, long long n, do
 // field: v * (16384 / |max|) rounded to the store's kind, compact interior.
 template <int K>
 __global__ void snapshot_of_field_kernel(const float* __restrict__ f, Layout L, void* snap,
-                                         const unsigned* amax) {
+                                         const unsigned* amax, long long cz) {
     const float m = __uint_as_float(*amax);
     const float inv = m > 0.0f ? SNAP_QMAX / m : 0.0f;
     const long long total = L.nx * L.ny * L.nz;
@@ -1590,8 +1620,15 @@ __global__ void snapshot_of_field_kernel(const float* __restrict__ f, Layout L, 
         const long long r = e - ix * (L.ny * L.nz);
         const long long iy = r / L.nz;
         const long long iz = r - iy * L.nz;
-        snap_store<K>(snap, e, f[L.at(ix, iy, iz)] * inv);
+        snap_store<K>(snap, (ix * L.ny + iy) * cz + iz, f[L.at(ix, iy, iz)] * inv);
     }
+}
+
+__global__ void unpad_rows_kernel(const float* __restrict__ src, float* __restrict__ dst, long long rows, long long cz,
+                                  long long nz) {
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < rows * nz;
+         e += (long long)gridDim.x * blockDim.x)
+        dst[e] = src[e / nz * cz + e % nz];
 }
 
 __global__ void interior_copy_kernel(const float* __restrict__ f, Layout L, float* __restrict__ out) {
@@ -1674,6 +1711,7 @@ int launch_fd_step(const Layout& L, const FieldMaps& mcur, const FieldMaps& mpre
     a.nz = (int)L.nz;
     a.NZP = (int)L.NZP;
     a.plane = L.plane;
+    if (a.cz == 0) a.cz = a.nz;
     if (a.timeout_ns == 0) a.timeout_ns = 2000000000ull;
     ST_CHECK(!a.zlim || epi == EPI_NONE, ST_ERR_UNSUPPORTED, "terrain limits apply to plain forward steps only");
     const CUtensorMap& ms = msnap ? *msnap : mc.ctr[0];  // unused unless epi == gradient
@@ -1736,8 +1774,9 @@ int launch_fd_step2_image(const Layout& L, const FieldMaps& mcur, const FieldMap
     a.nz = (int)L.nz;
     a.NZP = (int)L.NZP;
     a.plane = L.plane;
+    if (a.cz == 0) a.cz = a.nz;
     if (a.timeout_ns == 0) a.timeout_ns = 2000000000ull;
-    ST_CHECK(image_maps_supported(snap_in, L), ST_ERR_UNSUPPORTED, "two-step imaging needs staged image maps");
+    ST_CHECK(image_maps_supported(snap_in, L, a.cz), ST_ERR_UNSUPPORTED, "two-step imaging needs staged image maps");
     ST_CHECK(a.out && a.out2 && a.image && a.illum && a.amax_in && a.amax_in2 && a.snap_t >= 1, ST_ERR_ARG,
              "two-step imaging: missing operands");
     ST_CHECK(!a.zlim && !a.seis_row && !a.snap_out && a.inj_x < 0, ST_ERR_UNSUPPORTED,
@@ -1758,6 +1797,7 @@ int launch_fd_step2_grad(const Layout& L, const FieldMaps& mcur, const FieldMaps
     a.nz = (int)L.nz;
     a.NZP = (int)L.NZP;
     a.plane = L.plane;
+    if (a.cz == 0) a.cz = a.nz;
     if (a.timeout_ns == 0) a.timeout_ns = 2000000000ull;
     ST_CHECK(L.nz % 4 == 0, ST_ERR_UNSUPPORTED, "two-step gradient needs nz %% 4 == 0");
     ST_CHECK(a.out && a.out2 && a.grad && a.amax_in && a.amax_in2 && a.snap_t >= 1, ST_ERR_ARG,
@@ -1783,11 +1823,13 @@ int launch_fd_step2_forward(const Layout& L, const FieldMaps& mcur, const FieldM
     a.nz = (int)L.nz;
     a.NZP = (int)L.NZP;
     a.plane = L.plane;
+    if (a.cz == 0) a.cz = a.nz;
     if (a.timeout_ns == 0) a.timeout_ns = 2000000000ull;
     ST_CHECK(a.out && a.out2, ST_ERR_ARG, "two-step forward: missing outputs");
     ST_CHECK(!a.zlim && !a.force_row && !a.force_row2 && !a.image && !a.grad, ST_ERR_UNSUPPORTED,
              "two-step forward: forward steps without terrain only");
-    ST_CHECK(L.nz % 4 == 0, ST_ERR_UNSUPPORTED, "two-step forward needs nz %% 4 == 0");
+    ST_CHECK(snap_out == SNAP_NONE || a.cz % 4 == 0, ST_ERR_UNSUPPORTED,
+             "two-step forward snapshots need rows of a multiple of 4 values");
     ST_CHECK(snap_out == SNAP_NONE || (a.snap_out && a.amax_cur && a.amax_next && a.amax_next2 &&
                                        (!a.snap_out2 || a.amax_cur2)),
              ST_ERR_ARG, "two-step forward: missing snapshot operands");
@@ -1801,28 +1843,30 @@ int launch_fd_step2_forward(const Layout& L, const FieldMaps& mcur, const FieldM
 }
 
 int build_image_maps(ImageMaps* m, const void* snaps, int kind, long long nt, const float* image,
-                     const float* illum, const Layout& L) {
-    ST_CHECK(image_maps_supported(kind, L), ST_ERR_UNSUPPORTED, "staged imaging needs nz * %d bytes divisible by 16",
+                     const float* illum, const Layout& L, long long cz) {
+    ST_CHECK(image_maps_supported(kind, L, cz), ST_ERR_UNSUPPORTED, "staged imaging needs rows of a multiple of 16 bytes (%d a value)",
              snap_bytes(kind));
-    ST_TRY(make_snap_map(&m->snap, snaps, kind, L, nt, TZ, 16));
-    ST_TRY(make_compact_map(&m->image, image, L, TZ, 16));
-    ST_TRY(make_compact_map(&m->illum, illum, L, TZ, 16));
+    ST_TRY(make_snap_map(&m->snap, snaps, kind, L, nt, TZ, 16, cz));
+    ST_TRY(make_compact_map(&m->image, image, L, TZ, 16, cz));
+    ST_TRY(make_compact_map(&m->illum, illum, L, TZ, 16, cz));
     return ST_OK;
 }
 
-bool image_maps_supported(int kind, const Layout& L) {
+bool image_maps_supported(int kind, const Layout& L, long long cz) {
     const int es = snap_bytes(kind);
-    return es > 0 && (L.nz * es) % 16 == 0 && (L.nz % 4) == 0;
+    if (cz == 0) cz = L.nz;
+    return es > 0 && (cz * es) % 16 == 0 && (cz % 4) == 0;
 }
 
 // 3-D map over a compact interior FP32 volume [nx][ny][nz], box {bz, by, 1}.
-int make_compact_map(CUtensorMap* map, const float* base, const Layout& L, int bz, int by) {
+int make_compact_map(CUtensorMap* map, const float* base, const Layout& L, int bz, int by, long long cz) {
+    if (cz == 0) cz = L.nz;
     EncodeTiledFn enc = nullptr;
     ST_TRY(get_encode_tiled(&enc));
     ST_CHECK((reinterpret_cast<uintptr_t>(base) & 15) == 0, ST_ERR_ARG, "volume base not 16-byte aligned");
-    ST_CHECK((L.nz * 4) % 16 == 0, ST_ERR_ARG, "compact volume rows must be multiples of 16 bytes");
+    ST_CHECK((cz * 4) % 16 == 0, ST_ERR_ARG, "compact volume rows must be multiples of 16 bytes");
     cuuint64_t dims[3] = {(cuuint64_t)L.nz, (cuuint64_t)L.ny, (cuuint64_t)L.nx};
-    cuuint64_t strides[2] = {(cuuint64_t)L.nz * 4, (cuuint64_t)(L.ny * L.nz) * 4};
+    cuuint64_t strides[2] = {(cuuint64_t)cz * 4, (cuuint64_t)(L.ny * cz) * 4};
     cuuint32_t box[3] = {(cuuint32_t)bz, (cuuint32_t)by, 1};
     cuuint32_t estr[3] = {1, 1, 1};
     CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(base), dims, strides, box, estr,
@@ -1909,14 +1953,22 @@ int launch_sumsq_finite(const float* f, long long n, double* out, cudaStream_t s
 }
 
 int launch_snapshot_of_field(const float* f, const Layout& L, void* snap, int kind, const unsigned* amax,
-                             cudaStream_t st) {
+                             cudaStream_t st, long long cz) {
     const int g = grid_for(L.nx * L.ny * L.nz);
+    if (cz == 0) cz = L.nz;
     switch (kind) {
-        case SNAP_BF16: snapshot_of_field_kernel<SNAP_BF16><<<g, 256, 0, st>>>(f, L, snap, amax); break;
-        case SNAP_FP16: snapshot_of_field_kernel<SNAP_FP16><<<g, 256, 0, st>>>(f, L, snap, amax); break;
-        case SNAP_FP32: snapshot_of_field_kernel<SNAP_FP32><<<g, 256, 0, st>>>(f, L, snap, amax); break;
+        case SNAP_BF16: snapshot_of_field_kernel<SNAP_BF16><<<g, 256, 0, st>>>(f, L, snap, amax, cz); break;
+        case SNAP_FP16: snapshot_of_field_kernel<SNAP_FP16><<<g, 256, 0, st>>>(f, L, snap, amax, cz); break;
+        case SNAP_FP32: snapshot_of_field_kernel<SNAP_FP32><<<g, 256, 0, st>>>(f, L, snap, amax, cz); break;
         default: ST_CHECK(false, ST_ERR_ARG, "bad snapshot kind %d", kind);
     }
+    ::stg::count_launch();
+    ST_CUDA(cudaGetLastError());
+    return ST_OK;
+}
+
+int launch_unpad_rows(const float* src, float* dst, long long rows, long long cz, long long nz, cudaStream_t st) {
+    unpad_rows_kernel<<<grid_for(rows * nz), 256, 0, st>>>(src, dst, rows, cz, nz);
     ::stg::count_launch();
     ST_CUDA(cudaGetLastError());
     return ST_OK;
@@ -1961,20 +2013,22 @@ int get_encode_tiled(EncodeTiledFn* out) {
     return ST_OK;
 }
 
-int make_snap_map(CUtensorMap* map, const void* base, int kind, const Layout& L, long long nt, int bz, int by) {
+int make_snap_map(CUtensorMap* map, const void* base, int kind, const Layout& L, long long nt, int bz, int by,
+                  long long cz) {
+    if (cz == 0) cz = L.nz;
     EncodeTiledFn enc = nullptr;
     ST_TRY(get_encode_tiled(&enc));
     const int es = snap_bytes(kind);
     ST_CHECK(es > 0, ST_ERR_ARG, "bad snapshot kind %d", kind);
     ST_CHECK((reinterpret_cast<uintptr_t>(base) & 15) == 0, ST_ERR_ARG, "snapshot store not 16-byte aligned");
-    ST_CHECK((L.nz * es) % 16 == 0, ST_ERR_UNSUPPORTED,
+    ST_CHECK((cz * es) % 16 == 0, ST_ERR_UNSUPPORTED,
              "gradient snapshots need nz*%d bytes to be a multiple of 16 (nz=%lld)", es, (long long)L.nz);
     const CUtensorMapDataType dt = kind == SNAP_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
                                    : kind == SNAP_FP16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
                                                        : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
     cuuint64_t dims[4] = {(cuuint64_t)L.nz, (cuuint64_t)L.ny, (cuuint64_t)L.nx, (cuuint64_t)std::max<long long>(nt, 1)};
-    cuuint64_t strides[3] = {(cuuint64_t)(L.nz * es), (cuuint64_t)(L.ny * L.nz * es),
-                             (cuuint64_t)(L.nx * L.ny * L.nz * es)};
+    cuuint64_t strides[3] = {(cuuint64_t)(cz * es), (cuuint64_t)(L.ny * cz * es),
+                             (cuuint64_t)(L.nx * L.ny * cz * es)};
     cuuint32_t box[4] = {(cuuint32_t)bz, (cuuint32_t)by, 1, 1};
     cuuint32_t estr[4] = {1, 1, 1, 1};
     CUresult r = enc(map, dt, 4, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
