@@ -11,24 +11,45 @@
 // in[rows + s][128 x 32] . W_tap[32 x 32]^T: an implicit GEMM with M = 128
 // voxels, N = 32 output channels and K = 27 x 32.
 //
-// Data path per CTA (persistent, one per SM, 6 warps). The work is cut into
-// units: one in-plane tile position (128 rows) for a run of consecutive
-// planes d0..d1-1, so a CTA marches along d and every plane window it loads
-// serves three consecutive tiles (taps kd = 2, 1, 0):
-//   warp 0  TMA producer: loads the 128 + 2(W+3)-row window of each plane the
-//           unit needs (d0 .. d1+1 in padded planes) as 16-byte channel-block
-//           columns ([cb][row][8 channels], no swizzle) into a ring of four
-//           window slots, a slot refilled once its last tile's MMAs are done;
-//   warp 1  allocates 64 TMEM columns (two FP32 accumulators of 128 x 32) and
-//           issues 54 tcgen05.mma.kind::f16 (BF16 x BF16 -> FP32, M=128,
-//           N=32, K=16) per tile: every tap is a 16-byte-aligned start row
-//           inside the windows, read in the canonical no-swizzle K-major
-//           layout (8-row x 16-byte core matrices: LBO = channel-block
-//           stride, SBO = 128 bytes); the weights (55,296 bytes, packed in the
-//           same layout) stay resident in shared memory;
-//   warps 2-5  epilogue: tcgen05.ld of the accumulator, + bias, + optional
-//           residual input, optional ReLU, BF16 (or FP32) store of the row,
-//           zero on border rows so the output keeps the padded convention.
+// Layout of the contraction. With the voxels as the matrix unit's 128 rows and
+// the 32 output channels as its columns, every instruction reads 4 KB of voxels
+// from shared memory for 32 columns: the operand feed, not the multiply, set the
+// pace (0.129 ms on a 100^3 volume, the multiply unit busy 18.5%). So the weights
+// are the M operand and the voxels the N operand, and the three depth taps are
+// stacked along M: one instruction multiplies N voxels of input plane p (shifted
+// by one in-plane tap) by the 32 x 32 weights of kd = 2, 1, 0 for the output planes
+// p - 1, p, p + 1. Output plane q lives in TMEM lanes 32 (q mod 4) .. + 31 (lane =
+// channel, column = voxel), so a plane's three contributions meet in its block as
+// the CTA marches along depth, and each input plane is read once. 100^3: 0.069 ms,
+// 802 TFLOP/s (40% of BF16; a quarter of the M rows is disabled, and at 256 voxels
+// the instruction's operands take three quarters of the shared-memory bandwidth
+// that the epilogue needs as well); 32^3: 13 us, mostly start and end. The M rows are a
+// window of four 32-row blocks into [kd2 kd1 kd0 - kd2 kd1 kd0], started at the
+// block that puts kd2 on plane p - 1; the lanes of the fourth block, and of
+// planes outside the CTA's range, are disabled for the instruction.
+//
+// Data path per CTA (persistent, one per SM, 18 warps). The work is cut into
+// units: one in-plane tile position (N voxels) for a run of consecutive planes
+// d0..d1-1, marched over the input planes d0-1..d1:
+//   warp 0  loads per input plane the N + 2(W+3)-row
+//           window ([row][32 channels], 64-byte swizzled: one copy of whole rows,
+//           where 16-byte channel-block columns made the copy engine the bound at
+//           four requests a row) into a ring of window slots;
+//   warp 1  allocates N TMEM columns and issues 18 tcgen05.mma.kind::f16 (9
+//           in-plane taps x 2 K steps; BF16 x BF16 -> FP32, M = 128, K = 16) per
+//           input plane: every tap is a start row inside the window (the swizzle
+//           goes by the address, and eight rows follow eight rows at 512 bytes);
+//           the weights lie in the canonical no-swizzle K-major layout (8-row x
+//           16-byte core matrices);
+//   warps 2-17 epilogue, four warps per lane quarter (= block): when an output
+//           plane is complete they read its block (tcgen05.ld), write zeros
+//           back for the plane that takes the block next, and then, while the
+//           matrix unit goes on, turn four voxels at a time through shared memory
+//           (lane = channel in, four channels of a voxel out): + optional residual
+//           input, + bias, optional ReLU, BF16 (or FP32) store of 8-byte pieces, zero
+//           on border rows so the output keeps the padded convention. (Pairs of
+//           channels exchanged by shuffles took four times the instructions and set
+//           the pace: 82 us at 100^3.)
 // Every mbarrier wait is bounded by a %globaltimer deadline: on expiry the
 // kernel records CONV_FLAG_TIMEOUT, drains its own copies and MMAs (bounded
 // too), frees TMEM and returns.
@@ -43,14 +64,16 @@ namespace {
 constexpr int CH = 32;
 constexpr int TM = 128;
 constexpr int NTAP = 27;
-constexpr int W_BYTES = NTAP * CH * CH * 2;  // 55,296: [tap][cb][co][8 ci]
-// plane-window slots: three in use by a tile, the rest loading ahead; the
-// host takes MAX_SLOT where it fits in shared memory, else MIN_SLOT (six
-// measured 3% faster than four on a 100^3 volume, eight no faster than six)
-constexpr int MIN_SLOT = 4, MAX_SLOT = 6;
-constexpr int CONV_THREADS = 192;
-constexpr int TMEM_COLS = 64;
-constexpr int SMEM_LIMIT = 232448 - 1024;
+constexpr int WB_BLOCK = CH * 16;                // 512 B: 32 output channels x 8 input channels
+constexpr int WB_CB = 7 * WB_BLOCK;              // one channel block: kd2 kd1 kd0 - kd2 kd1 kd0
+constexpr int WB_TAP = 4 * WB_CB;                // one in-plane tap
+constexpr int W_BYTES = 9 * WB_TAP;              // 129,024
+constexpr int MAX_SLOT = 3;
+constexpr int MAX_WIDTH = 269;
+constexpr int STAGE_FLOATS = 4 * CH;             // four voxels per epilogue warp (small: the windows want the room)
+constexpr int EPI_WARPS = 16;                    // four per lane quarter
+constexpr int CONV_THREADS = 64 + 32 * EPI_WARPS;
+constexpr int SMEM_LIMIT = 232448;
 constexpr unsigned CONV_FLAG_TIMEOUT = 1u;
 
 struct ConvArgs {
@@ -62,6 +85,7 @@ struct ConvArgs {
     int D, H, W;
     int relu;
     int rows_box, nload;    // TMA box rows and boxes per window column
+    int nslot;              // window slots
     int tiles_per_plane;    // in-plane tile positions (units' columns)
     int dchunk, units;      // planes per unit, units = tiles_per_plane * ceil(D / dchunk)
     unsigned* flags;
@@ -82,14 +106,6 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, u
         : "memory");
 }
 
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned bytes, uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-            smem_u32(dst)),
-        "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(smem_u32(bar))
-        : "memory");
-}
-
 // Shared-memory matrix descriptor, canonical K-major layout without swizzle:
 // start address, leading (K-direction) and stride (M/N-direction) byte
 // offsets between 8-row x 16-byte core matrices, descriptor version 1.
@@ -98,9 +114,18 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
            ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
 
+// The same for K-major rows of 64 bytes, 64-byte swizzled, eight rows every 512
+// bytes.
+__device__ __forceinline__ uint64_t smem_desc_sw64(uint32_t addr) {
+    return (uint64_t)((addr & 0x3FFFFu) >> 4) | (1ull << 16) | ((uint64_t)(512u >> 4) << 32) | (1ull << 46) | (4ull << 61);
+}
+
 // Instruction descriptor of kind::f16: FP32 accumulator, BF16 A and B, both
-// K-major, N = 32, M = 128.
-constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(CH >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
+// K-major, M = 128.
+constexpr uint32_t idesc_n(int n) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
+}
+constexpr uint32_t IDESC = idesc_n(CH);
 
 __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
     asm volatile(
@@ -108,6 +133,25 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
         "l"(adesc), "l"(bdesc), "r"(IDESC), "r"(accumulate)
         : "memory");
+}
+
+// Accumulating form that leaves the TMEM lanes set in off[] as they are; the
+// descriptors as low and high words.
+__device__ __forceinline__ void mma_bf16_lanes(uint32_t tmem_d, uint32_t alo, uint32_t ahi, uint32_t blo, uint32_t bhi,
+                                               uint32_t idesc, const uint32_t off[4]) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, 1, 0;\n\tmov.b64 da, {%1, %2};\n\t"
+        "mov.b64 db, {%3, %4};\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, {%6, %7, %8, %9}, p;\n\t}" ::"r"(tmem_d),
+        "r"(alo), "r"(ahi), "r"(blo), "r"(bhi), "r"(idesc), "r"(off[0]), "r"(off[1]), "r"(off[2]), "r"(off[3])
+        : "memory");
+}
+
+// True in one lane of a converged warp.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(r));
+    return r != 0;
 }
 
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
@@ -134,8 +178,18 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float v[32]) {
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-struct ConvSmem {
-    uint64_t full[MAX_SLOT], empty[MAX_SLOT], tfull[2], tempty[2], wbar;
+// Zeros into 32 consecutive columns of this warp's TMEM lanes.
+__device__ __forceinline__ void tmem_zero32(uint32_t taddr) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, "
+        "%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1};" ::"r"(taddr),
+        "r"(0)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+struct __align__(16) ConvSmem {
+    uint64_t full[MAX_SLOT], empty[MAX_SLOT], tfull[4], tempty[4], done;
     uint32_t tmem_base;
     int abort;
 };
@@ -152,42 +206,42 @@ __device__ __forceinline__ ConvUnit unit_of(const ConvArgs& a, int u) {
     return r;
 }
 
-template <int NSLOT>
+template <int N>
 __global__ void __launch_bounds__(CONV_THREADS, 1)
-    conv3d_tc_kernel(const __grid_constant__ CUtensorMap m0, const __grid_constant__ CUtensorMap m1,
-                     const __grid_constant__ CUtensorMap m2, const __grid_constant__ CUtensorMap m3,
-                     const ConvArgs a) {
+    conv3d_tc_kernel(const __grid_constant__ CUtensorMap map, const ConvArgs a) {
+    constexpr uint32_t ID = idesc_n(N);
+    constexpr int HC = N / 4;  // columns of one epilogue warp
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    // every TMA destination below is a multiple of 128 bytes from this base
-    unsigned char* smem = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
+    // the swizzle pattern repeats every 512 bytes: slots and boxes start on one
+    unsigned char* smem = smem_raw + ((512u - (smem_u32(smem_raw) & 511u)) & 511u);
     const int W2 = a.W + 2;
     const int PL = (a.H + 2) * W2;
-    const int win_rows = a.rows_box * a.nload;          // rows per (kd, cb) column
-    const uint32_t lbo_a = (uint32_t)win_rows * 16u;    // channel-block stride
-    const uint32_t slot_bytes = 4u * lbo_a;           // one plane window, 4 channel-block columns
-    unsigned char* wsm = smem;                           // weights
-    unsigned char* slots = smem + W_BYTES;               // 128-byte aligned (W_BYTES = 54 KB)
-    ConvSmem* cs = reinterpret_cast<ConvSmem*>(slots + NSLOT * slot_bytes);
+    const uint32_t box_bytes = (uint32_t)a.rows_box * (CH * 2);
+    const uint32_t slot_bytes = box_bytes * (uint32_t)a.nload;  // one plane window
+    unsigned char* wsm = smem;                                   // weights
+    unsigned char* slots = smem + W_BYTES;                       // 512-byte aligned
+    ConvSmem* cs = reinterpret_cast<ConvSmem*>(slots + a.nslot * slot_bytes);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint64_t lim = a.timeout_ns;
+    const uint64_t dlim = lim > WAIT_DRAIN_NS ? lim : WAIT_DRAIN_NS;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < NSLOT; ++s) {
+        for (int s = 0; s < a.nslot; ++s) {
             mbar_init(&cs->full[s], 1);
             mbar_init(&cs->empty[s], 1);
         }
-        for (int s = 0; s < 2; ++s) {
+        for (int s = 0; s < 4; ++s) {
             mbar_init(&cs->tfull[s], 1);
             mbar_init(&cs->tempty[s], 128);
         }
-        mbar_init(&cs->wbar, 1);
+        mbar_init(&cs->done, 1);
         cs->abort = 0;
         fence_mbar_init();
     }
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                          smem_u32(&cs->tmem_base)),
-                     "r"(TMEM_COLS)
+                     "r"(N)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
         tc_fence_before();
@@ -195,24 +249,44 @@ __global__ void __launch_bounds__(CONV_THREADS, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = cs->tmem_base;
-    const CUtensorMap* maps[4] = {&m0, &m1, &m2, &m3};
+    // The weights, 16 bytes a thread and both of a block's places (512-byte bulk
+    // copies, 216 of them, kept the copy engine busy for 10 us).
+    {
+        const uint4* src = static_cast<const uint4*>(a.w);  // [tap][channel block][32 rows] of 16 bytes
+        for (int c = threadIdx.x; c < NTAP * CH * 4; c += CONV_THREADS) {
+            const int tap = c >> 7, cb = (c >> 5) & 3, row = c & 31, kd = tap / 9, t = tap - 9 * kd;
+            unsigned char* dst = wsm + t * WB_TAP + cb * WB_CB + (2 - kd) * WB_BLOCK + row * 16;
+            const uint4 w = __ldg(src + c);
+            *reinterpret_cast<uint4*>(dst) = w;
+            *reinterpret_cast<uint4*>(dst + 4 * WB_BLOCK) = w;
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    // the epilogue warps' lane quarter and columns; the accumulators start at zero
+    const int quarter = warp & 3, half = (warp - 2) >> 2;
+    const uint32_t tlane = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * HC);
+    if (warp >= 2) {
+#pragma unroll
+        for (int c = 0; c < HC; c += 32) tmem_zero32(tlane + (uint32_t)c);
+        tmem_wait_st();
+        tc_fence_before();
+    }
+    __syncthreads();
+    tc_fence_after();
 
-    // Window fills are numbered g = 0, 1, ... in the CTA's unit order; fill g
-    // goes to slot g % NSLOT. A unit of planes [d0, d1) takes d1 - d0 + 2 fills
-    // (padded planes d0 .. d1 + 1); its k-th tile reads fills g0 + k + kd.
+    // Windows are numbered g = 0, 1, ... in the CTA's unit order; window g goes
+    // to slot g % nslot. A unit of planes [d0, d1) takes d1 - d0 + 2 of them.
     if (warp == 0) {
         if (lane == 0) {
-            mbar_arrive_expect_tx(&cs->wbar, W_BYTES);
-            bulk_load(wsm, a.w, W_BYTES, &cs->wbar);
             int g = 0;
             bool stop = false;
             for (int u = blockIdx.x; u < a.units && !stop; u += gridDim.x) {
                 const ConvUnit U = unit_of(a, u);
-                const int p0 = U.col * TM;
+                const int p0 = U.col * N;
                 const int nfill = U.d1 - U.d0 + 2;
                 for (int j = 0; j < nfill; ++j, ++g) {
-                    const int slot = g % NSLOT;
-                    if (g >= NSLOT && !mbar_wait_bounded(&cs->empty[slot], ((g / NSLOT) - 1) & 1, lim)) {
+                    const int slot = g % a.nslot;
+                    if (g >= a.nslot && !mbar_wait_bounded(&cs->empty[slot], ((g / a.nslot) - 1) & 1, lim)) {
                         atomicOr(a.flags, CONV_FLAG_TIMEOUT);
                         cs->abort = 1;
                         stop = true;
@@ -224,96 +298,104 @@ __global__ void __launch_bounds__(CONV_THREADS, 1)
                     }
                     unsigned char* sb = slots + slot * slot_bytes;
                     const int q0 = (U.d0 + j) * PL + p0 - (W2 + 1);
-                    mbar_arrive_expect_tx(&cs->full[slot], 4u * (uint32_t)a.nload * (uint32_t)a.rows_box * 16u);
-                    for (int cb = 0; cb < 4; ++cb)
-                        for (int l = 0; l < a.nload; ++l)
-                            tma_load_2d(sb + cb * lbo_a + l * a.rows_box * 16, maps[cb], &cs->full[slot], 0,
-                                        q0 + l * a.rows_box);
+                    mbar_arrive_expect_tx(&cs->full[slot], slot_bytes);
+                    for (int l = 0; l < a.nload; ++l)
+                        tma_load_2d(sb + l * box_bytes, &map, &cs->full[slot], 0, q0 + l * a.rows_box);
                 }
             }
             // drain: every issued window has landed before the CTA may exit
-            for (int f = (g > NSLOT ? g - NSLOT : 0); f < g; ++f)
-                if (!mbar_wait_bounded(&cs->full[f % NSLOT], (f / NSLOT) & 1, lim > WAIT_DRAIN_NS ? lim : WAIT_DRAIN_NS))
+            for (int f = (g > a.nslot ? g - a.nslot : 0); f < g; ++f)
+                if (!mbar_wait_bounded(&cs->full[f % a.nslot], (f / a.nslot) & 1, dlim))
                     atomicOr(a.flags, CONV_FLAG_TIMEOUT);
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            bool ok = mbar_wait_bounded(&cs->wbar, 0, lim);
-            int committed = 0, i = 0, g0 = 0;
-            const uint32_t wb = smem_u32(wsm);
-            for (int u = blockIdx.x; ok && u < a.units; u += gridDim.x) {
-                const ConvUnit U = unit_of(a, u);
-                const int nt = U.d1 - U.d0;
-                for (int k = 0; ok && k < nt; ++k, ++i) {
-                    const int acc = i & 1;
-                    if (i >= 2 && !mbar_wait_bounded(&cs->tempty[acc], ((i >> 1) & 1) ^ 1, lim)) {
+        // The whole warp runs the loop and one elected lane issues: addresses and
+        // descriptors stay in uniform registers. Issued from a branch on the lane
+        // number every instruction moved its nine operands there first (290
+        // cycles each, whatever its size).
+        bool ok = true;
+        unsigned used = 0;  // four byte counts modulo 256: planes that have taken each block
+        int g = 0;
+        const uint32_t wb = smem_u32(wsm) >> 4, slots4 = smem_u32(slots) >> 4;
+        const uint64_t adesc = smem_desc(0, WB_CB, 128u), bdesc = smem_desc_sw64(0);
+        const uint32_t alo0 = (uint32_t)adesc, ahi = (uint32_t)(adesc >> 32), blo0 = (uint32_t)bdesc,
+                       bhi = (uint32_t)(bdesc >> 32);
+        const uint32_t rowstep = (uint32_t)W2 * (CH * 2u / 16u);
+        for (int u = blockIdx.x; ok && u < a.units; u += gridDim.x) {
+            const ConvUnit U = unit_of(a, u);
+            for (int p = U.d0 - 1; p <= U.d1; ++p, ++g) {
+                // a plane that starts here takes its block once that has been read and zeroed
+                if (p + 1 < U.d1) {
+                    const int sh = ((p + 1) & 3) * 8;
+                    const unsigned n = (used >> sh) & 255u;
+                    if (n > 0 && !__all_sync(0xffffffffu, mbar_wait_bounded(&cs->tempty[(p + 1) & 3], (n - 1) & 1, lim))) {
                         ok = false;
                         break;
                     }
-                    uint32_t sbase[3];
-                    for (int kd = 0; kd < 3; ++kd) {
-                        const int f = g0 + k + kd;
-                        if (!mbar_wait_bounded(&cs->full[f % NSLOT], (f / NSLOT) & 1, lim)) ok = false;
-                        sbase[kd] = smem_u32(slots + (f % NSLOT) * slot_bytes);
-                    }
-                    if (!ok || read_abort(&cs->abort)) {
-                        ok = ok && !read_abort(&cs->abort);
-                        break;
-                    }
-                    tc_fence_after();
-                    const uint32_t d_tmem = tmem + (uint32_t)(acc * CH);
-                    for (int kd = 0; kd < 3; ++kd)
-                        for (int kh = 0; kh < 3; ++kh)
-                            for (int kw = 0; kw < 3; ++kw) {
-                                const int tap = (kd * 3 + kh) * 3 + kw;
-                                const uint32_t roff = (uint32_t)(W2 + 1 + (kh - 1) * W2 + (kw - 1)) * 16u;
-#pragma unroll
-                                for (int ks = 0; ks < 2; ++ks) {
-                                    const uint64_t ad = smem_desc(sbase[kd] + (uint32_t)(2 * ks) * lbo_a + roff, lbo_a,
-                                                                  128u);
-                                    const uint64_t bd = smem_desc(wb + (uint32_t)tap * 2048u + (uint32_t)ks * 1024u,
-                                                                  512u, 128u);
-                                    mma_bf16(d_tmem, ad, bd, (tap | ks) != 0);
-                                }
-                            }
-                    mma_commit(&cs->tfull[acc]);
-                    // the window of plane d (tap kd = 0) has served its last tile; at
-                    // the unit's end so have the two after it
-                    mma_commit(&cs->empty[(g0 + k) % NSLOT]);
-                    if (k == nt - 1) {
-                        mma_commit(&cs->empty[(g0 + k + 1) % NSLOT]);
-                        mma_commit(&cs->empty[(g0 + k + 2) % NSLOT]);
-                    }
-                    ++committed;
+                    // 255 wraps to 2, not to 0: the same parity, and a block once taken stays so
+                    used = (used & ~(255u << sh)) | ((n == 255u ? 2u : n + 1) << sh);
                 }
-                g0 += nt + 2;
-            }
-            if (!ok) {
-                atomicOr(a.flags, CONV_FLAG_TIMEOUT);
-                cs->abort = 1;
-            }
-            // drain: the last commit tracks every MMA this thread issued
-            if (committed > 0) {
-                const int last = committed - 1;
-                if (!mbar_wait_bounded(&cs->tfull[last & 1], (last >> 1) & 1, lim > WAIT_DRAIN_NS ? lim : WAIT_DRAIN_NS))
-                    atomicOr(a.flags, CONV_FLAG_TIMEOUT);
+                const int slot = g % a.nslot;
+                if (!__all_sync(0xffffffffu,
+                                mbar_wait_bounded(&cs->full[slot], (g / a.nslot) & 1, lim) && !read_abort(&cs->abort))) {
+                    ok = false;
+                    break;
+                }
+                tc_fence_after();
+                uint32_t off[4];
+#pragma unroll
+                for (int b = 0; b < 4; ++b) {
+                    // the output plane among p - 1 .. p + 2 that lives in block b
+                    const int q = p - 1 + ((b - (p - 1)) & 3);
+                    off[b] = (q <= p + 1 && q >= U.d0 && q < U.d1) ? 0u : 0xffffffffu;
+                }
+                const uint32_t alo = alo0 + wb + (uint32_t)((1 - p) & 3) * (WB_BLOCK / 16);
+                const uint32_t blo = blo0 + slots4 + (uint32_t)slot * (slot_bytes >> 4);
+                if (elect_one()) {
+#pragma unroll
+                    for (int t = 0; t < 9; ++t)
+#pragma unroll
+                        for (int ks = 0; ks < 2; ++ks)
+                            mma_bf16_lanes(tmem, alo + (uint32_t)(t * (WB_TAP / 16) + ks * (2 * WB_CB / 16)), ahi,
+                                           blo + (uint32_t)(t / 3) * rowstep + (uint32_t)((t % 3) * 4 + ks * 2), bhi, ID,
+                                           off);
+                    mma_commit(&cs->empty[slot]);
+                    if (p - 1 >= U.d0) mma_commit(&cs->tfull[(p - 1) & 3]);
+                }
+                __syncwarp();
             }
         }
+        if (!ok && lane == 0) {
+            atomicOr(a.flags, CONV_FLAG_TIMEOUT);
+            cs->abort = 1;
+        }
+        // drain: no MMA runs when TMEM is freed (commits of the lane that issued them)
+        if (elect_one()) {
+            mma_commit(&cs->done);
+            if (!mbar_wait_bounded(&cs->done, 0, dlim)) atomicOr(a.flags, CONV_FLAG_TIMEOUT);
+        }
+        __syncwarp();
     } else {
-        // epilogue: warps 2..5 own TMEM lane quarters (warp % 4)
-        const int quarter = warp & 3;
-        const int row = quarter * 32 + lane;
-        float bias[CH];
+        const int vl = lane >> 3, cg = lane & 7;  // the voxel of four and the four channels this lane stores
+        float* stage = reinterpret_cast<float*>(cs + 1) + (warp - 2) * STAGE_FLOATS;
+        float bias[4];
 #pragma unroll
-        for (int c = 0; c < CH; ++c) bias[c] = a.bias ? a.bias[c] : 0.0f;
-        int i = 0;
+        for (int c = 0; c < 4; ++c) bias[c] = a.bias ? a.bias[4 * cg + c] : 0.0f;
+        int cnt = 0;
         bool stop = false;
         for (int u = blockIdx.x; u < a.units && !stop; u += gridDim.x) {
             const ConvUnit U = unit_of(a, u);
-            for (int d = U.d0; d < U.d1; ++d, ++i) {
-                const int acc = i & 1;
-                // warp-uniform outcome: the TMEM load below is a warp-collective
-                const bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(&cs->tfull[acc], (i >> 1) & 1, lim));
+            const int pc = U.col * N + half * HC;  // in-plane position of this warp's first column
+            unsigned inside[HC / 32], valid[HC / 32];
+#pragma unroll
+            for (int w = 0; w < HC / 32; ++w) {
+                const int p = pc + 32 * w + lane, h = p / W2, x = p - h * W2;
+                inside[w] = __ballot_sync(0xffffffffu, h >= 1 && h <= a.H && x >= 1 && x <= a.W) >> vl;
+                valid[w] = __ballot_sync(0xffffffffu, p < PL) >> vl;
+            }
+            for (int d = U.d0 + ((quarter - U.d0) & 3); d < U.d1; d += 4, ++cnt) {
+                // warp-uniform outcome: the TMEM accesses below are warp-collective
+                const bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(&cs->tfull[quarter], cnt & 1, lim));
                 if (!ok) {
                     if (lane == 0) atomicOr(a.flags, CONV_FLAG_TIMEOUT);
                     cs->abort = 1;
@@ -321,54 +403,60 @@ __global__ void __launch_bounds__(CONV_THREADS, 1)
                     break;
                 }
                 tc_fence_after();
-                float v[CH];
-                tmem_ld32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * CH), v);
+                const long long q0 = ((long long)(d + 1) * PL + pc + vl) * CH + 4 * cg;
+                float v[HC];
+#pragma unroll
+                for (int c = 0; c < HC; c += 32) tmem_ld32(tlane + (uint32_t)c, v + c);
+#pragma unroll
+                for (int c = 0; c < HC; c += 32) tmem_zero32(tlane + (uint32_t)c);
+                tmem_wait_st();
                 tc_fence_before();
-                mbar_arrive(&cs->tempty[acc]);
-                const int p = U.col * TM + row;
-                if (p >= PL) continue;
-                const int h = p / W2, w = p - h * W2;
-                const bool inside = h >= 1 && h <= a.H && w >= 1 && w <= a.W;
-                const long long q = (long long)(d + 1) * PL + p;
-                if (inside) {
-                    if (a.add) {
-                        const uint4* ap = reinterpret_cast<const uint4*>(a.add + q * CH);
+                mbar_arrive(&cs->tempty[quarter]);  // the block is free for the plane after next
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const uint4 uu = ap[j];
-                            const __nv_bfloat162* b2 = reinterpret_cast<const __nv_bfloat162*>(&uu);
+                for (int h = 0; h < HC / 4; h += 8) {  // eight groups' residual inputs in flight
+                    uint2 add[8];
 #pragma unroll
-                            for (int e = 0; e < 4; ++e) {
-                                const float2 f = __bfloat1622float2(b2[e]);
-                                v[8 * j + 2 * e] += f.x;
-                                v[8 * j + 2 * e + 1] += f.y;
+                    for (int k = 0; k < 8; ++k) {
+                        const int i = 4 * (h + k);
+                        add[k] = make_uint2(0u, 0u);
+                        if (a.add && ((inside[i / 32] >> (i % 32)) & 1u))
+                            add[k] = *reinterpret_cast<const uint2*>(a.add + q0 + (long long)i * CH);
+                    }
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        const int i = 4 * (h + k);
+                        __syncwarp();
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) stage[e * CH + lane] = v[i + e];
+                        __syncwarp();
+                        float x[4];
+                        *reinterpret_cast<float4*>(x) = *reinterpret_cast<const float4*>(stage + vl * CH + 4 * cg);
+                        const __nv_bfloat162* ab = reinterpret_cast<const __nv_bfloat162*>(&add[k]);
+                        const bool ins = (inside[i / 32] >> (i % 32)) & 1u;
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            const float2 f = __bfloat1622float2(ab[e]);
+                            x[2 * e] = (x[2 * e] + f.x) + bias[2 * e];
+                            x[2 * e + 1] = (x[2 * e + 1] + f.y) + bias[2 * e + 1];
+                        }
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            if (a.relu) x[e] = fmaxf(x[e], 0.0f);
+                            if (!ins) x[e] = 0.0f;
+                        }
+                        if ((valid[i / 32] >> (i % 32)) & 1u) {
+                            const long long q = q0 + (long long)i * CH;
+                            if (a.out_f32) {
+                                *reinterpret_cast<float4*>(static_cast<float*>(a.out) + q) =
+                                    make_float4(x[0], x[1], x[2], x[3]);
+                            } else {
+                                uint2 u;
+                                __nv_bfloat162* b2 = reinterpret_cast<__nv_bfloat162*>(&u);
+                                b2[0] = __floats2bfloat162_rn(x[0], x[1]);
+                                b2[1] = __floats2bfloat162_rn(x[2], x[3]);
+                                *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(a.out) + q) = u;
                             }
                         }
-                    }
-#pragma unroll
-                    for (int c = 0; c < CH; ++c) {
-                        v[c] += bias[c];
-                        if (a.relu) v[c] = fmaxf(v[c], 0.0f);
-                    }
-                } else {
-#pragma unroll
-                    for (int c = 0; c < CH; ++c) v[c] = 0.0f;
-                }
-                if (a.out_f32) {
-                    float4* op = reinterpret_cast<float4*>(static_cast<float*>(a.out) + q * CH);
-#pragma unroll
-                    for (int j = 0; j < 8; ++j)
-                        op[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-                } else {
-                    uint4* op = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(a.out) + q * CH);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        uint4 uu;
-                        __nv_bfloat162* b2 = reinterpret_cast<__nv_bfloat162*>(&uu);
-#pragma unroll
-                        for (int e = 0; e < 4; ++e)
-                            b2[e] = __floats2bfloat162_rn(v[8 * j + 2 * e], v[8 * j + 2 * e + 1]);
-                        op[j] = uu;
                     }
                 }
             }
@@ -377,7 +465,7 @@ __global__ void __launch_bounds__(CONV_THREADS, 1)
     __syncthreads();
     if (warp == 1) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(N) : "memory");
     }
 }
 
@@ -406,17 +494,17 @@ int num_sms_conv() {
     return n;
 }
 
-// One 2-D map per 8-channel block over the padded volume viewed as
-// [rows][32 channels]: box {8 channels, rows_box rows}.
-int make_conv_map(CUtensorMap* map, const __nv_bfloat16* base, long long rows, int cb, int rows_box) {
+// The padded volume viewed as [rows][32 channels], box {32 channels, box_rows},
+// 64-byte swizzled in shared memory.
+int make_rows_map(CUtensorMap* map, const __nv_bfloat16* base, long long rows, int box_rows) {
     EncodeTiledFn enc = nullptr;
     ST_TRY(get_encode_tiled(&enc));
-    cuuint64_t dims[2] = {8, (cuuint64_t)rows};
+    cuuint64_t dims[2] = {CH, (cuuint64_t)rows};
     cuuint64_t strides[1] = {(cuuint64_t)CH * 2};
-    cuuint32_t box[2] = {8, (cuuint32_t)rows_box};
+    cuuint32_t box[2] = {CH, (cuuint32_t)box_rows};
     cuuint32_t estr[2] = {1, 1};
-    CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<__nv_bfloat16*>(base + cb * 8), dims,
-                     strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+    CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<__nv_bfloat16*>(base), dims, strides, box,
+                     estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
                      CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     ST_CHECK(r == CUDA_SUCCESS, ST_ERR_CUDA, "cuTensorMapEncodeTiled (conv) failed (%d)", (int)r);
     return ST_OK;
@@ -685,22 +773,6 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
     }
 }
 
-// The padded volume viewed as [rows][32 channels], box {32 channels, 64 rows},
-// 64-byte swizzled in shared memory.
-int make_wgrad_map(CUtensorMap* map, const __nv_bfloat16* base, long long rows) {
-    EncodeTiledFn enc = nullptr;
-    ST_TRY(get_encode_tiled(&enc));
-    cuuint64_t dims[2] = {CH, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)CH * 2};
-    cuuint32_t box[2] = {CH, WG_KSTEP};
-    cuuint32_t estr[2] = {1, 1};
-    CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<__nv_bfloat16*>(base), dims, strides, box,
-                     estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
-                     CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    ST_CHECK(r == CUDA_SUCCESS, ST_ERR_CUDA, "cuTensorMapEncodeTiled (wgrad) failed (%d)", (int)r);
-    return ST_OK;
-}
-
 __device__ unsigned g_conv_flags;
 
 }  // namespace
@@ -732,26 +804,54 @@ int st_conv3d_bf16(const void* in, const void* packed_w, const float* bias, cons
              "conv buffers must be 16-byte aligned");
     const long long W2 = W + 2, PL = (H + 2) * W2, rows = (D + 2) * PL;
     ST_CHECK(rows < (1ll << 31), ST_ERR_ARG, "volume too large");
-    // window column of one plane and channel block: win rows, loaded as nload
-    // boxes of rows_box rows (<= 256, a multiple of 8 so that every TMA
-    // destination stays 128-byte aligned)
-    const long long win = TM + 2 * (W2 + 1);
-    int nload = (int)((win + 255) / 256);
-    int rows_box = (int)((((win + nload - 1) / nload) + 7) / 8 * 8);
-    while (rows_box > 256) {
-        ++nload;
-        rows_box = (int)((((win + nload - 1) / nload) + 7) / 8 * 8);
-    }
-    auto smem_of = [&](int ns) {
-        return (size_t)W_BYTES + (size_t)ns * 4 * 16 * nload * rows_box + sizeof(ConvSmem) + 128;
+    ST_CHECK(W <= MAX_WIDTH, ST_ERR_UNSUPPORTED, "volume width %lld too large for the conv tiles", (long long)W);
+    // Voxels per instruction (256 or 128) and planes per unit: the fewest cycles
+    // over the rounds of units on the SMs. A unit of dc planes takes dc + 2 input
+    // planes of 18 instructions; one of 256 voxels measured 128 cycles, of 128 64
+    // (of 64 49); a round's first window and last epilogue are not hidden. 100^3:
+    // 256 voxels; volumes whose planes fill few tiles (32^3) take 128 so that more
+    // SMs have work.
+    const long long nsm = num_sms_conv();
+    auto window = [&](int n, int* nl, int* rb) {
+        // one plane's window: win rows, loaded as nl boxes of rb rows (<= 256, a
+        // multiple of 8 so that every TMA destination stays 512-byte aligned)
+        const long long win = n + 2 * (W2 + 1);
+        *nl = (int)((win + 255) / 256);
+        *rb = (int)((((win + *nl - 1) / *nl) + 7) / 8 * 8);
+        while (*rb > 256) {
+            ++*nl;
+            *rb = (int)((((win + *nl - 1) / *nl) + 7) / 8 * 8);
+        }
     };
-    const int nslot = smem_of(MAX_SLOT) <= (size_t)SMEM_LIMIT ? MAX_SLOT : MIN_SLOT;
-    const size_t smem = smem_of(nslot);
-    ST_CHECK(smem <= (size_t)SMEM_LIMIT, ST_ERR_UNSUPPORTED, "volume width %lld too large for the conv tiles",
-             (long long)W);
+    auto smem_of = [&](int n, int slots) {
+        int nl, rb;
+        window(n, &nl, &rb);
+        return (size_t)W_BYTES + (size_t)slots * (CH * 2) * nl * rb + sizeof(ConvSmem) + EPI_WARPS * STAGE_FLOATS * 4 + 512;
+    };
+    int N = 0;
+    long long best_cost = -1, best_dc = 1;
+    for (int n = 256; n >= 128; n /= 2) {
+        if (smem_of(n, n == 256 ? 2 : 1) > (size_t)SMEM_LIMIT) continue;  // 256: widths up to 197
+        const long long tiles = (PL + n - 1) / n, mma = n / 2;
+        for (long long dc = 1; dc <= D; ++dc) {
+            const long long units = tiles * ((D + dc - 1) / dc);
+            const long long cost = (units + nsm - 1) / nsm * ((dc + 2) * 18 * mma + 3000);
+            if (best_cost < 0 || cost < best_cost) {
+                best_cost = cost;
+                best_dc = dc;
+                N = n;
+            }
+        }
+    }
+    ST_CHECK(N > 0, ST_ERR_UNSUPPORTED, "volume width %lld too large for the conv tiles", (long long)W);
+    int nload, rows_box;
+    window(N, &nload, &rows_box);
+    int nslot = MAX_SLOT;  // two from widths of 102 (256 voxels) and 165 (128), one from 263
+    while (smem_of(N, nslot) > (size_t)SMEM_LIMIT) --nslot;
+    const size_t smem = smem_of(N, nslot);
     const __nv_bfloat16* src = static_cast<const __nv_bfloat16*>(in);
-    CUtensorMap maps[4];
-    for (int cb = 0; cb < 4; ++cb) ST_TRY(make_conv_map(&maps[cb], src, rows, cb, rows_box));
+    CUtensorMap map;
+    ST_TRY(make_rows_map(&map, src, rows, rows_box));
     unsigned* flags = nullptr;
     ST_CUDA(cudaGetSymbolAddress(reinterpret_cast<void**>(&flags), g_conv_flags));
     ConvArgs a{};
@@ -766,29 +866,18 @@ int st_conv3d_bf16(const void* in, const void* packed_w, const float* bias, cons
     a.relu = relu;
     a.rows_box = rows_box;
     a.nload = nload;
-    a.tiles_per_plane = (int)((PL + TM - 1) / TM);
-    // planes per unit: the fewest rounds of units over the SMs, each unit
-    // paying two extra window loads (its first two planes)
-    const long long nsm = num_sms_conv();
-    long long best_cost = -1;
-    for (long long dc = 1; dc <= D; ++dc) {
-        const long long units = (long long)a.tiles_per_plane * ((D + dc - 1) / dc);
-        const long long rounds = (units + nsm - 1) / nsm;
-        const long long cost = rounds * (dc + 2);
-        if (best_cost < 0 || cost < best_cost) {
-            best_cost = cost;
-            a.dchunk = (int)dc;
-        }
-    }
+    a.nslot = nslot;
+    a.tiles_per_plane = (int)((PL + N - 1) / N);
+    a.dchunk = (int)best_dc;
     a.units = (int)((long long)a.tiles_per_plane * ((D + a.dchunk - 1) / a.dchunk));
     a.flags = flags;
     a.timeout_ns = 2000000000ull;
-    auto kern = nslot == MAX_SLOT ? conv3d_tc_kernel<MAX_SLOT> : conv3d_tc_kernel<MIN_SLOT>;
+    auto kern = N == 256 ? conv3d_tc_kernel<256> : conv3d_tc_kernel<128>;
     static std::mutex mu;
     static size_t configured[2] = {0, 0};
     {
         std::lock_guard<std::mutex> lk(mu);
-        size_t& c = configured[nslot == MAX_SLOT ? 1 : 0];
+        size_t& c = configured[N == 256 ? 1 : 0];
         if (c < smem) {
             ST_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             c = smem;
@@ -796,7 +885,7 @@ int st_conv3d_bf16(const void* in, const void* packed_w, const float* bias, cons
     }
     const int grid = std::min(a.units, num_sms_conv());
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    kern<<<grid, CONV_THREADS, smem, st>>>(maps[0], maps[1], maps[2], maps[3], a);
+    kern<<<grid, CONV_THREADS, smem, st>>>(map, a);
     count_launch();
     ST_CUDA(cudaGetLastError());
     return ST_OK;
@@ -810,8 +899,8 @@ int st_conv3d_wgrad(const void* x, const void* g, float* dw, int64_t nx, int64_t
     const long long rows = (nx + 2) * (ny + 2) * (nz + 2);
     ST_CHECK(rows + (ny + 2) * (nz + 2) + nz + 3 < (1ll << 31), ST_ERR_ARG, "volume too large");
     CUtensorMap mx, mg;
-    ST_TRY(make_wgrad_map(&mx, static_cast<const __nv_bfloat16*>(x), rows));
-    ST_TRY(make_wgrad_map(&mg, static_cast<const __nv_bfloat16*>(g), rows));
+    ST_TRY(make_rows_map(&mx, static_cast<const __nv_bfloat16*>(x), rows, WG_KSTEP));
+    ST_TRY(make_rows_map(&mg, static_cast<const __nv_bfloat16*>(g), rows, WG_KSTEP));
     unsigned* flags = nullptr;
     ST_CUDA(cudaGetSymbolAddress(reinterpret_cast<void**>(&flags), g_conv_flags));
     WgradArgs a{};
