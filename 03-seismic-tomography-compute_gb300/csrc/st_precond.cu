@@ -133,53 +133,170 @@ __global__ void in_conv_wgrad_kernel(const float* __restrict__ r, const float* _
     }
 }
 
-// zhat = C_out(h); z = dinv * r + s_out * zhat (zhat kept for training).
-__global__ void out_conv_kernel(const __nv_bfloat16* __restrict__ h, const float* __restrict__ w, Vol v,
-                                const float* __restrict__ r, const float* __restrict__ dinv, const float* s_out,
-                                float* __restrict__ zhat, float* __restrict__ z) {
-    __shared__ float ws[CH * NTAP];
-    for (int i = threadIdx.x; i < CH * NTAP; i += blockDim.x) ws[i] = w[i];
+// Two FP32 fused multiply-adds in one instruction.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    return (f32x2)__float_as_uint(lo) | ((f32x2)__float_as_uint(hi) << 32);
+}
+__device__ __forceinline__ float sum2(f32x2 v) {
+    return __uint_as_float((unsigned)v) + __uint_as_float((unsigned)(v >> 32));
+}
+// Two BF16 values (low half first) as FP32.
+__device__ __forceinline__ f32x2 unpack2(unsigned u) {
+    return (f32x2)(u << 16) | ((f32x2)(u & 0xffff0000u) << 32);
+}
+
+// A warp's eight z positions x four groups of eight channels: lane = 4 z + group,
+// so that a row access of the warp is 512 contiguous bytes.
+//
+// zhat = C_out(h); z = dinv * r + s_out * zhat (zhat kept for training). Each lane
+// forms the partial sums of its channels for 4 x 2 outputs (x, y): a row that is
+// loaded and unpacked serves up to six of them, and a weight two. Bound by
+// instructions and their latency: 0.86 G products at 100^3 in 75 us; one output per
+// thread unpacked every row 27 times and read a weight per product (275 us).
+constexpr int OC_X = 4, OC_Y = 2;
+__global__ void __launch_bounds__(128, 3) out_conv_kernel(const __nv_bfloat16* __restrict__ h, const float* __restrict__ w,
+                                                       Vol v, const float* __restrict__ r,
+                                                       const float* __restrict__ dinv, const float* s_out,
+                                                       float* __restrict__ zhat, float* __restrict__ z) {
+    __shared__ __align__(16) float ws[NTAP * CH];  // [tap][channel]
+    for (int i = threadIdx.x; i < CH * NTAP; i += blockDim.x) ws[i] = w[(i % CH) * NTAP + i / CH];
     __syncthreads();
     const float so = s_out ? *s_out : 0.0f;
-    const int W2 = v.nz + 2, P2 = (v.ny + 2) * W2;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < v.n(); i += (long long)gridDim.x * blockDim.x) {
-        int x, y, zz;
-        decode(i, v, x, y, zz);
-        const long long q = v.pad_row(x, y, zz);
-        float acc = 0.0f;
-        for (int tap = 0; tap < NTAP; ++tap) {
-            const long long qq = q + (long long)(tap / 9 - 1) * P2 + ((tap / 3) % 3 - 1) * W2 + (tap % 3 - 1);
-            float f[CH];
-            load_row32(h + qq * CH, f);  // the zero border supplies the padding
+    const int lane = threadIdx.x & 31, cg = lane & 3;
+    const int W2 = v.nz + 2;
+    const long long P2 = (long long)(v.ny + 2) * W2;
+    const unsigned ZT = (v.nz + 7) / 8, YT = (v.ny + OC_Y - 1) / OC_Y, XT = (v.nx + OC_X - 1) / OC_X;
+    for (unsigned g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < ZT * YT * XT; g += gridDim.x * blockDim.x >> 5) {
+        const unsigned col = g / ZT;
+        const int zt = (int)(g - col * ZT), xt = (int)(col / YT), yt = (int)(col - xt * YT);
+        const int x0 = xt * OC_X, y0 = yt * OC_Y, z0 = zt * 8 + (lane >> 2), zc = min(z0, v.nz - 1);
+        f32x2 acc[OC_X][OC_Y] = {};
+#pragma unroll 1
+        for (int kz = 0; kz < 3; ++kz) {
+            const float* wz = ws + kz * CH + cg * 8;
 #pragma unroll
-            for (int c = 0; c < CH; ++c) acc = fmaf(ws[c * NTAP + tap], f[c], acc);
+            for (int xi = 0; xi < OC_X + 2; ++xi) {
+                const __nv_bfloat16* hp = h + (min(x0 + xi, v.nx + 1) * P2 + zc + kz) * CH + cg * 8;
+                f32x2 row[OC_Y + 2][4];
+#pragma unroll
+                for (int yj = 0; yj < OC_Y + 2; ++yj) {
+                    const uint4 u = *reinterpret_cast<const uint4*>(hp + (long long)min(y0 + yj, v.ny + 1) * W2 * CH);
+                    row[yj][0] = unpack2(u.x);
+                    row[yj][1] = unpack2(u.y);
+                    row[yj][2] = unpack2(u.z);
+                    row[yj][3] = unpack2(u.w);
+                }
+#pragma unroll
+                for (int kx = 0; kx < 3; ++kx) {
+                    const int i = xi - kx;
+                    if (i < 0 || i >= OC_X) continue;
+#pragma unroll
+                    for (int ky = 0; ky < 3; ++ky) {
+                        const float4 wa = *reinterpret_cast<const float4*>(wz + (kx * 9 + ky * 3) * CH);
+                        const float4 wb = *reinterpret_cast<const float4*>(wz + (kx * 9 + ky * 3) * CH + 4);
+                        const f32x2 w4[4] = {pack2(wa.x, wa.y), pack2(wa.z, wa.w), pack2(wb.x, wb.y),
+                                             pack2(wb.z, wb.w)};
+#pragma unroll
+                        for (int j = 0; j < OC_Y; ++j)
+#pragma unroll
+                            for (int c = 0; c < 4; ++c) acc[i][j] = fma2(w4[c], row[j + ky][c], acc[i][j]);
+                    }
+                }
+            }
         }
-        if (zhat) zhat[i] = acc;
-        if (z) z[i] = fmaf(so, acc, dinv[i] * r[i]);
+#pragma unroll
+        for (int i = 0; i < OC_X; ++i)
+#pragma unroll
+            for (int j = 0; j < OC_Y; ++j) {
+                float s = sum2(acc[i][j]);
+                s += __shfl_xor_sync(0xffffffffu, s, 1);
+                s += __shfl_xor_sync(0xffffffffu, s, 2);
+                const int x = x0 + i, y = y0 + j;
+                if (cg == i && x < v.nx && y < v.ny && z0 < v.nz) {  // lane group i stores column x0 + i
+                    const long long e = ((long long)x * v.ny + y) * v.nz + z0;
+                    if (zhat) zhat[e] = s;
+                    if (z) z[e] = fmaf(so, s, dinv[e] * r[e]);
+                }
+            }
     }
 }
 
-// Backward of C_out: dh[v][c] = sum_tap w[c][tap] * dzhat[v - s_tap] (BF16,
-// interior rows), and dW_out[c][tap] += sum_v dzhat[v] * h[v + s_tap][c].
-__global__ void out_conv_dgrad_kernel(const float* __restrict__ dz, const float* __restrict__ w, Vol v,
-                                      __nv_bfloat16* __restrict__ dh) {
-    __shared__ float ws[CH * NTAP];
-    for (int i = threadIdx.x; i < CH * NTAP; i += blockDim.x) ws[i] = w[i];
+// Backward of C_out (and C^T itself): dh[v][c] = sum_tap w[c][tap] * dzhat[v - s_tap]
+// (BF16, interior rows). Each lane forms its eight channels of 2 x 2 voxels, so a
+// weight that is read serves four of them and the rows leave as 16-byte stores:
+// 61 us at 100^3, bound by instruction issue (71%); a thread per voxel read a
+// weight per product (113 us).
+constexpr int OD_X = 2, OD_Y = 2;
+__global__ void __launch_bounds__(128, 5) out_conv_dgrad_kernel(const float* __restrict__ dz, const float* __restrict__ w,
+                                                             Vol v, __nv_bfloat16* __restrict__ dh) {
+    __shared__ __align__(16) float ws[NTAP * CH];  // [tap][channel]
+    for (int i = threadIdx.x; i < CH * NTAP; i += blockDim.x) ws[i] = w[(i % CH) * NTAP + i / CH];
     __syncthreads();
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < v.n(); i += (long long)gridDim.x * blockDim.x) {
-        int x, y, z;
-        decode(i, v, x, y, z);
-        float acc[CH];
+    const int lane = threadIdx.x & 31, cg = lane & 3;
+    const unsigned ZT = (v.nz + 7) / 8, YT = (v.ny + OD_Y - 1) / OD_Y, XT = (v.nx + OD_X - 1) / OD_X;
+    for (unsigned g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < ZT * YT * XT; g += gridDim.x * blockDim.x >> 5) {
+        const unsigned col = g / ZT;
+        const int zt = (int)(g - col * ZT), xt = (int)(col / YT), yt = (int)(col - xt * YT);
+        const int x0 = xt * OD_X, y0 = yt * OD_Y, z0 = zt * 8 + (lane >> 2);
+        float acc[OD_X][OD_Y][8] = {};
+        unsigned inside = 0;  // bit 4 xi + yj: column (x0 + xi - 1, y0 + yj - 1) is in the volume
 #pragma unroll
-        for (int c = 0; c < CH; ++c) acc[c] = 0.0f;
-        for (int tap = 0; tap < NTAP; ++tap) {
-            const int xx = x - (tap / 9 - 1), yy = y - ((tap / 3) % 3 - 1), zz = z - (tap % 3 - 1);
-            if (xx < 0 || xx >= v.nx || yy < 0 || yy >= v.ny || zz < 0 || zz >= v.nz) continue;
-            const float g = dz[((long long)xx * v.ny + yy) * v.nz + zz];
+        for (int xi = 0; xi < OD_X + 2; ++xi)
 #pragma unroll
-            for (int c = 0; c < CH; ++c) acc[c] = fmaf(ws[c * NTAP + tap], g, acc[c]);
+            for (int yj = 0; yj < OD_Y + 2; ++yj) {
+                const int xx = x0 + xi - 1, yy = y0 + yj - 1;
+                inside |= (xx >= 0 && xx < v.nx && yy >= 0 && yy < v.ny ? 1u : 0u) << (4 * xi + yj);
+            }
+        const float* corner = dz + ((long long)(x0 - 1) * v.ny + (y0 - 1)) * v.nz;  // read only where inside
+        float in[OD_X + 2][OD_Y + 2][3];  // [..][..][kz]
+#pragma unroll
+        for (int kz = 0; kz < 3; ++kz) {
+            const int zz = z0 + 1 - kz;
+            const unsigned ok = zz >= 0 && zz < v.nz ? inside : 0u;
+#pragma unroll
+            for (int xi = 0; xi < OD_X + 2; ++xi)
+#pragma unroll
+                for (int yj = 0; yj < OD_Y + 2; ++yj)
+                    in[xi][yj][kz] = (ok >> (4 * xi + yj)) & 1u ? __ldg(corner + (xi * v.ny + yj) * v.nz + zz) : 0.0f;
         }
-        store_row32(dh + v.pad_row(x, y, z) * CH, acc);
+        // in the order of the taps: the sums are rounded to BF16, and another order
+        // would round some of them the other way
+#pragma unroll
+        for (int kx = 0; kx < 3; ++kx)
+#pragma unroll
+            for (int ky = 0; ky < 3; ++ky)
+#pragma unroll
+                for (int kz = 0; kz < 3; ++kz) {
+                    const float* wt = ws + (kx * 9 + ky * 3 + kz) * CH + cg * 8;
+                    const float4 wa = *reinterpret_cast<const float4*>(wt);
+                    const float4 wb = *reinterpret_cast<const float4*>(wt + 4);
+                    const float w8[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
+#pragma unroll
+                    for (int i = 0; i < OD_X; ++i)
+#pragma unroll
+                        for (int j = 0; j < OD_Y; ++j)
+#pragma unroll
+                            for (int c = 0; c < 8; ++c)
+                                acc[i][j][c] = fmaf(w8[c], in[i + 2 - kx][j + 2 - ky][kz], acc[i][j][c]);
+                }
+#pragma unroll
+        for (int i = 0; i < OD_X; ++i)
+#pragma unroll
+            for (int j = 0; j < OD_Y; ++j) {
+                const int x = x0 + i, y = y0 + j;
+                if (x >= v.nx || y >= v.ny || z0 >= v.nz) continue;
+                uint4 u;
+                __nv_bfloat162* b = reinterpret_cast<__nv_bfloat162*>(&u);
+#pragma unroll
+                for (int c = 0; c < 4; ++c) b[c] = __floats2bfloat162_rn(acc[i][j][2 * c], acc[i][j][2 * c + 1]);
+                *reinterpret_cast<uint4*>(dh + v.pad_row(x, y, z0) * CH + cg * 8) = u;
+            }
     }
 }
 
@@ -284,6 +401,12 @@ __global__ void pc_combine_kernel(const float* __restrict__ y, const float* __re
         z[i] = fmaf(inv * sqrtf(dinv[i]), y[i], dinv[i] * r[i]);
 }
 
+// CTAs of four warps, a warp per group of bx x by x 8 voxels, all at once up to 16 per SM.
+unsigned grid_groups(const Vol& v, int bx, int by) {
+    const long long g = (long long)((v.nz + 7) / 8) * ((v.ny + by - 1) / by) * ((v.nx + bx - 1) / bx);
+    return (unsigned)std::max<long long>(1, std::min<long long>((g + 3) / 4, 152 * 16));
+}
+
 unsigned grid_for(long long n, int cap = 152 * 16) {
     return (unsigned)std::max<long long>(1, std::min<long long>((n + 255) / 256, cap));
 }
@@ -321,8 +444,8 @@ int st_pc_out_conv(const void* h, const float* w, const float* r, const float* d
                    float* z, int64_t nx, int64_t ny, int64_t nz, void* stream) {
     ST_CHECK(h && w && (!z || (r && dinv && s_out)), ST_ERR_ARG, "null argument");
     const Vol v{(int)nx, (int)ny, (int)nz};
-    out_conv_kernel<<<grid_for(v.n()), 256, 0, (cudaStream_t)stream>>>(static_cast<const __nv_bfloat16*>(h), w, v, r,
-                                                                       dinv, s_out, zhat, z);
+    out_conv_kernel<<<grid_groups(v, OC_X, OC_Y), 128, 0, (cudaStream_t)stream>>>(static_cast<const __nv_bfloat16*>(h), w,
+                                                                                  v, r, dinv, s_out, zhat, z);
     count_launch();
     ST_CUDA(cudaGetLastError());
     return ST_OK;
@@ -333,7 +456,7 @@ int st_pc_out_conv_bwd(const float* dzhat, const void* h, const float* w, void* 
     ST_CHECK(dzhat && h && w && dh && dw, ST_ERR_ARG, "null argument");
     const Vol v{(int)nx, (int)ny, (int)nz};
     cudaStream_t st = (cudaStream_t)stream;
-    out_conv_dgrad_kernel<<<grid_for(v.n()), 256, 0, st>>>(dzhat, w, v, static_cast<__nv_bfloat16*>(dh));
+    out_conv_dgrad_kernel<<<grid_groups(v, OD_X, OD_Y), 128, 0, st>>>(dzhat, w, v, static_cast<__nv_bfloat16*>(dh));
     count_launch();
     out_conv_wgrad_kernel<<<dim3(grid_for(v.n(), 64), NTAP), 256, 0, st>>>(dzhat, static_cast<const __nv_bfloat16*>(h),
                                                                             v, dw);
@@ -385,7 +508,8 @@ int st_pc_combine(const float* y, const float* r, const float* dinv, const float
 int st_pc_tconv1(const float* a, const float* w, void* h, int64_t nx, int64_t ny, int64_t nz, void* stream) {
     ST_CHECK(a && w && h, ST_ERR_ARG, "null argument");
     const Vol v{(int)nx, (int)ny, (int)nz};
-    out_conv_dgrad_kernel<<<grid_for(v.n()), 256, 0, (cudaStream_t)stream>>>(a, w, v, static_cast<__nv_bfloat16*>(h));
+    out_conv_dgrad_kernel<<<grid_groups(v, OD_X, OD_Y), 128, 0, (cudaStream_t)stream>>>(a, w, v,
+                                                                                       static_cast<__nv_bfloat16*>(h));
     count_launch();
     ST_CUDA(cudaGetLastError());
     return ST_OK;
