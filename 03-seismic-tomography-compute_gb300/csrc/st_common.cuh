@@ -11,6 +11,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <string>
+#include <utility>
 
 #include "seismic_gb300.h"
 
@@ -135,6 +136,30 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, unsigned parity
 // wait gave up: always the full default, whatever limit the pipeline ran with,
 // so that no copy can land in shared memory after the CTA has exited.
 constexpr uint64_t WAIT_DRAIN_NS = 2000000000ull;
+
+// Programmatic dependent launch. A kernel launched with launch_dependent may be
+// set up while its predecessor in the stream still runs; pdl_wait returns when
+// every grid before it has finished and its writes are visible, so it stands
+// before the first access to anything an earlier kernel writes. pdl_launch lets
+// the successor be set up as soon as this grid's last block runs.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <class... P, class... A>
+inline cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                                    A&&... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
 
 // 3-D tiled TMA load of one box into shared memory, completing on `bar`.
 // c0 is the innermost (z) coordinate and must be a multiple of 4 elements

@@ -425,6 +425,10 @@ __global__ void __launch_bounds__(NTHREADS, (Geo<EPI, SNAP_IN>::MINB))
     RA.inj = a.inj_x >= 0 && a.inj_y == RA.iy && inj_k >= 0 && inj_k < zvalid;
     RB.inj = RPT == 2 && a.inj_x >= 0 && a.inj_y == RB.iy && inj_k >= 0 && inj_k < zvalid;
 
+    // nothing above reads what an earlier launch writes (the sponge table is
+    // fixed); one launch's setup under the last one's end: see fd_step2_kernel
+    pdl_wait();
+    pdl_launch();
     float snap_inv = 0.0f;
     if constexpr (SNAP_OUT != SNAP_NONE) {
         const float m = __uint_as_float(*a.amax_cur);
@@ -693,16 +697,15 @@ int launch_variant(const Layout& L, const FieldMaps& mcur, const FieldMaps& mpre
     // The forward variants run best as one wave of long x-chunks; the imaging
     // and gradient variants (one row per thread, more resident CTAs) keep more
     // loads in flight with at least four waves of shorter chunks.
-    const int chunks = fd_step_grid_chunks(L, G::TYV, G::MINB, is_forward(EPI) ? 1 : 4);
+    const int chunks = fd_step_grid_chunks(L, G::TYV, G::MINB, is_forward(EPI) ? 1 : 4, 2, a.withhold ? 4 : 1);
     a.x_chunk = (int)((L.nx + chunks - 1) / chunks);
     const int nch = (int)((L.nx + a.x_chunk - 1) / a.x_chunk);
     dim3 grid((unsigned)((L.nz + TZ - 1) / TZ), (unsigned)((L.ny + G::TYV - 1) / G::TYV), (unsigned)nch);
     const CUtensorMap& mi = mimg ? *mimg : msnap;  // unused unless EPI == EPI_IMAGE_T
     const CUtensorMap& ml = mill ? *mill : msnap;
-    fd_step_kernel<SO, SI, EPI><<<grid, NTHREADS, SMEM, st>>>(mcur.cur[ti], mprev.ctr[ti], mc.ctr[ti], msnap, mi, ml,
-                                                             a);
+    ST_CUDA(launch_dependent(fd_step_kernel<SO, SI, EPI>, grid, dim3(NTHREADS), SMEM, st, mcur.cur[ti], mprev.ctr[ti],
+                             mc.ctr[ti], msnap, mi, ml, a));
     ::stg::count_launch();
-    ST_CUDA(cudaGetLastError());
     return ST_OK;
 }
 
@@ -982,6 +985,11 @@ __global__ void __launch_bounds__(NTHREADS, (Geo2<MODE, SK>::MINB))
     const float Dq = (dyz_q >= 0 && dyz_q < a.sw) ? a.dtab[dyz_q] : 1.0f;
     // imaging: snapshot scales of steps t and t-1; forward: inverse scales of
     // the two stored snapshots (u_t and u_{t-1})
+    // (nothing above reads what an earlier launch writes: the sponge table is
+    // fixed). The setup above runs under the end of the launch before: RTM 256^3
+    // 21.2 -> 20.7 ms, 150x203x171 7.08 -> 6.60 ms, 384x384x320 41.7 -> 41.4 ms.
+    pdl_wait();
+    pdl_launch();
     float scale_a = 0.0f, scale_b = 0.0f;
     if constexpr (BACK) {
         scale_a = __uint_as_float(*a.amax_in) / SNAP_QMAX;
@@ -1443,7 +1451,7 @@ int launch_step2_rows(const Layout& L, const FieldMaps& mcur, const FieldMaps& m
             configured = true;
         }
     }
-    const int chunks = fd_step_grid_chunks(L, G::TYV, G::MINB, 1, 4);
+    const int chunks = fd_step_grid_chunks(L, G::TYV, G::MINB, 1, 4, a.withhold ? 4 : 1);
     a.x_chunk = (int)((L.nx + chunks - 1) / chunks);
     const int nch = (int)((L.nx + a.x_chunk - 1) / a.x_chunk);
     dim3 grid((unsigned)((L.nz + TZ - 1) / TZ), (unsigned)((L.ny + G::TYV - 1) / G::TYV), (unsigned)nch);
@@ -1451,9 +1459,9 @@ int launch_step2_rows(const Layout& L, const FieldMaps& mcur, const FieldMaps& m
     const CUtensorMap& ms = im ? im->snap : mc.cur[0];
     const CUtensorMap& mi = im ? im->image : mc.cur[0];
     const CUtensorMap& ml = im ? im->illum : mc.cur[0];
-    fd_step2_kernel<MODE, SK, RAG><<<grid, NTHREADS, G::SMEM, st>>>(mcur.cur2, mprev.cur[0], mc.cur[0], ms, mi, ml, a);
+    ST_CUDA(launch_dependent(fd_step2_kernel<MODE, SK, RAG>, grid, dim3(NTHREADS), G::SMEM, st, mcur.cur2, mprev.cur[0],
+                             mc.cur[0], ms, mi, ml, a));
     ::stg::count_launch();
-    ST_CUDA(cudaGetLastError());
     return ST_OK;
 }
 
@@ -1686,7 +1694,7 @@ int build_field_maps(FieldMaps* m, const float* base, const Layout& L) {
     return ST_OK;
 }
 
-int fd_step_grid_chunks(const Layout& L, int tyv, int minb, int min_waves, int halo) {
+int fd_step_grid_chunks(const Layout& L, int tyv, int minb, int min_waves, int halo, int min_len) {
     const long long gx = (L.nz + TZ - 1) / TZ, gy = (L.ny + tyv - 1) / tyv;
     const long long tiles = gx * gy;
     // tuning override: SEISMIC_GB300_XCHUNKS=<chunks> (1..nx)
@@ -1701,6 +1709,14 @@ int fd_step_grid_chunks(const Layout& L, int tyv, int minb, int min_waves, int h
     long long best = 1;
     double best_eff = -1.0;
     const long long max_chunks = std::max<long long>(1, std::min<long long>(L.nx / 4, 256));
+    // A grid that leaves SMs idle even in chunks of four planes: the launch takes
+    // as long as one block's march (chunk + halo planes), so the chunks are as
+    // short as one wave of blocks allows. 48 x 40 x 56: one plane instead of 8,
+    // 5.7 -> 2.6 us per step; 128^3: 3 planes instead of 7, 8.4 -> 6.9 us. Past
+    // that line the recomputed halo planes cost bandwidth, and the search below
+    // weighs them.
+    if ((double)(tiles * max_chunks) <= slots)
+        return (int)std::max<long long>(1, std::min<long long>(L.nx / min_len, (long long)slots / tiles));
     const long long need = min_waves > 1 ? (long long)std::ceil(min_waves * slots / (double)tiles) : 1;
     const long long first = std::min<long long>(std::max<long long>(1, need), max_chunks);
     for (long long ch = first; ch <= max_chunks; ++ch) {
