@@ -25,6 +25,12 @@
 namespace stg {
 namespace {
 
+// Steps from which a resident shot is used. It starts its blocks and loads the
+// model once; whole shots by launches of two steps / resident: 24^3 4 steps
+// 45 / 50 us, 8 steps 58 / 58, 16 steps 75 / 67; 64^3 8 steps 61 / 59; 128^3 4
+// steps 71 / 69.
+constexpr int RES_MIN_STEPS = 8;
+
 // f[receiver q] += (c at q) * row[q] over a receiver grid (times the sponge
 // factor D at q with the stable sponge: mu = c D lambda).
 __global__ void rec_force_kernel(float* f, const float* c, Layout L, st_receiver_grid R, const float* row,
@@ -108,6 +114,18 @@ int shot_forward_impl(st_solver* s, const st_shot* shot, float* seis, int snap_k
     const int nt = shot->nt;
     const size_t per = (size_t)(L.nx * L.ny * cz) * (size_t)snap_bytes(snap_kind);
     if (snap_kind != SNAP_NONE) ST_CUDA(cudaMemsetAsync(amax, 0, sizeof(unsigned) * (size_t)(nt + 1), s->stream));
+    // a small grid without snapshots: every step in one launch. The switches of
+    // the chunked path (one step per launch, the wait limit and its test, a
+    // fixed chunking) select that path.
+    if (nt >= RES_MIN_STEPS && snap_kind == SNAP_NONE && s->fused_steps == 2 && !s->zlim && !(slices && s->slices) &&
+        !s->withhold && !s->wait_limit_ns && !std::getenv("SEISMIC_GB300_XCHUNKS")) {
+        StepArgs a = base_args(s, nullptr);
+        set_injection(a, shot->src_ix, shot->src_iy, shot->src_iz, 0.0f);
+        if (nrec > 0 && seis) set_receivers(a, R);
+        bool done = false;
+        ST_TRY(resident_shot(s, a, shot, nrec > 0 ? seis : nullptr, &done));
+        if (done) return ST_OK;
+    }
     const long long src = dev_index(s, shot->src_ix, shot->src_iy, shot->src_iz);
     float w = 0.0f;
     if (nt > 0 && finite_sample(shot->wavelet, shot->wavelet_len, 0, &w))

@@ -536,6 +536,7 @@ int st_solver_destroy(st_solver* s) {
     cudaFree(s->aux_buf);
     cudaFree(s->data_buf);
     cudaFree(s->ckpt_buf);
+    cudaFree(s->res_buf);
     cudaFree(s->zlim);
     cudaFree(s->vel_dev);
     for (int k = 0; k < 3; ++k)

@@ -94,6 +94,9 @@ struct st_solver {
     size_t data_cap = 0;
     void* ckpt_buf = nullptr;       // checkpointed adjoint: working set, state slots, segment snapshots
     size_t ckpt_cap = 0;
+    void* res_buf = nullptr;        // resident shots: exchange words and the wavelet
+    size_t res_cap = 0;
+    unsigned res_tag = 1;           // first tag of the next resident launch
     int sponge_mode = ST_SPONGE_REFERENCE;  // ST_SPONGE_STABLE: damp the new field (Cerjan form)
     unsigned long long wait_limit_ns = 0;   // bounded-wait limit of the stencil kernels (0: 2 s)
     int withhold = 0;                       // st_solver_set_wait_test: plane + 1 withheld at the next launch
@@ -147,6 +150,10 @@ int fused_step2_forward(st_solver* s, StepArgs a, int snap_out);
 // Two adjoint steps with the gradient epilogue in one launch (launch_fd_step2_grad).
 int fused_step2_grad(st_solver* s, StepArgs a, int snap_in, const CUtensorMap& msnap, const CUtensorMap& mgrad);
 int zero_fields(st_solver* s);
+// All steps of a forward shot without snapshots in one launch (st_resident.cu),
+// from zeroed fields to cur = u_nt, prev = u_{nt-1}; *done = false: not on this
+// grid, nothing launched.
+int resident_shot(st_solver* s, const StepArgs& a, const st_shot* shot, float* seis, bool* done);
 long long dev_index(const st_solver* s, int64_t ix, int64_t iy, int64_t iz);
 bool finite_sample(const double* w, int64_t len, int64_t t, float* out);
 inline void set_injection(StepArgs& a, int64_t ix, int64_t iy, int64_t iz, float val) {

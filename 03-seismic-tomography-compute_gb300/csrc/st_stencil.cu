@@ -38,6 +38,7 @@
 // a 3- or 4-deep mbarrier ring; u at x-1/x/x+1 rides in a register queue. HBM
 // traffic is 16 B per point (read u, prev, c; write out) plus the epilogue's.
 #include "st_kernels.cuh"
+#include "st_update.cuh"
 
 #include <algorithm>
 #include <cfloat>
@@ -180,60 +181,6 @@ __device__ __forceinline__ void snap_smem4(const unsigned char* tile, int e, flo
         const uint2 w = *reinterpret_cast<const uint2*>(reinterpret_cast<const unsigned short*>(tile) + e);
         snap_unpack4<K>(w, f);
     }
-}
-
-__device__ __forceinline__ void f4_to(const float4& v, float a[4]) {
-    a[0] = v.x;
-    a[1] = v.y;
-    a[2] = v.z;
-    a[3] = v.w;
-}
-
-// The update of one point: out = 2u - upd + c * L u, upd = D * prev.
-__device__ __forceinline__ float update_fast(float u, float upd, float xm, float xp, float ym, float yp, float zm,
-                                             float zp, float c, float ax, float ay, float az) {
-    const float lap = fmaf(-2.0f, u, xp + xm) * ax + fmaf(-2.0f, u, yp + ym) * ay + fmaf(-2.0f, u, zp + zm) * az;
-    return fmaf(c, lap, fmaf(2.0f, u, -upd));
-}
-
-// The reference's guarded update (wave_equation.cpp:342-399), taken only when
-// the fast result is non-finite or beyond the amplitude limit. A non-finite
-// input always makes the fast result non-finite (c, 1/d^2 > 0), so the fast
-// path is exact whenever it is taken. GINL: inlined at the call site (the
-// two-step kernels measured faster so); otherwise one out-of-line copy
-// shared by the call sites.
-template <bool GINL = false>
-__device__ __forceinline__ float update_guarded(float u, float upd, float xm, float xp, float ym, float yp, float zm,
-                                                float zp, float c, float ax, float ay, float az, float amp,
-                                                int* fired);
-__device__ __forceinline__ float guarded_body(float u, float upd, float xm, float xp, float ym, float yp, float zm,
-                                              float zp, float c, float ax, float ay, float az, float amp,
-                                              int* fired) {
-    if (!isfinite(u) || !isfinite(upd)) {
-        *fired = 1;
-        return 0.0f;
-    }
-    if (!isfinite(xm) || !isfinite(xp) || !isfinite(ym) || !isfinite(yp) || !isfinite(zm) || !isfinite(zp)) {
-        *fired = 1;
-        return u;
-    }
-    float nv = update_fast(u, upd, xm, xp, ym, yp, zm, zp, c, ax, ay, az);
-    if (!isfinite(nv)) {
-        nv = u;
-        *fired = 1;
-    }
-    return fminf(fmaxf(nv, -amp), amp);
-}
-__device__ __noinline__ float guarded_call(float u, float upd, float xm, float xp, float ym, float yp, float zm,
-                                           float zp, float c, float ax, float ay, float az, float amp, int* fired) {
-    return guarded_body(u, upd, xm, xp, ym, yp, zm, zp, c, ax, ay, az, amp, fired);
-}
-template <bool GINL>
-__device__ __forceinline__ float update_guarded(float u, float upd, float xm, float xp, float ym, float yp, float zm,
-                                                float zp, float c, float ax, float ay, float az, float amp,
-                                                int* fired) {
-    if constexpr (GINL) return guarded_body(u, upd, xm, xp, ym, yp, zm, zp, c, ax, ay, az, amp, fired);
-    else return guarded_call(u, upd, xm, xp, ym, yp, zm, zp, c, ax, ay, az, amp, fired);
 }
 
 // Per-row bookkeeping of one thread (4 consecutive z of one y row).
@@ -794,58 +741,6 @@ __device__ __forceinline__ int rec_line(int v, int v0, int sv, int nv) {
     const int d = v - v0;
     if (d < 0 || d % sv) return -1;
     return d / sv < nv ? d / sv : -1;
-}
-
-__device__ __forceinline__ void ld4(const float* p, float v[4]) { f4_to(*reinterpret_cast<const float4*>(p), v); }
-__device__ __forceinline__ void st4(float* p, const float v[4]) {
-    *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
-}
-
-// Four point updates in fd_step_kernel's order, first part: the update (the
-// guarded form where the fast one is out of range). The caller then adds the
-// adjoint receiver forcing, applies the stable damping (stable_damp4) and, in
-// the forward mode, samples the receivers and injects the source.
-template <bool GINL>
-__device__ __forceinline__ void update4(const StepArgs& a, const float u0[4], const float pv[4], const float um[4],
-                                        const float up[4], const float ym[4], const float yp[4], float zm0, float zp3,
-                                        const float cv[4], const float D[4], float res[4], int* fired) {
-    float upd[4];
-    bool bad = false;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const float zm = k == 0 ? zm0 : u0[k - 1];
-        const float zp = k == 3 ? zp3 : u0[k + 1];
-        upd[k] = D[k] * pv[k];
-        res[k] = update_fast(u0[k], upd[k], um[k], up[k], ym[k], yp[k], zm, zp, cv[k], a.ax, a.ay, a.az);
-        bad = bad || !(fabsf(res[k]) <= a.amp);
-    }
-    if (bad) {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            if (fabsf(res[k]) <= a.amp) continue;
-            const float zm = k == 0 ? zm0 : u0[k - 1];
-            const float zp = k == 3 ? zp3 : u0[k + 1];
-            res[k] = update_guarded<GINL>(u0[k], upd[k], um[k], up[k], ym[k], yp[k], zm, zp, cv[k], a.ax, a.ay, a.az,
-                                          a.amp, fired);
-        }
-    }
-}
-
-// The stable sponge mode damps the new values as well.
-__device__ __forceinline__ void stable_damp4(const StepArgs& a, const float D[4], float res[4]) {
-    if (a.stable_sponge) {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) res[k] *= D[k];
-    }
-}
-
-// Sponge factors of a 4-point group: D(min(dx, dyz)) for each point, formed
-// as min(D(dx), D(dyz)) from the plane's x factor Dx and the y/z factors Dyz
-// the thread looked up once (the table is non-decreasing in the distance and
-// at most 1, so this is bit for bit the same).
-__device__ __forceinline__ void sponge4f(float Dx, const float Dyz[4], float D[4]) {
-#pragma unroll
-    for (int k = 0; k < 4; ++k) D[k] = fminf(Dx, Dyz[k]);
 }
 
 // Laplacian of a snapshot at the four z of a centre group, scaled, with the
