@@ -125,16 +125,6 @@ __device__ __forceinline__ uint64_t smem_desc_sw64(uint32_t addr) {
 constexpr uint32_t idesc_n(int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
 }
-constexpr uint32_t IDESC = idesc_n(CH);
-
-__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(IDESC), "r"(accumulate)
-        : "memory");
-}
-
 // Accumulating form that leaves the TMEM lanes set in off[] as they are; the
 // descriptors as low and high words.
 __device__ __forceinline__ void mma_bf16_lanes(uint32_t tmem_d, uint32_t alo, uint32_t ahi, uint32_t blo, uint32_t bhi,
@@ -513,61 +503,70 @@ int make_rows_map(CUtensorMap* map, const __nv_bfloat16* base, long long rows, i
 // ---------------------------------------------------------------- weight gradient
 // dW[co][ci][tap] += sum over interior voxels v of g[v][co] x[v + s_tap][ci]
 // for a 32 -> 32 layer, on the tensor cores: an implicit GEMM with
-// M = (tap, ci) in 7 tiles of 4 taps x 32 input channels (the last tile has 3
-// taps), N = 32 output channels and K = the padded volume's rows q, split
-// over CTAs (each CTA one M tile and one K range; FP32 atomics add the
-// partial tiles). g's border rows are zeroed on the way in, so a K step may
-// run over them; x's border is zero by the padded convention, and rows past
-// the volume arrive as zeros from the TMA bounds fill.
+// M = (kw, ci), N = co and K = the padded volume's rows q, cut into 9 tiles
+// (kd, kh) and split over CTAs along K. g's border rows are zeroed on the way
+// in, so a K step may run over them; x's border is zero by the padded
+// convention, and rows past the volume arrive as zeros from the TMA bounds fill.
 //
-// Per K step of 64 rows the TMA brings [64 rows][32 ch] tiles of x (one per
-// tap of the tile, shifted by the tap's row offset) and of g into a ring of
-// raw stages. Channels-last rows are channel-contiguous, but both operands
-// of the contraction over q must be K-major (q contiguous): warps 2-5
-// transpose the tiles 8x8 at a time with ldmatrix.trans / stmatrix into the
-// canonical no-swizzle K-major layout (8 rows x 16-byte core matrices; A:
-// LBO 2048 between K blocks, SBO 128 between M blocks; B: LBO 512, SBO 128)
-// of an operand stage; warp 1 issues four tcgen05.mma (M=128, N=32, K=16) per
-// step into a 32-column TMEM accumulator; warps 2-5 then read it back
-// (tcgen05.ld) and add it to dW. Every wait is bounded as in the forward conv.
-constexpr int WG_KSTEP = 64;
-constexpr int WG_TILES = 7;
-constexpr int WG_NRAW = 3;
-constexpr int WG_NOP = 2;
-constexpr int WG_RAW_TILE = WG_KSTEP * CH * 2;  // 4096
-constexpr int WG_RAW_BYTES = 5 * WG_RAW_TILE;   // four x tiles + the g tile
-constexpr int WG_A_BYTES = TM * WG_KSTEP * 2;   // 16384
-constexpr int WG_B_BYTES = CH * WG_KSTEP * 2;   // 4096
-constexpr int WG_OP_BYTES = WG_A_BYTES + WG_B_BYTES;
+// Both operands are contiguous along their channels (M and N) in memory, and the
+// matrix unit takes them so: a 64-byte swizzled tile of rows is its M-major
+// layout, 32 channels wide, eight rows (K) every 512 bytes. The three kw taps are
+// the same rows of x one row apart, so one window of x serves them: the M
+// blocks of an instruction lie 64 bytes, one row, apart (the fourth, kw = 2, is
+// not used). Per K step of 128 rows the TMA brings that window and g's rows into
+// a ring of slots, warps 2-5 zero g's border rows, and warp 1 issues eight
+// tcgen05.mma (M = 128, N = 32, K = 16), in turn into four accumulators so that
+// no sum runs longer than a quarter of the K range. The epilogue adds the four,
+// turns them through shared memory and adds them to dW (FP32 atomics, three
+// neighbouring taps each). Every wait is bounded as in the forward conv.
+//
+// 32^3: 13.3 us, 100^3: 176 us (316 TFLOP/s of the products counted, bound by the
+// 32-column instructions, a quarter of whose rows is not used). Transposing both
+// operands through registers (ldmatrix / stmatrix) to K-major tiles of four taps
+// took 37.5 and 606 us, bound by the transposes and by the atomics of 44 partial
+// sums per weight. Error against 64 bits 4.4e-7 and 1.7e-5 (7.7e-7 and 2.7e-5).
+constexpr int WG_KSTEP = 128;
+constexpr int WG_TILES = 9;
+constexpr int WG_SLOTS = 6;
+constexpr int WG_X_ROWS = WG_KSTEP + 8;              // kw = -1 .. 2, in whole groups of eight rows
+constexpr int WG_X_BYTES = WG_X_ROWS * CH * 2;
+constexpr int WG_SLOT_BYTES = WG_X_BYTES + WG_KSTEP * CH * 2;
+constexpr int WG_ACC = 4;
 constexpr int WG_THREADS = 192;
-constexpr int WG_TMEM_COLS = 32;
+constexpr int WG_TMEM_COLS = WG_ACC * CH;
+static_assert(WG_X_BYTES % 512 == 0 && WG_SLOT_BYTES % 512 == 0, "swizzle blocks");
 
 struct WgradArgs {
     float* dw;
     int D, H, W;
-    long long rows;  // (D+2)(H+2)(W+2)
-    int ksteps;      // ceil(rows / 64)
-    int splits;      // CTAs per M tile
+    int ksteps;      // ceil((D+2)(H+2)(W+2) / WG_KSTEP)
+    int splits;      // CTAs per tile
     unsigned* flags;
     unsigned long long timeout_ns;
 };
 
 struct WgradSmem {
-    uint64_t raw_full[WG_NRAW], raw_empty[WG_NRAW], op_full[WG_NOP], op_empty[WG_NOP], done;
+    uint64_t full[WG_SLOTS], ready[WG_SLOTS], empty[WG_SLOTS], done;
     uint32_t tmem_base;
     int abort;
 };
 
-__device__ __forceinline__ void ldsm_x4_trans(uint32_t addr, uint32_t r[4]) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(addr)
-                 : "memory");
+// Descriptor of an M-major (N-major) operand, 64-byte swizzled: blocks of 32
+// channels every lbo bytes, groups of eight rows every 512 bytes.
+__device__ __forceinline__ uint64_t smem_desc_mn64(uint32_t addr, uint32_t lbo) {
+    return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(512u >> 4) << 32) |
+           (1ull << 46) | (4ull << 61);
 }
-__device__ __forceinline__ void stsm_x4(uint32_t addr, const uint32_t r[4]) {
-    asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(r[0]),
-                 "r"(r[1]), "r"(r[2]), "r"(r[3])
-                 : "memory");
+constexpr uint32_t WG_IDESC = idesc_n(CH) | (1u << 15) | (1u << 16);  // A and B M- / N-major
+
+__device__ __forceinline__ void mma_bf16_words(uint32_t tmem_d, uint32_t alo, uint32_t ahi, uint32_t blo, uint32_t bhi,
+                                               uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %6, 0;\n\tmov.b64 da, {%1, %2};\n\t"
+        "mov.b64 db, {%3, %4};\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t}" ::"r"(tmem_d),
+        "r"(alo), "r"(ahi), "r"(blo), "r"(bhi), "r"(idesc), "r"(accumulate)
+        : "memory");
 }
 __device__ __forceinline__ void named_sync_128() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
@@ -575,13 +574,10 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
     conv32_wgrad_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant__ CUtensorMap mg,
                            const WgradArgs a) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    unsigned char* raw = smem;
-    unsigned char* ops = smem + WG_NRAW * WG_RAW_BYTES;
-    WgradSmem* cs = reinterpret_cast<WgradSmem*>(ops + WG_NOP * WG_OP_BYTES);
+    unsigned char* slots = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    WgradSmem* cs = reinterpret_cast<WgradSmem*>(slots + WG_SLOTS * WG_SLOT_BYTES);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tile = blockIdx.x % WG_TILES, split = blockIdx.x / WG_TILES;
-    const int ntap = tile == WG_TILES - 1 ? NTAP - 4 * (WG_TILES - 1) : 4;
     const int k0 = (int)((long long)a.ksteps * split / a.splits);
     const int nk = (int)((long long)a.ksteps * (split + 1) / a.splits) - k0;
     const int W2 = a.W + 2;
@@ -590,13 +586,10 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
     const uint64_t dlim = lim > WAIT_DRAIN_NS ? lim : WAIT_DRAIN_NS;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < WG_NRAW; ++s) {
-            mbar_init(&cs->raw_full[s], 1);
-            mbar_init(&cs->raw_empty[s], 128);
-        }
-        for (int s = 0; s < WG_NOP; ++s) {
-            mbar_init(&cs->op_full[s], 128);
-            mbar_init(&cs->op_empty[s], 1);
+        for (int s = 0; s < WG_SLOTS; ++s) {
+            mbar_init(&cs->full[s], 1);
+            mbar_init(&cs->ready[s], 128);
+            mbar_init(&cs->empty[s], 1);
         }
         mbar_init(&cs->done, 1);
         cs->abort = 0;
@@ -616,154 +609,115 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
 
     if (warp == 0) {
         if (lane == 0) {
+            const int shift = (tile / 3 - 1) * PL + (tile % 3 - 1) * W2 - 1;
             int k = 0;
             for (; k < nk; ++k) {
-                const int s = k % WG_NRAW;
-                if (k >= WG_NRAW && !mbar_wait_bounded(&cs->raw_empty[s], ((k / WG_NRAW) - 1) & 1, lim)) {
+                const int s = k % WG_SLOTS;
+                if (k >= WG_SLOTS && !mbar_wait_bounded(&cs->empty[s], ((k / WG_SLOTS) - 1) & 1, lim)) {
                     atomicOr(a.flags, CONV_FLAG_TIMEOUT);
                     cs->abort = 1;
                     break;
                 }
                 if (read_abort(&cs->abort)) break;
                 const int q0 = (k0 + k) * WG_KSTEP;
-                unsigned char* rb = raw + s * WG_RAW_BYTES;
-                mbar_arrive_expect_tx(&cs->raw_full[s], (uint32_t)(ntap + 1) * WG_RAW_TILE);
-                for (int t = 0; t < ntap; ++t) {
-                    const int tap = 4 * tile + t;
-                    const int shift = (tap / 9 - 1) * PL + ((tap / 3) % 3 - 1) * W2 + (tap % 3 - 1);
-                    tma_load_2d(rb + t * WG_RAW_TILE, &mx, &cs->raw_full[s], 0, q0 + shift);
-                }
-                tma_load_2d(rb + 4 * WG_RAW_TILE, &mg, &cs->raw_full[s], 0, q0);
+                unsigned char* sb = slots + s * WG_SLOT_BYTES;
+                mbar_arrive_expect_tx(&cs->full[s], WG_SLOT_BYTES);
+                tma_load_2d(sb, &mx, &cs->full[s], 0, q0 + shift);
+                tma_load_2d(sb + WG_X_BYTES, &mg, &cs->full[s], 0, q0);
             }
-            // drain: every issued stage has landed before the CTA may exit
-            for (int f = (k > WG_NRAW ? k - WG_NRAW : 0); f < k; ++f)
-                if (!mbar_wait_bounded(&cs->raw_full[f % WG_NRAW], (f / WG_NRAW) & 1, dlim))
+            // drain: every issued slot has landed before the CTA may exit
+            for (int f = (k > WG_SLOTS ? k - WG_SLOTS : 0); f < k; ++f)
+                if (!mbar_wait_bounded(&cs->full[f % WG_SLOTS], (f / WG_SLOTS) & 1, dlim))
                     atomicOr(a.flags, CONV_FLAG_TIMEOUT);
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            int k = 0;
-            for (; k < nk; ++k) {
-                const int o = k % WG_NOP;
-                if (!mbar_wait_bounded(&cs->op_full[o], (k / WG_NOP) & 1, lim) || read_abort(&cs->abort)) {
-                    atomicOr(a.flags, CONV_FLAG_TIMEOUT);
-                    cs->abort = 1;
-                    break;
-                }
-                tc_fence_after();
-                const uint32_t ab = smem_u32(ops + o * WG_OP_BYTES), bb = ab + WG_A_BYTES;
+        // the whole warp runs the loop and one elected lane issues (as in the forward conv)
+        bool ok = true;
+        const uint32_t slots4 = smem_u32(slots) >> 4;
+        const uint64_t ad = smem_desc_mn64(0, CH * 2), bd = smem_desc_mn64(WG_X_BYTES, 512);
+        const uint32_t alo0 = (uint32_t)ad + slots4, ahi = (uint32_t)(ad >> 32), blo0 = (uint32_t)bd + slots4,
+                       bhi = (uint32_t)(bd >> 32);
+        for (int k = 0; k < nk; ++k) {
+            const int s = k % WG_SLOTS;
+            if (!__all_sync(0xffffffffu,
+                            mbar_wait_bounded(&cs->ready[s], (k / WG_SLOTS) & 1, lim) && !read_abort(&cs->abort))) {
+                ok = false;
+                break;
+            }
+            tc_fence_after();
+            const uint32_t off = (uint32_t)s * (WG_SLOT_BYTES / 16);
+            if (elect_one()) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    mma_bf16(tmem, smem_desc(ab + (uint32_t)j * 4096u, 2048u, 128u),
-                             smem_desc(bb + (uint32_t)j * 1024u, 512u, 128u), (k | j) != 0);
-                mma_commit(&cs->op_empty[o]);
+                for (int j = 0; j < WG_KSTEP / 16; ++j)  // 16 rows of 64 bytes each
+                    mma_bf16_words(tmem + (uint32_t)(j % WG_ACC) * CH, alo0 + off + j * 64u, ahi, blo0 + off + j * 64u, bhi,
+                                   WG_IDESC, j >= WG_ACC || k > 0);
+                mma_commit(&cs->empty[s]);
             }
-            // the last commit tracks every MMA issued: the accumulator is final
-            // (and, after an abort, no MMA is left running when TMEM is freed)
-            if (k > 0) {
-                mma_commit(&cs->done);
-                if (!mbar_wait_bounded(&cs->done, 0, dlim)) atomicOr(a.flags, CONV_FLAG_TIMEOUT);
-            }
+            __syncwarp();
         }
+        if (!ok && lane == 0) {
+            atomicOr(a.flags, CONV_FLAG_TIMEOUT);
+            cs->abort = 1;
+        }
+        // the last commit tracks every MMA issued: the accumulators are final
+        // (and, after an abort, no MMA is left running when TMEM is freed)
+        if (elect_one()) {
+            mma_commit(&cs->done);
+            if (!mbar_wait_bounded(&cs->done, 0, dlim)) atomicOr(a.flags, CONV_FLAG_TIMEOUT);
+        }
+        __syncwarp();
     } else {
-        // warps 2-5: transposes, then the epilogue. The four warps meet at a
-        // named barrier every step, so none leaves the loop early: after a
-        // failed wait (or another warp's abort) a warp stops waiting and
-        // working but still takes every barrier.
-        const int tt = threadIdx.x - 64, tw = warp - 2;
-        // this lane's row of each of the warp's ten groups of four 8 x 8 blocks
-        // (groups tw, tw + 4, ...; A: 4 taps x 8 row blocks x 4 channel blocks,
-        // B: 8 x 4): source offset in a raw stage, destination offset in an
-        // operand stage. The raw tiles arrive 64-byte swizzled (16-byte chunk c
-        // of row v at chunk c ^ ((v >> 1) & 3)), so the eight rows an ldmatrix
-        // reads fall in eight different bank groups.
-        constexpr uint32_t SKIP = 0xffffffffu;
-        uint32_t so[10], dof[10];
-        {
-            const int r = lane & 7;
-#pragma unroll
-            for (int j = 0; j < 10; ++j) {
-                const int b = (tw + 4 * j) * 4 + (lane >> 3);
-                int t, vb, cb;
-                uint32_t dst;
-                if (b < 128) {
-                    t = b >> 5;
-                    vb = (b & 31) >> 2;
-                    cb = b & 3;
-                    dst = (uint32_t)(vb * 2048 + (t * 4 + cb) * 128 + r * 16);
-                } else {
-                    t = 4;
-                    vb = (b - 128) >> 2;
-                    cb = (b - 128) & 3;
-                    dst = (uint32_t)(WG_A_BYTES + vb * 512 + cb * 128 + r * 16);
-                }
-                const int row = vb * 8 + r;
-                so[j] = (b < 128 && t >= ntap) ? SKIP  // uniform over the group (32 blocks per tap)
-                                               : (uint32_t)(t * WG_RAW_TILE + row * (CH * 2) + ((cb ^ ((row >> 1) & 3)) << 4));
-                dof[j] = dst;
-            }
-        }
+        const int tt = threadIdx.x - 64;
         bool ok = true;
         for (int k = 0; k < nk; ++k) {
-            const int s = k % WG_NRAW, o = k % WG_NOP;
-            if (ok) {
-                bool w = !read_abort(&cs->abort) && mbar_wait_bounded(&cs->raw_full[s], (k / WG_NRAW) & 1, lim);
-                if (w && k >= WG_NOP) w = mbar_wait_bounded(&cs->op_empty[o], ((k / WG_NOP) - 1) & 1, lim);
-                // ldmatrix / stmatrix are warp-collective: a warp-uniform outcome
-                if (!__all_sync(0xffffffffu, w && !read_abort(&cs->abort))) {
-                    if (lane == 0) atomicOr(a.flags, CONV_FLAG_TIMEOUT);
-                    cs->abort = 1;
-                    ok = false;
-                }
+            const int s = k % WG_SLOTS;
+            if (!mbar_wait_bounded(&cs->full[s], (k / WG_SLOTS) & 1, lim) || read_abort(&cs->abort)) {
+                atomicOr(a.flags, CONV_FLAG_TIMEOUT);
+                cs->abort = 1;
+                ok = false;
+                break;
             }
-            unsigned char* rb = raw + s * WG_RAW_BYTES;
-            unsigned char* ob = ops + o * WG_OP_BYTES;
-            if (ok && tt < WG_KSTEP) {
-                // g rows outside the interior contribute nothing
-                const long long q = (long long)(k0 + k) * WG_KSTEP + tt;
-                const int d = (int)(q / PL), rem = (int)(q - (long long)d * PL), h = rem / W2, wv = rem - h * W2;
-                const bool inside = d >= 1 && d <= a.D && h >= 1 && h <= a.H && wv >= 1 && wv <= a.W;
-                if (!inside) {
-                    uint4* row = reinterpret_cast<uint4*>(rb + 4 * WG_RAW_TILE + tt * (CH * 2));
+            // g rows outside the interior contribute nothing (rows past the volume are zero already)
+            const unsigned q = (unsigned)(k0 + k) * WG_KSTEP + tt;
+            const unsigned d = q / (unsigned)PL, rem = q - d * PL, h = rem / (unsigned)W2, w = rem - h * W2;
+            if (d - 1u >= (unsigned)a.D || h - 1u >= (unsigned)a.H || w - 1u >= (unsigned)a.W) {
+                uint4* row = reinterpret_cast<uint4*>(slots + s * WG_SLOT_BYTES + WG_X_BYTES + tt * (CH * 2));
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) row[j] = make_uint4(0u, 0u, 0u, 0u);
-                }
+                for (int j = 0; j < 4; ++j) row[j] = make_uint4(0u, 0u, 0u, 0u);
             }
-            named_sync_128();
-            if (!ok) continue;
-            // four 8 x 8 blocks per ldmatrix / stmatrix pair; lane l addresses row
-            // l % 8 of block l / 8 of the group
-            const uint32_t rbu = smem_u32(rb), obu = smem_u32(ob);
-#pragma unroll
-            for (int j = 0; j < 10; ++j) {
-                if (so[j] == SKIP) continue;
-                uint32_t v4[4];
-                ldsm_x4_trans(rbu + so[j], v4);
-                stsm_x4(obu + dof[j], v4);
-            }
-            // generic-proxy writes read by the tensor cores, and a raw stage the
-            // TMA overwrites next
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            mbar_arrive(&cs->op_full[o]);
-            mbar_arrive(&cs->raw_empty[s]);
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic writes read by the tensor cores
+            mbar_arrive(&cs->ready[s]);
         }
-        if (ok && nk > 0) {
-            const bool got = __all_sync(0xffffffffu, mbar_wait_bounded(&cs->done, 0, dlim));
-            if (!got) {
-                if (lane == 0) atomicOr(a.flags, CONV_FLAG_TIMEOUT);
-            } else {
-                tc_fence_after();
-                const int quarter = warp & 3;  // TMEM lanes 32 quarter .. : tap quarter of the tile, ci = lane
-                float v[CH];
-                tmem_ld32(tmem + ((uint32_t)(quarter * 32) << 16), v);
-                tc_fence_before();
-                if (quarter < ntap) {
-                    const int tap = 4 * tile + quarter;
-#pragma unroll
-                    for (int co = 0; co < CH; ++co) atomicAdd(&a.dw[((size_t)co * CH + lane) * NTAP + tap], v[co]);
-                }
-            }
+        if (ok) ok = mbar_wait_bounded(&cs->done, 0, dlim) && !read_abort(&cs->abort);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok && lane == 0) {
+            atomicOr(a.flags, CONV_FLAG_TIMEOUT);
+            cs->abort = 1;
         }
+        // every slot has been read: the sums go through the first one, [co][ci][kw]
+        float* out = reinterpret_cast<float*>(slots);
+        const int kw = warp & 3;  // TMEM lanes 32 kw .. : lane = ci
+        if (ok && kw < 3) {
+            tc_fence_after();
+            float v[CH];
+            tmem_ld32(tmem + ((uint32_t)(kw * 32) << 16), v);
+#pragma unroll
+            for (int i = 1; i < WG_ACC; ++i) {
+                float t[CH];
+                tmem_ld32(tmem + ((uint32_t)(kw * 32) << 16) + (uint32_t)i * CH, t);
+#pragma unroll
+                for (int co = 0; co < CH; ++co) v[co] += t[co];
+            }
+            tc_fence_before();
+#pragma unroll
+            for (int co = 0; co < CH; ++co) out[(co * CH + lane) * 3 + kw] = v[co];
+        }
+        named_sync_128();
+        if (!read_abort(&cs->abort))
+            for (int i = tt; i < CH * CH * 3; i += 128) {
+                const int cc = i / 3;
+                atomicAdd(&a.dw[(size_t)cc * NTAP + tile * 3 + (i - cc * 3)], out[i]);
+            }
     }
     __syncthreads();
     if (warp == 1) {
@@ -899,7 +853,7 @@ int st_conv3d_wgrad(const void* x, const void* g, float* dw, int64_t nx, int64_t
     const long long rows = (nx + 2) * (ny + 2) * (nz + 2);
     ST_CHECK(rows + (ny + 2) * (nz + 2) + nz + 3 < (1ll << 31), ST_ERR_ARG, "volume too large");
     CUtensorMap mx, mg;
-    ST_TRY(make_rows_map(&mx, static_cast<const __nv_bfloat16*>(x), rows, WG_KSTEP));
+    ST_TRY(make_rows_map(&mx, static_cast<const __nv_bfloat16*>(x), rows, WG_X_ROWS));
     ST_TRY(make_rows_map(&mg, static_cast<const __nv_bfloat16*>(g), rows, WG_KSTEP));
     unsigned* flags = nullptr;
     ST_CUDA(cudaGetSymbolAddress(reinterpret_cast<void**>(&flags), g_conv_flags));
@@ -908,13 +862,12 @@ int st_conv3d_wgrad(const void* x, const void* g, float* dw, int64_t nx, int64_t
     a.D = (int)nx;
     a.H = (int)ny;
     a.W = (int)nz;
-    a.rows = rows;
     a.ksteps = (int)((rows + WG_KSTEP - 1) / WG_KSTEP);
-    // two CTAs per SM over the 7 M tiles, at least one K step each
-    a.splits = (int)std::max<long long>(1, std::min<long long>(a.ksteps, (2LL * num_sms_conv() + WG_TILES - 1) / WG_TILES));
+    // one CTA per SM over the 9 tiles, at least one K step each
+    a.splits = std::max(1, std::min(a.ksteps, num_sms_conv() / WG_TILES));
     a.flags = flags;
     a.timeout_ns = 2000000000ull;
-    const size_t smem = (size_t)WG_NRAW * WG_RAW_BYTES + (size_t)WG_NOP * WG_OP_BYTES + sizeof(WgradSmem) + 1024;
+    const size_t smem = (size_t)WG_SLOTS * WG_SLOT_BYTES + sizeof(WgradSmem) + 1024;
     static std::once_flag once;
     static cudaError_t attr = cudaSuccess;
     std::call_once(once, [&] {
