@@ -49,3 +49,27 @@ def test_wgrad_edges(se, shape):
     ref += start.double().numpy().reshape(32, 32, 27)
     got = dw.cpu().double().numpy().reshape(32, 32, 27)
     assert np.linalg.norm(got - ref) <= 3e-5 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1), (1, 9, 8), (5, 8, 9), (3, 17, 33), (32, 32, 32), (2, 7, 300)])
+def test_one_channel_wgrad_edges(se, shape):
+    import torch
+    from seismic_engine._lib import call
+    st = torch.cuda.current_stream().cuda_stream
+    D, H, W = shape
+    gen = torch.Generator().manual_seed(sum(shape))
+    h = torch.zeros((D + 2, H + 2, W + 2, 32))
+    h[1:-1, 1:-1, 1:-1] = torch.randn((D, H, W, 32), generator=gen)
+    hb = h.bfloat16()
+    dz = torch.randn((D, H, W), generator=gen)
+    start = torch.randn(32 * 27, generator=gen)
+    dw, dzd, hd = start.cuda(), dz.cuda(), hb.cuda()
+    call("st_pc_conv1_wgrad", dzd.data_ptr(), hd.data_ptr(), dw.data_ptr(), D, H, W, st)
+    torch.cuda.synchronize()
+    hf, g = hb.double().numpy(), dz.double().numpy().reshape(-1)
+    ref = start.double().numpy().reshape(32, 27).copy()
+    for tap in range(27):
+        kd, kh, kw = tap // 9, (tap // 3) % 3, tap % 3
+        ref[:, tap] += g @ hf[kd:kd + D, kh:kh + H, kw:kw + W].reshape(-1, 32)
+    got = dw.cpu().double().numpy().reshape(32, 27)
+    assert np.linalg.norm(got - ref) <= 3e-5 * np.linalg.norm(ref)
