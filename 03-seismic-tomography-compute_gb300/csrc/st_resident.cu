@@ -149,8 +149,14 @@ __device__ __noinline__ float4 guarded_group(const float* own, const float* pvp,
     f4_to(Dyz4, Dyz);
     sponge4f(Dx, Dyz, D);
     int fired = 0;
-    update4<true>(a, u, pv, um, up, ym, yp, zm0, zp3, cv, D, res, &fired);
-    stable_damp4(a, D, res);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float zm = k == 0 ? zm0 : u[k - 1], zp = k == 3 ? zp3 : u[k + 1], upd = D[k] * pv[k];
+        res[k] = update_fast(u[k], upd, um[k], up[k], ym[k], yp[k], zm, zp, cv[k], a.ax, a.ay, a.az);
+        if (!(fabsf(res[k]) <= a.amp))
+            res[k] = guarded_body(u[k], upd, um[k], up[k], ym[k], yp[k], zm, zp, cv[k], a.ax, a.ay, a.az, a.amp, &fired);
+    }
+    if (a.stable_sponge) damp4(D, res);
     if (fired) atomicOr(a.flags, FLAG_GUARD);
     return make_float4(res[0], res[1], res[2], res[3]);
 }

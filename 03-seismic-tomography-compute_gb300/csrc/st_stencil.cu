@@ -780,7 +780,8 @@ struct PlaneKind {
 // grid; the points beyond it hold 0 (they are stored, into the field's zero halo
 // and the compact rows' padding). A variant of its own: the masks tested at run
 // time cost the aligned grids 1-10%.
-template <int MODE, int SK, bool RAG>
+// STABLE: the stable sponge rule (StepArgs::stable_sponge).
+template <int MODE, int SK, bool RAG, bool STABLE>
 __global__ void __launch_bounds__(NTHREADS, (Geo2<MODE, SK>::MINB))
     fd_step2_kernel(const __grid_constant__ CUtensorMap map_cur, const __grid_constant__ CUtensorMap map_prev,
                     const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_snap,
@@ -1046,7 +1047,7 @@ __global__ void __launch_bounds__(NTHREADS, (Geo2<MODE, SK>::MINB))
                             if (k == rk) lp[k] = fmaf(cnow[k], a.force_row[q], lp[k]);
                     }
                 }
-                stable_damp4(a, D, lp);
+                if constexpr (STABLE) damp4(D, lp);
                 if constexpr (FWD) {
                     if (special) {
                         if (own && rc) {
@@ -1102,7 +1103,7 @@ __global__ void __launch_bounds__(NTHREADS, (Geo2<MODE, SK>::MINB))
                                                    &fired);
                     if (BACK && special && irx_a >= 0 && iry_q >= 0)
                         res = fmaf(c, a.force_row[irx_a * a.rny + iry_q], res);
-                    if (a.stable_sponge) res *= D;
+                    if constexpr (STABLE) res *= D;
                     if (FWD && special && inj_a && inj_q) res += a.inj_val;
                 }
                 Lw[rq] = res;
@@ -1129,7 +1130,7 @@ __global__ void __launch_bounds__(NTHREADS, (Geo2<MODE, SK>::MINB))
                         if (k == rk) res[k] = fmaf(cprev[k], a.force_row2[q], res[k]);
                 }
             }
-            stable_damp4(a, D, res);
+            if constexpr (STABLE) damp4(D, res);
             if constexpr (FWD) {
                 if (special) {
                     if (rc) {
@@ -1167,7 +1168,7 @@ __global__ void __launch_bounds__(NTHREADS, (Geo2<MODE, SK>::MINB))
                 ld4(st_ill(csp) + ccen, il);
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
-                    const float w = a.stable_sponge ? cprev[k] * D[k] : cprev[k];
+                    const float w = STABLE ? cprev[k] * D[k] : cprev[k];
                     float f = fa[k] * scale_a;
                     float ad = __fdividef(um[k], w);
                     if (!(fabsf(f) <= FLT_MAX)) f = 0.0f;  // not finite
@@ -1332,7 +1333,7 @@ __global__ void __launch_bounds__(NTHREADS, (Geo2<MODE, SK>::MINB))
     }
 }
 
-template <int MODE, int SK, bool RAG>
+template <int MODE, int SK, bool RAG, bool STABLE>
 int launch_step2_rows(const Layout& L, const FieldMaps& mcur, const FieldMaps& mprev, const FieldMaps& mc,
                          const ImageMaps* im, StepArgs a, cudaStream_t st) {
     using G = Geo2<MODE, SK>;
@@ -1341,7 +1342,7 @@ int launch_step2_rows(const Layout& L, const FieldMaps& mcur, const FieldMaps& m
     {
         std::lock_guard<std::mutex> lk(mu);
         if (!configured) {
-            ST_CUDA(cudaFuncSetAttribute(fd_step2_kernel<MODE, SK, RAG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            ST_CUDA(cudaFuncSetAttribute(fd_step2_kernel<MODE, SK, RAG, STABLE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          G::SMEM));
             configured = true;
         }
@@ -1354,7 +1355,7 @@ int launch_step2_rows(const Layout& L, const FieldMaps& mcur, const FieldMaps& m
     const CUtensorMap& ms = im ? im->snap : mc.cur[0];
     const CUtensorMap& mi = im ? im->image : mc.cur[0];
     const CUtensorMap& ml = im ? im->illum : mc.cur[0];
-    ST_CUDA(launch_dependent(fd_step2_kernel<MODE, SK, RAG>, grid, dim3(NTHREADS), G::SMEM, st, mcur.cur2, mprev.cur[0],
+    ST_CUDA(launch_dependent(fd_step2_kernel<MODE, SK, RAG, STABLE>, grid, dim3(NTHREADS), G::SMEM, st, mcur.cur2, mprev.cur[0],
                              mc.cur[0], ms, mi, ml, a));
     ::stg::count_launch();
     return ST_OK;
@@ -1365,8 +1366,10 @@ int launch_step2_variant(const Layout& L, const FieldMaps& mcur, const FieldMaps
                          const ImageMaps* im, StepArgs a, cudaStream_t st) {
     if constexpr (MODE != MODE_GRAD)  // gradients take aligned rows only
         if (a.cz != a.nz || a.nz % 4 != 0)
-            return launch_step2_rows<MODE, SK, true>(L, mcur, mprev, mc, im, a, st);
-    return launch_step2_rows<MODE, SK, false>(L, mcur, mprev, mc, im, a, st);
+            return a.stable_sponge ? launch_step2_rows<MODE, SK, true, true>(L, mcur, mprev, mc, im, a, st)
+                                   : launch_step2_rows<MODE, SK, true, false>(L, mcur, mprev, mc, im, a, st);
+    return a.stable_sponge ? launch_step2_rows<MODE, SK, false, true>(L, mcur, mprev, mc, im, a, st)
+                           : launch_step2_rows<MODE, SK, false, false>(L, mcur, mprev, mc, im, a, st);
 }
 
 int num_sms() {

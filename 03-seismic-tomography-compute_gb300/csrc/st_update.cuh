@@ -66,23 +66,65 @@ __device__ __forceinline__ void st4(float* p, const float v[4]) {
     *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
 }
 
+// Two values per instruction, each rounded as the scalar form rounds it.
+struct F2 {
+    unsigned long long v;
+};
+__device__ __forceinline__ F2 pack(float x, float y) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ void unpack(F2 a, float& x, float& y) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
+}
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+// update_fast of two points, with the contractions the compiler makes of it:
+// lap = fma(lz, az, fma(lx, ax, ly * ay)); nD = -D.
+__device__ __forceinline__ F2 update2(F2 u, F2 nD, F2 pv, F2 xs, F2 ys, F2 zs, F2 c, float ax, float ay, float az) {
+    const F2 m2 = pack(-2.0f, -2.0f), p2 = pack(2.0f, 2.0f);
+    const F2 lx = fma2(m2, u, xs), ly = fma2(m2, u, ys), lz = fma2(m2, u, zs);
+    const F2 lap = fma2(lz, pack(az, az), fma2(lx, pack(ax, ax), mul2(ly, pack(ay, ay))));
+    return fma2(c, lap, fma2(p2, u, mul2(nD, pv)));
+}
+
 // Four point updates in fd_step_kernel's order, first part: the update (the
-// guarded form where the fast one is out of range). The caller then adds the
-// adjoint receiver forcing, applies the stable damping (stable_damp4) and, in
-// the forward mode, samples the receivers and injects the source.
+// guarded form where the fast one is out of range), two points per instruction:
+// the two-step kernels are bound by the latency of their instructions more than
+// by memory (issue slots 50% busy, 39% of the DRAM rate at 192^3). With the sponge
+// rule a compile-time choice: 150 x 203 x 171 RTM 6.60 -> 6.43 ms, 192^3 FWI 22.0 ->
+// 21.7, 384 x 384 x 320 41.3 -> 40.4, 256^3 RTM 21.0 -> 20.9; the sponge rule alone gives
+// about half. The caller then adds the adjoint receiver forcing, applies the
+// stable damping (damp4) and, in the forward mode, samples the receivers and
+// injects the source.
 template <bool GINL>
 __device__ __forceinline__ void update4(const StepArgs& a, const float u0[4], const float pv[4], const float um[4],
                                         const float up[4], const float ym[4], const float yp[4], float zm0, float zp3,
                                         const float cv[4], const float D[4], float res[4], int* fired) {
-    float upd[4];
     bool bad = false;
+    const float zs[4] = {u0[1] + zm0, u0[2] + u0[0], u0[3] + u0[1], zp3 + u0[2]};
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const float zm = k == 0 ? zm0 : u0[k - 1];
-        const float zp = k == 3 ? zp3 : u0[k + 1];
-        upd[k] = D[k] * pv[k];
-        res[k] = update_fast(u0[k], upd[k], um[k], up[k], ym[k], yp[k], zm, zp, cv[k], a.ax, a.ay, a.az);
-        bad = bad || !(fabsf(res[k]) <= a.amp);
+    for (int j = 0; j < 4; j += 2) {
+        const F2 xs = add2(pack(up[j], up[j + 1]), pack(um[j], um[j + 1]));
+        const F2 ys = add2(pack(yp[j], yp[j + 1]), pack(ym[j], ym[j + 1]));
+        unpack(update2(pack(u0[j], u0[j + 1]), pack(-D[j], -D[j + 1]), pack(pv[j], pv[j + 1]), xs, ys,
+                       pack(zs[j], zs[j + 1]), pack(cv[j], cv[j + 1]), a.ax, a.ay, a.az),
+               res[j], res[j + 1]);
+        bad = bad || !(fabsf(res[j]) <= a.amp) || !(fabsf(res[j + 1]) <= a.amp);
     }
     if (bad) {
 #pragma unroll
@@ -90,18 +132,16 @@ __device__ __forceinline__ void update4(const StepArgs& a, const float u0[4], co
             if (fabsf(res[k]) <= a.amp) continue;
             const float zm = k == 0 ? zm0 : u0[k - 1];
             const float zp = k == 3 ? zp3 : u0[k + 1];
-            res[k] = update_guarded<GINL>(u0[k], upd[k], um[k], up[k], ym[k], yp[k], zm, zp, cv[k], a.ax, a.ay, a.az,
+            res[k] = update_guarded<GINL>(u0[k], D[k] * pv[k], um[k], up[k], ym[k], yp[k], zm, zp, cv[k], a.ax, a.ay, a.az,
                                           a.amp, fired);
         }
     }
 }
 
 // The stable sponge mode damps the new values as well.
-__device__ __forceinline__ void stable_damp4(const StepArgs& a, const float D[4], float res[4]) {
-    if (a.stable_sponge) {
+__device__ __forceinline__ void damp4(const float D[4], float res[4]) {
 #pragma unroll
-        for (int k = 0; k < 4; ++k) res[k] *= D[k];
-    }
+    for (int k = 0; k < 4; ++k) res[k] *= D[k];
 }
 
 // Sponge factors of a 4-point group: D(min(dx, dyz)) for each point, formed
