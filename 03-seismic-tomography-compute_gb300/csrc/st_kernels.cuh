@@ -84,8 +84,9 @@ int build_field_maps(FieldMaps* m, const float* base, const Layout& L);
 // x-chunks per CTA column for a tile height and resident CTAs per SM, with at
 // least min_waves waves of resident CTAs when the grid allows it; each chunk
 // re-reads halo extra x-planes.
-// min_len: planes a chunk has at least (the wait test withholds one of them).
-int fd_step_grid_chunks(const Layout& L, int tyv, int minb, int min_waves, int halo = 2, int min_len = 1);
+// min_len: planes a chunk has at least (the wait test withholds one of them); max_len: at most (0: no limit).
+int fd_step_grid_chunks(const Layout& L, int tyv, int minb, int min_waves, int halo = 2, int min_len = 1,
+                        int max_len = 0);
 
 // Maps of the staged imaging variant: the snapshot store (box {64, 16} at
 // (z, y, x, t)) and the compact image / illumination volumes (box {64, 16}).

@@ -1347,7 +1347,7 @@ int launch_step2_rows(const Layout& L, const FieldMaps& mcur, const FieldMaps& m
             configured = true;
         }
     }
-    const int chunks = fd_step_grid_chunks(L, G::TYV, G::MINB, 1, 4, a.withhold ? 4 : 1);
+    const int chunks = fd_step_grid_chunks(L, G::TYV, G::MINB, 1, 4, a.withhold ? 4 : 1, 48);
     a.x_chunk = (int)((L.nx + chunks - 1) / chunks);
     const int nch = (int)((L.nx + a.x_chunk - 1) / a.x_chunk);
     dim3 grid((unsigned)((L.nz + TZ - 1) / TZ), (unsigned)((L.ny + G::TYV - 1) / G::TYV), (unsigned)nch);
@@ -1592,7 +1592,7 @@ int build_field_maps(FieldMaps* m, const float* base, const Layout& L) {
     return ST_OK;
 }
 
-int fd_step_grid_chunks(const Layout& L, int tyv, int minb, int min_waves, int halo, int min_len) {
+int fd_step_grid_chunks(const Layout& L, int tyv, int minb, int min_waves, int halo, int min_len, int max_len) {
     const long long gx = (L.nz + TZ - 1) / TZ, gy = (L.ny + tyv - 1) / tyv;
     const long long tiles = gx * gy;
     // tuning override: SEISMIC_GB300_XCHUNKS=<chunks> (1..nx)
@@ -1615,7 +1615,16 @@ int fd_step_grid_chunks(const Layout& L, int tyv, int minb, int min_waves, int h
     // weighs them.
     if ((double)(tiles * max_chunks) <= slots)
         return (int)std::max<long long>(1, std::min<long long>(L.nx / min_len, (long long)slots / tiles));
-    const long long need = min_waves > 1 ? (long long)std::ceil(min_waves * slots / (double)tiles) : 1;
+    long long need = min_waves > 1 ? (long long)std::ceil(min_waves * slots / (double)tiles) : 1;
+    // Chunks of at most max_len planes: blocks of one long wave fill, march and
+    // drain together, and the slowest sets the time; several shorter waves even
+    // that out at the price of more halo planes. Two-step kernels (forward shot /
+    // RTM us per step): 300^3 3 chunks 66.2 / 179.5, 9 chunks 61.6 / 169.6; 384 x 384 x
+    // 320 5: 101.8 / 291.0, 10: 96.6 / 273.6; 448 x 320 x 384 5: 116.4 / 335.1, 10:
+    // 110.9 / 315.7; 512^3 7: 248 / 733, 13: 240 / 712. At 640 x 160 x 96 (one full
+    // wave of 43 planes, 31.4 / 76.9) shorter ones lose (28 chunks of 23: 34.2 / 81.6),
+    // so the line lies above that.
+    if (max_len > 0) need = std::max<long long>(need, (L.nx + max_len - 1) / max_len);
     const long long first = std::min<long long>(std::max<long long>(1, need), max_chunks);
     for (long long ch = first; ch <= max_chunks; ++ch) {
         const double waves = (double)(tiles * ch) / slots;

@@ -1,5 +1,5 @@
 """Grids that leave multiprocessors idle are marched in the shortest x-chunks one wave of
-blocks allows, down to one plane. A chunk recomputes its halo planes with the arithmetic of
+blocks allows, down to one plane; larger ones in chunks of at most 48 planes. A chunk recomputes its halo planes with the arithmetic of
 their owner, so the fields, the image and the traces are those of a single chunk bit for bit."""
 import os
 
@@ -44,9 +44,10 @@ def run(se, n, nt, fused):
         s.close()
 
 
-# one plane; chunks of one plane (few tiles); a length that the chunks do not divide; many tiles, chunks of three
+# one plane; chunks of one plane (few tiles); a length that the chunks do not divide; many tiles, chunks of
+# three; 52 tiles, where one wave would take longer chunks
 @pytest.mark.parametrize("fused", [1, 2])
-@pytest.mark.parametrize("n", [(1, 20, 24), (13, 33, 72), (31, 130, 64), (37, 100, 128)])
+@pytest.mark.parametrize("n", [(1, 20, 24), (13, 33, 72), (31, 130, 64), (37, 100, 128), (97, 200, 256)])
 def test_shortest_chunks_against_one_chunk(se, monkeypatch, n, fused):
     got = run(se, n, 13, fused)
     monkeypatch.setenv("SEISMIC_GB300_XCHUNKS", "1")
