@@ -270,29 +270,38 @@ __global__ void __launch_bounds__(256, K >= 10 ? 5 : 6) spmv_kernel(const long l
     }
 }
 
-// Short rows (fewer than ten entries on average): a CTA takes 256 consecutive
-// rows at a time, streams their entries as 16-byte loads (whatever row they
-// belong to), multiplies each by its x into shared memory, and then every
-// thread adds up its own row there. Four gathers per load are
-// in flight and no lane idles over a row's end, where a group of lanes per row
-// spends most of its instructions on predicates and waits for the row pointers,
-// the columns and the gathers one after another for 28 bytes of values. A tile
-// with more entries than fit in shared memory is summed a warp per row.
-// 7 entries per row on a 256^3 grid, 72 bytes per row: 600 us a product with
-// four lanes per row, 242 us so (a copy of the bytes takes 178).
-constexpr int SR_ROWS = 256;
-constexpr int SR_CAP = 2816;  // entries of a tile (11 per row): 11 KB, eight CTAs per SM
-__global__ void __launch_bounds__(SR_ROWS, 8) spmv_rows_kernel(const long long* __restrict__ rp, const int* __restrict__ col,
+__device__ __forceinline__ void copy16_async(void* dst, const void* src, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
+}
+
+// Short rows (fewer than ten entries on average): a CTA takes 128 consecutive
+// rows at a time, copies their columns and values to shared memory as a stream of
+// 16-byte pieces (whatever row they belong to), and every thread then works
+// through its own row there. Neighbouring rows gather neighbouring x, so a warp's
+// gather is a line or two; multiplied along the stream a gather met all the offsets
+// of a row, seven lines, and the L1 set the pace. A group of lanes per row spends
+// most of its instructions on predicates and waits for the row pointers, the
+// columns and the gathers one after another for 28 bytes of values. A tile with
+// more entries than fit in shared memory is summed a warp per row.
+// 7 entries per row on a 256^3 grid, 72 bytes per row: 199 us a product (a copy of
+// the bytes takes 178); products along the stream 244, four lanes per row 600. 40
+// CG iterations there with tiles of 256 / 128 / 64 rows 24.3 / 23.5 / 23.3 ms
+// (smaller tiles overflow more easily), a tile per warp 25.9 (spills), two tiles in
+// turn at fewer warps per SM 28.0.
+constexpr int SR_ROWS = 128;
+constexpr int SR_CAP = 1408;  // entries of a tile (11 per row): 11 KB, sixteen CTAs per SM
+__global__ void __launch_bounds__(SR_ROWS, 16) spmv_rows_kernel(const long long* __restrict__ rp, const int* __restrict__ col,
                                                               const float* __restrict__ val,
                                                               const float* __restrict__ x, float* __restrict__ y,
-                                                              long long rows, long long nnz,
+                                                              long long rows,
                                                               const float* __restrict__ add, float add_scale,
                                                               const float* __restrict__ pdot,
                                                               double* __restrict__ dot_acc,
                                                               const int* __restrict__ done) {
     if (done && *done) return;
-    __shared__ __align__(16) float prod[SR_CAP + 8];
-    __shared__ double red[8];
+    __shared__ __align__(16) int scol[SR_CAP + 8];
+    __shared__ __align__(16) float sval[SR_CAP + 8];
+    __shared__ double red[SR_ROWS / 32];
     const int tid = threadIdx.x;
     double local = 0.0;
     for (long long r0 = (long long)blockIdx.x * SR_ROWS; r0 < rows; r0 += (long long)gridDim.x * SR_ROWS) {
@@ -304,35 +313,33 @@ __global__ void __launch_bounds__(SR_ROWS, 8) spmv_rows_kernel(const long long* 
         const long long a = active ? rp[row] : 0, b = active ? rp[row + 1] : 0;
         float sum = 0.0f;
         if (e1 - base <= SR_CAP) {
-            for (long long e = base + 4 * tid; e < e1; e += 4 * SR_ROWS) {
-                float4 o = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                if (e >= e0 && e + 4 <= e1) {
-                    const int4 c = __ldg(reinterpret_cast<const int4*>(col + e));
-                    const float4 v = __ldg(reinterpret_cast<const float4*>(val + e));
-                    o = make_float4(v.x * __ldg(x + c.x), v.y * __ldg(x + c.y), v.z * __ldg(x + c.z),
-                                    v.w * __ldg(x + c.w));
-                } else {
-                    float* of = &o.x;
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        if (e + k >= e0 && e + k < e1) of[k] = __ldg(val + e + k) * __ldg(x + __ldg(col + e + k));
-                }
-                *reinterpret_cast<float4*>(prod + (e - base)) = o;
+            const int m = (int)(e1 - base);
+            for (int k = 4 * tid; k < m; k += 4 * SR_ROWS) {
+                const int bytes = min(16, 4 * (m - k));
+                copy16_async(scol + k, col + base + k, bytes);
+                copy16_async(sval + k, val + base + k, bytes);
             }
+            asm volatile("cp.async.wait_all;" ::: "memory");
             __syncthreads();
             // four strided partial sums, as four lanes per row would hold
             float t0 = 0.0f, t1 = 0.0f, t2 = 0.0f, t3 = 0.0f;
             const int kb = (int)(b - base);
             int k = (int)(a - base);
             for (; k + 4 <= kb; k += 4) {
-                t0 += prod[k];
-                t1 += prod[k + 1];
-                t2 += prod[k + 2];
-                t3 += prod[k + 3];
+                const float x0 = __ldg(x + scol[k]), x1 = __ldg(x + scol[k + 1]), x2 = __ldg(x + scol[k + 2]),
+                            x3 = __ldg(x + scol[k + 3]);
+                t0 += __fmul_rn(sval[k], x0);
+                t1 += __fmul_rn(sval[k + 1], x1);
+                t2 += __fmul_rn(sval[k + 2], x2);
+                t3 += __fmul_rn(sval[k + 3], x3);
             }
-            if (k < kb) t0 += prod[k];
-            if (k + 1 < kb) t1 += prod[k + 1];
-            if (k + 2 < kb) t2 += prod[k + 2];
+            float x0 = 0.0f, x1 = 0.0f, x2 = 0.0f;
+            if (k < kb) x0 = __ldg(x + scol[k]);
+            if (k + 1 < kb) x1 = __ldg(x + scol[k + 1]);
+            if (k + 2 < kb) x2 = __ldg(x + scol[k + 2]);
+            if (k < kb) t0 += __fmul_rn(sval[k], x0);
+            if (k + 1 < kb) t1 += __fmul_rn(sval[k + 1], x1);
+            if (k + 2 < kb) t2 += __fmul_rn(sval[k + 2], x2);
             sum = (t0 + t2) + (t1 + t3);
             __syncthreads();
         } else {
@@ -367,9 +374,9 @@ __global__ void __launch_bounds__(SR_ROWS, 8) spmv_rows_kernel(const long long* 
 int launch_spmv_rows(const DevCsr& A, const float* x, float* y, const float* add, float add_scale, const float* pdot,
                      double* dot_acc, const int* done, cudaStream_t st) {
     const long long tiles = (A.rows + SR_ROWS - 1) / SR_ROWS;
-    const unsigned blocks = (unsigned)std::max<long long>(1, std::min<long long>(tiles, grid_cap() / 2));  // 8 per SM
-    spmv_rows_kernel<<<blocks, SR_ROWS, 0, st>>>(A.row_ptr, A.col, A.val, x, y, A.rows, A.nnz, add, add_scale, pdot,
-                                                 dot_acc, done);
+    const unsigned blocks = (unsigned)std::max<long long>(1, std::min<long long>(tiles, grid_cap()));  // 16 per SM
+    spmv_rows_kernel<<<blocks, SR_ROWS, 0, st>>>(A.row_ptr, A.col, A.val, x, y, A.rows, add, add_scale, pdot, dot_acc,
+                                                 done);
     count_launch();
     ST_CUDA(cudaGetLastError());
     return ST_OK;
@@ -672,18 +679,19 @@ __global__ void normal_jacobi_kernel(const long long* __restrict__ rp, const flo
     }
 }
 
-__global__ void __launch_bounds__(SR_ROWS) normal_jacobi_rows_kernel(const long long* __restrict__ rp,
+constexpr int NJ_ROWS = 256;
+__global__ void __launch_bounds__(NJ_ROWS) normal_jacobi_rows_kernel(const long long* __restrict__ rp,
                                                                      const float* __restrict__ val, long long rows,
                                                                      double lam, float* __restrict__ dinv) {
-    constexpr int CAP = 24 * SR_ROWS;
+    constexpr int CAP = 24 * NJ_ROWS;
     __shared__ float v[CAP];
-    for (long long r0 = (long long)blockIdx.x * SR_ROWS; r0 < rows; r0 += (long long)gridDim.x * SR_ROWS) {
+    for (long long r0 = (long long)blockIdx.x * NJ_ROWS; r0 < rows; r0 += (long long)gridDim.x * NJ_ROWS) {
         const long long i = r0 + threadIdx.x;
-        const long long e0 = rp[r0], e1 = rp[min(r0 + SR_ROWS, rows)];
+        const long long e0 = rp[r0], e1 = rp[min(r0 + NJ_ROWS, rows)];
         const long long a = i < rows ? rp[i] : 0, b = i < rows ? rp[i + 1] : 0;
         const bool staged = e1 - e0 <= CAP;
         if (staged)
-            for (long long e = e0 + threadIdx.x; e < e1; e += SR_ROWS) v[e - e0] = __ldg(val + e);
+            for (long long e = e0 + threadIdx.x; e < e1; e += NJ_ROWS) v[e - e0] = __ldg(val + e);
         __syncthreads();
         PairSum s;
         bool safe = staged;
@@ -927,7 +935,7 @@ int launch_normal_jacobi(const DevCsr& AT, double lam, float* dinv, cudaStream_t
     if (AT.nnz >= 24 * AT.rows)
         normal_jacobi_kernel<<<blocks_for(AT.rows * 32) / 2 + 1, 256, 0, st>>>(AT.row_ptr, AT.val, AT.rows, lam, dinv);
     else
-        normal_jacobi_rows_kernel<<<blocks_for(AT.rows), SR_ROWS, 0, st>>>(AT.row_ptr, AT.val, AT.rows, lam, dinv);
+        normal_jacobi_rows_kernel<<<blocks_for(AT.rows), NJ_ROWS, 0, st>>>(AT.row_ptr, AT.val, AT.rows, lam, dinv);
     count_launch();
     ST_CUDA(cudaGetLastError());
     return ST_OK;

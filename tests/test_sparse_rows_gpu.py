@@ -1,5 +1,5 @@
 """Short-row SpMV, the normal-equation diagonal and the CG vector kernels at
-their edges: tiles of 256 rows, tiles with more entries than fit in shared
+their edges: tiles of 128 rows, tiles with more entries than fit in shared
 memory, empty rows, a start that is not 16-byte aligned, an unaligned solution
 vector. Reference: FP64 numpy; bounds from FP32 rounding (a row of m entries:
 (m + 1) 2^-24 sum |a x|; the squares' sums and their inverse: 2^-23)."""
@@ -36,7 +36,7 @@ def _lengths(kind, rows, rng):
 
 
 @pytest.mark.parametrize("kind", ["seven", "mixed", "long"])
-@pytest.mark.parametrize("rows", [1, 255, 256, 257, 5003])
+@pytest.mark.parametrize("rows", [1, 127, 128, 129, 255, 256, 257, 5003])
 def test_short_rows(kind, rows):
     rng = np.random.default_rng(rows)
     lengths = _lengths(kind, rows, rng)
