@@ -46,6 +46,8 @@ struct ResArgs {
     const float* c;         // device layout
     float* cur;             // u_nt, u_{nt-1}: interior written at the end
     float* prev;
+    float* next;            // u_{next_step}, as launches of two steps leave the third field
+    int next_step;
     const float* wav;       // nt + 1 values, NaN: no injection
     unsigned char* xch;     // head | per block and parity: xlo | xhi | ylo | yhi
     float* seis;
@@ -499,6 +501,11 @@ __global__ void __launch_bounds__(RES_THREADS, 1) resident_shot_kernel(const __g
         }
         if (warp_rec && !warp_src) sample();
         seis_t += r.nrec;
+        if (t + 1 == r.next_step && act) {
+#pragma unroll
+            for (int k = 0; k < K; ++k)
+                if (k < xcnt) st4(r.next + at0 + k * a.plane, u[k]);
+        }
         if (t + 1 < r.nt) receive(t + 1, tag, Sn);
         return __syncthreads_or(!ok) != 0;
     };
@@ -629,6 +636,8 @@ int resident_shot(st_solver* s, const StepArgs& a, const st_shot* shot, float* s
     r.c = s->c;
     r.cur = s->f[s->ic];
     r.prev = s->f[s->ip];
+    r.next = s->f[s->in];
+    r.next_step = nt % 2 ? nt - 2 : nt - 3;
     r.wav = reinterpret_cast<const float*>(xch + wav_at);
     r.xch = xch;
     r.seis = seis;

@@ -97,6 +97,22 @@ def test_resident_shot_clamps_alike(se):
         s.close()
 
 
+@pytest.mark.parametrize("nt", [8, 21])
+def test_resident_shot_leaves_the_third_field_alike(se, monkeypatch, nt):
+    n = (24, 30, 44)
+    rec = se.workloads.ReceiverGrid(0, 1, 24, 0, 1, 30, 20)
+    s = solver(se, n, nt, "reference")
+    try:
+        wav = se.workloads.ricker(30.0, se.workloads.cfl_dt(10.0, 3000.0), nt) + 1e-3
+        got = shot(se, s, n, nt, (12, 9, 20), wav, rec) + (s.get_field(2),)
+        monkeypatch.setenv("SEISMIC_GB300_XCHUNKS", "3")  # launches of two steps
+        want = shot(se, s, n, nt, (12, 9, 20), wav, rec) + (s.get_field(2),)
+        compare(want, got)
+        assert np.abs(want[4]).max() > 0 and np.array_equal(want[4], got[4])
+    finally:
+        s.close()
+
+
 def test_resident_shots_from_two_streams(se):
     import threading
     n, nt = (48, 40, 56), 100
