@@ -194,7 +194,9 @@ int st_solver_device_field(st_solver* s, int which, float** out);
 /* Time steps per launch of the shot-level passes (st_shot_forward, st_rtm_shot
  * and its host variant, the forward and adjoint passes of the FWI gradient
  * and of the checkpointed entry points): 2 (default) runs two
- * steps in one launch (with the imaging or gradient terms of both fused), 1
+ * steps in one launch (with the imaging or gradient terms of both fused; a
+ * forward shot without snapshots of at least eight steps on a grid that fits
+ * on the GPU's SMs, up to about 2.4 million points, is one launch), 1
  * one step per launch; seismograms, snapshots, images, gradients and fields
  * are bit-identical either way. The time loops of WaveEquationSolver::
  * forward_propagate (solver/wave_equation.cpp:100-152) and
