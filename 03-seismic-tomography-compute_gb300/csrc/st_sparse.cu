@@ -179,6 +179,42 @@ struct PairSum {
     __device__ __forceinline__ double value() const { return (double)h + (double)l; }
 };
 
+// A sum of products held as an unevaluated triple of FP32 values (the three-fold
+// sum of Ogita, Rump and Oishi, "Accurate sum and dot product", 2005): the products
+// are split exactly by FMA, the rounding errors of the leading sum and of the sum
+// of those errors are kept, and only the third part is rounded. n products lose at
+// most about (n 2^-24)^3 of the sum of their magnitudes, a chain of FP64 additions
+// n 2^-53, so up to TRIPLE_MAX products (2^-48) the triple is no less precise than
+// FP64. The FP64 pipe takes a warp's operation in 16 cycles here (conversions
+// too), the FP32 one in a quarter of a cycle. Only for factors that triple_safe
+// admits: zero or 2^-50 .. 2^50, so that no error term underflows and 2^27
+// products stay below 2^128; the callers take FP64 sums otherwise (tiny values,
+// infinities, NaN).
+constexpr int TRIPLE_MAX = 256;
+__device__ __forceinline__ bool triple_safe(float a) {
+    const unsigned m = __float_as_uint(a) & 0x7fffffffu;
+    return (m - 0x26800000u <= 0x58800000u - 0x26800000u) | (m == 0u);
+}
+// a + b = s + returned error, exactly.
+__device__ __forceinline__ float two_sum(float a, float b, float& s) {
+    s = __fadd_rn(a, b);
+    const float z = __fsub_rn(s, a);
+    return __fadd_rn(__fsub_rn(a, __fsub_rn(s, z)), __fsub_rn(b, z));
+}
+struct TripleSum {
+    float h = 0.0f, m = 0.0f, l = 0.0f;
+    __device__ __forceinline__ void add(float a, float b) {
+        const float p = __fmul_rn(a, b);
+        const float e = two_sum(h, p, h), f = two_sum(m, __fmaf_rn(a, b, -p), m), g = two_sum(m, e, m);
+        l = __fadd_rn(l, __fadd_rn(f, g));
+    }
+    __device__ __forceinline__ void merge(const TripleSum& t) {
+        const float e = two_sum(h, t.h, h), f = two_sum(m, t.m, m), g = two_sum(m, e, m);
+        l = __fadd_rn(__fadd_rn(l, t.l), __fadd_rn(f, g));
+    }
+    __device__ __forceinline__ double value() const { return (double)h + ((double)m + (double)l); }
+};
+
 // ---------------------------------------------------------------- SpMV
 // y[row] = sum val*x[col] with G threads per row (FP32 accumulation, a
 // G-way strided partial sum per row reduced by shuffles), optional
@@ -626,45 +662,47 @@ __global__ void jacobi_kernel(const long long* __restrict__ rp, const int* __res
 // per row, its lanes over the entries (coalesced). The rows of a warp lie a grid
 // apart (neighbouring cells are heavy together: where rays meet, a row holds
 // thousands of entries), and each group of 32 keeps row w's sum on lane w, so
-// that the FP64 division runs on full warps; pairs of FP32 values carry the
-// squares until then. 1M rows of 361 entries: 0.48 ms (2.15 with FP64 sums and a
-// warp per row, 4.19 with a thread per row). Short rows (less than 24 entries) are staged through
-// shared memory instead, a thread per row.
+// that the FP64 division runs on full warps; triples of FP32 values carry the
+// squares until then, and rows they cannot hold are summed in FP64. 1M rows of 202
+// entries: 0.58 ms, bound by the FP32 instructions of the triples (1.21 with FP64
+// sums and a thread per row; pairs took 0.41 and lost what lies beyond 2^-48, and
+// the whole sum beyond 2^128). Short rows (less than 24 entries) are staged through
+// shared memory instead, a thread per row: 7.1M rows of 7 entries 0.18 ms (0.28
+// with FP64 sums).
 __global__ void normal_jacobi_kernel(const long long* __restrict__ rp, const float* __restrict__ val, long long rows,
                                      double lam, float* __restrict__ dinv) {
     const int lane = threadIdx.x & 31;
     const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
     const long long first = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
     for (long long r0 = first; r0 < rows; r0 += 32 * warps) {
-        float mh = 0.0f, ml = 0.0f;
-        double wide = -1.0;  // the sum where the pairs cannot hold it
+        TripleSum mine;
+        double wide = -1.0;  // the sum where the triples cannot hold it
         for (int w = 0; w < 32; ++w) {
             const long long r = r0 + w * warps;
             if (r >= rows) break;
             const long long ra = rp[r], rb = rp[r + 1];
-            PairSum s;
-            unsigned odd = 0;
-            for (long long q = ra + lane; q - lane < rb; q += 8 * 32) {
+            TripleSum s;
+            unsigned odd = rb - ra > 32 * TRIPLE_MAX ? 1u : 0u;
+            for (long long q = ra + lane; !odd && q - lane < rb; q += 8 * 32) {
                 float v[8];
 #pragma unroll
                 for (int k = 0; k < 8; ++k) v[k] = q + 32 * k < rb ? __ldg(val + q + 32 * k) : 0.0f;
 #pragma unroll
                 for (int k = 0; k < 8; ++k) {
-                    odd |= pair_safe(v[k]) ? 0u : 1u;
+                    odd |= triple_safe(v[k]) ? 0u : 1u;
                     s.add(v[k], v[k]);
                 }
             }
             if (!__any_sync(FULL, odd)) {
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) {
-                    const float h = __shfl_xor_sync(FULL, s.h, o), l = __shfl_xor_sync(FULL, s.l, o);
-                    s.add(h, 1.0f);
-                    s.l += l;
+                    TripleSum t;
+                    t.h = __shfl_xor_sync(FULL, s.h, o);
+                    t.m = __shfl_xor_sync(FULL, s.m, o);
+                    t.l = __shfl_xor_sync(FULL, s.l, o);
+                    s.merge(t);
                 }
-                if (lane == w) {
-                    mh = s.h;
-                    ml = s.l;
-                }
+                if (lane == w) mine = s;
             } else {
                 double t = 0.0;
                 for (long long e = ra + lane; e < rb; e += 32) t += (double)val[e] * (double)val[e];
@@ -673,9 +711,9 @@ __global__ void normal_jacobi_kernel(const long long* __restrict__ rp, const flo
                 if (lane == w) wide = t;
             }
         }
-        const double mine = wide >= 0.0 || wide != wide ? wide : (double)mh + (double)ml;
+        const double sum = wide >= 0.0 || wide != wide ? wide : mine.value();
         const long long i = r0 + lane * warps;
-        if (i < rows) dinv[i] = (float)(1.0 / (mine + lam));
+        if (i < rows) dinv[i] = (float)(1.0 / (sum + lam));
     }
 }
 
@@ -693,11 +731,11 @@ __global__ void __launch_bounds__(NJ_ROWS) normal_jacobi_rows_kernel(const long 
         if (staged)
             for (long long e = e0 + threadIdx.x; e < e1; e += NJ_ROWS) v[e - e0] = __ldg(val + e);
         __syncthreads();
-        PairSum s;
-        bool safe = staged;
-        if (staged)
+        TripleSum s;
+        bool safe = staged && b - a <= TRIPLE_MAX;
+        if (safe)
             for (int k = (int)(a - e0); k < (int)(b - e0); ++k) {
-                safe = safe & pair_safe(v[k]);
+                safe = safe & triple_safe(v[k]);
                 s.add(v[k], v[k]);
             }
         double t = s.value();

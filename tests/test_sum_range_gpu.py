@@ -1,0 +1,47 @@
+"""Sums of products at the edges of the FP32 triples that carry them: the
+normal-equation diagonal (both kernels) where the squares' sum leaves the FP32
+range and where it needs all of FP64's bits. Every expected value is exact."""
+import numpy as np
+import pytest
+import torch
+
+import seismic_engine as se
+from seismic_engine._lib import call
+
+pytestmark = pytest.mark.gpu
+
+
+def _matrix(columns, rows, fill):
+    """columns: the entries of the first columns; 100 more columns of `fill` ones (their mean picks the kernel)."""
+    r, c, v = [], [], []
+    for j, entries in enumerate(columns + [np.ones(fill)] * 100):
+        r.append(np.arange(len(entries)))
+        c.append(np.full(len(entries), j))
+        v.append(np.asarray(entries, np.float64))
+    cols = len(columns) + 100
+    return se.CSRMatrix().build_from_triplets(rows, cols, np.concatenate(r), np.concatenate(c), np.concatenate(v)), cols
+
+
+def _diagonal(A, cols, lam):
+    d = torch.zeros(cols, device="cuda")
+    torch.cuda.synchronize()
+    call("st_csr_normal_jacobi", A.handle, lam, d.data_ptr())
+    torch.cuda.synchronize()
+    return d.cpu().numpy()
+
+
+@pytest.mark.parametrize("fill", [2, 60])
+@pytest.mark.parametrize("power", [46, 50, 51, 58, 60, 61])
+def test_diagonal_of_large_entries(power, fill):
+    """Sums of 2^8 .. 2^14 squares up to 2^128 and beyond: the inverse, subnormal at the top, is a power of two."""
+    counts = (255, 256, 257, 300, 4096, 9000)
+    A, cols = _matrix([np.full(m, 2.0 ** power) for m in counts], 9000, fill)
+    want = np.float32(1.0 / (np.array(counts, np.float64) * 4.0 ** power))
+    assert np.array_equal(_diagonal(A, cols, 0.0)[:len(counts)], want)
+
+
+@pytest.mark.parametrize("fill", [2, 60])
+def test_diagonal_keeps_every_bit_of_fp64(fill):
+    # squares 2^24 + 1 + 4 * 2^-28, 53 bits in any order of summation; lam leaves the last
+    A, cols = _matrix([[2.0 ** 12, 1.0] + [2.0 ** -14] * 4], 100, fill)
+    assert _diagonal(A, cols, -(2.0 ** 24 + 1.0))[0] == 2.0 ** 26
