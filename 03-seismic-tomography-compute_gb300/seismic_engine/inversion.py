@@ -33,6 +33,15 @@ from .rays import SampledRays
 logger = logging.getLogger(__name__)
 
 
+def _stock(obj, cls, *names) -> bool:
+    """Whether obj's methods of these names are cls's own, bound to obj."""
+    for name in names:
+        m = getattr(obj, name, None)
+        if getattr(m, "__func__", None) is not getattr(cls, name) or m.__self__ is not obj:
+            return False
+    return True
+
+
 class FaultRecoveryPolicy:
     """inversion.py:22-81, unchanged semantics."""
 
@@ -197,15 +206,23 @@ class AdjointStateInversion:
             logger.warning(f"CFL condition may be violated: CFL={cfl:.4f} > 0.5.")
         return vp
 
+    def _fused_trials(self) -> bool:
+        """Whether nothing that forms a trial's misfit has been replaced, on a
+        class or on an instance, and its clamps are ranges in order."""
+        rng = self.fault_policy.velocity_clamp_range if self.enable_fault_tolerance else (0.0, 0.0)
+        return (_stock(self, AdjointStateInversion, "_forward", "_misfit", "_l1") and
+                _stock(self.rays, SampledRays, "forward_model", "misfit", "trial_misfit") and
+                _stock(self.fault_policy, FaultRecoveryPolicy, "clamp_velocity") and
+                self.model.vp_min <= self.model.vp_max and rng[0] <= rng[1])
+
     def _line_search(self, vp, gradient, current_misfit: float) -> float:
         """inversion.py:436-453. A trial is the table of its model, its
-        traveltimes and their misfit in four launches and one read; a subclass
-        or policy with its own clamp, forward model or misfit takes them."""
+        traveltimes and their misfit in four launches and one read; a driver,
+        ray object or policy with its own clamp, forward model or misfit takes
+        them."""
         step = self.step_length
         lo, hi = self.model.vp_min, self.model.vp_max  # update_from_flat's clamp, model left unchanged
-        cls, ref = type(self), AdjointStateInversion
-        fused = (cls._forward is ref._forward and cls._misfit is ref._misfit and
-                 type(self.fault_policy).clamp_velocity is FaultRecoveryPolicy.clamp_velocity)
+        fused = self._fused_trials()
         for _ in range(self.line_search_max):
             if fused:
                 trial_misfit = self.rays.trial_misfit(
