@@ -157,7 +157,21 @@ class AdjointStateInversion:
 
     def _misfit(self, times) -> float:
         """OBSDataCoordinator.compute_misfit (obs_data.py:116-129)."""
-        return self.rays.misfit(times, self.observed, self.weights, self._l1())
+        l1 = self._l1()
+        if self._per_pick(times):
+            return self.rays.misfit(times, self.observed, self.weights, l1)
+        r = self.observed - times
+        return float((self.weights * r.abs()).sum()) if l1 else float(0.5 * (self.weights * (r * r)).sum())
+
+    def _per_pick(self, times) -> bool:
+        """Whether times, the observations and the weights are device arrays of
+        one FP64 value per pick, as SampledRays.misfit takes them: weights that
+        broadcast, say, or another kind of ray object take the formula."""
+        import torch
+        return isinstance(self.rays, SampledRays) and all(
+            SampledRays._is_tensor(a) and a.dtype == torch.float64 and tuple(a.shape) == (self.rays.n_picks,) and
+            a.is_contiguous() and a.is_cuda and a.device.index == self.rays.device
+            for a in (times, self.observed, self.weights))
 
     def _l1(self) -> bool:
         if self.misfit_type not in ("l2", "cross_correlation", "l1"):
@@ -212,6 +226,7 @@ class AdjointStateInversion:
         rng = self.fault_policy.velocity_clamp_range if self.enable_fault_tolerance else (0.0, 0.0)
         return (_stock(self, AdjointStateInversion, "_forward", "_misfit", "_l1") and
                 _stock(self.rays, SampledRays, "forward_model", "misfit", "trial_misfit") and
+                self._per_pick(self.observed) and
                 _stock(self.fault_policy, FaultRecoveryPolicy, "clamp_velocity") and
                 self.model.vp_min <= self.model.vp_max and rng[0] <= rng[1])
 

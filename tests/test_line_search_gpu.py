@@ -1,6 +1,7 @@
-"""The inversion driver's line search with parts of the driver replaced: every override (a ray
-object's forward model, a method set on the instance, the policy's clamp) is used for the
-trials too."""
+"""The inversion driver's line search and misfit with parts of the driver replaced: every
+override (a ray object's forward model, a method set on the instance, the policy's clamp) is
+used for the trials too, and what the misfit formula takes -- weights that broadcast, a ray
+object with the two methods of the reference alone -- is taken."""
 import os
 
 import numpy as np
@@ -60,6 +61,21 @@ class _Bent(se.rays.SampledRays):
         return super().forward_model(vp, out) * 1.02
 
 
+class _TwoMethods:
+    """The reference's two methods and nothing else."""
+
+    def __init__(self, rays):
+        self._rays = rays
+        self.calls = 0
+
+    def forward_model(self, vp):
+        self.calls += 1
+        return self._rays.forward_model(vp)
+
+    def compute_gradient(self, vp, residuals):
+        return self._rays.compute_gradient(vp, residuals)
+
+
 class _Unfused(AdjointStateInversion):
     def _forward(self, vp):
         return self.rays.forward_model(vp)
@@ -100,6 +116,21 @@ def test_trials_of_a_foreign_method(golden):
     driver._forward = other._forward  # the same function, bound to another driver
     _search(driver)
     assert other.rays.calls == 3
+
+
+@pytest.mark.parametrize("misfit", ["l2", "l1"])
+def test_weights_that_broadcast(golden, misfit):
+    n = golden.z["travel_time"].size
+    want = _driver(golden, weights=np.full(n, 0.5), misfit_type=misfit).run()
+    got = _driver(golden, weights=0.5, misfit_type=misfit).run()
+    np.testing.assert_allclose(got["misfit_history"], want["misfit_history"], rtol=1e-12)
+
+
+def test_rays_with_the_two_methods_alone(golden):
+    rays = _TwoMethods(golden.rays())
+    want, got = _driver(golden).run(), _driver(golden, rays=rays).run()
+    np.testing.assert_allclose(got["misfit_history"], want["misfit_history"], rtol=1e-12)
+    assert rays.calls > len(got["misfit_history"])
 
 
 def test_ranges_out_of_order_end_at_the_upper_bound(golden):
