@@ -15,6 +15,11 @@
 // moves a third of the bytes in long runs. Measured: 45M entries, 125,000 columns
 // (two passes of 523 us) 1.3 ms against 5.1 ms of kernels; the first tomography
 // solve on a new 361M-entry matrix, transpose included, 74.4 -> 35.5 ms.
+//
+// The columns lie in arrays that callers may write (st_csr_device_arrays). The last
+// pass looks for columns outside the matrix and for entries that repeat one; a
+// matrix with either is transposed by the triplet sort, which drops the former and
+// sums the latter.
 #include "st_sort.cuh"
 #include "st_sparse.cuh"
 
@@ -172,10 +177,16 @@ __global__ void tr_rows_kernel(const long long* __restrict__ rp, long long rows,
 }
 
 // Row pointers from the sorted keys: entry u is the first of every row in (key[u-1], key[u]].
-__global__ void tr_rowptr_kernel(const int* __restrict__ key, long long n, long long rows, long long* __restrict__ rp) {
+// *irregular: a key outside the rows (such keys are passed over) or a repeated entry.
+__global__ void tr_rowptr_kernel(const int* __restrict__ key, const int* __restrict__ col, long long n, long long rows,
+                                 long long* __restrict__ rp, int* __restrict__ irregular) {
     for (long long u = blockIdx.x * (long long)blockDim.x + threadIdx.x; u < n; u += (long long)gridDim.x * blockDim.x) {
         const long long r = key[u];
         const long long prev = u == 0 ? -1 : key[u - 1];
+        if (r < 0 || r >= rows || prev < -1 || prev >= rows || (u > 0 && (prev == -1 || (prev == r && col[u - 1] == col[u])))) {
+            *irregular = 1;
+            continue;
+        }
         for (long long q = prev + 1; q <= r; ++q) rp[q] = u;
         if (u == n - 1)
             for (long long q = r + 1; q <= rows; ++q) rp[q] = n;
@@ -201,6 +212,14 @@ int build_transpose(const DevCsr& A, DevCsr* T, cudaStream_t st) {
     out.rows = A.cols;
     out.cols = A.rows;
     out.nnz = n;
+    int irregular = 0;
+    auto expand = [&](int* rowidx) -> int {
+        if (n >= 12 * A.rows) tr_rows_kernel<32><<<tr_blocks(A.rows * 32), 256, 0, st>>>(A.row_ptr, A.rows, rowidx);
+        else tr_rows_kernel<4><<<tr_blocks(A.rows * 4), 256, 0, st>>>(A.row_ptr, A.rows, rowidx);
+        count_launch();
+        ST_CUDA(cudaGetLastError());
+        return ST_OK;
+    };
     auto build = [&]() -> int {
         ST_CUDA(cudaMalloc(&out.row_ptr, (size_t)(A.cols + 1) * sizeof(long long)));
         if (n == 0) {
@@ -224,10 +243,12 @@ int build_transpose(const DevCsr& A, DevCsr* T, cudaStream_t st) {
         const long long hn = (long long)bins * grid;
         DeviceBuffers bufs;
         auto* rowidx = static_cast<int*>(bufs.get((size_t)n * 4));  // the rows, then the last pass's keys
-        auto* hist = static_cast<long long*>(bufs.get((size_t)hn * 8));
+        auto* hist = static_cast<long long*>(bufs.get((size_t)hn * 8 + sizeof(int)));  // the irregular word behind it
         auto* offs = static_cast<long long*>(bufs.get((size_t)hn * 8));
         void* stmp = bufs.get(scan_tmp_bytes(hn));
         if (!rowidx || !hist || !offs || !stmp) return bufs.fail();
+        int* flag = reinterpret_cast<int*>(hist + hn);
+        ST_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), st));
         int* bk[2] = {nullptr, nullptr};
         int* br[2] = {nullptr, nullptr};
         float* bv[2] = {nullptr, nullptr};
@@ -237,10 +258,7 @@ int build_transpose(const DevCsr& A, DevCsr* T, cudaStream_t st) {
             bv[p] = static_cast<float*>(bufs.get((size_t)n * 4));
             if (!bk[p] || !br[p] || !bv[p]) return bufs.fail();
         }
-        if (n >= 12 * A.rows) tr_rows_kernel<32><<<tr_blocks(A.rows * 32), 256, 0, st>>>(A.row_ptr, A.rows, rowidx);
-        else tr_rows_kernel<4><<<tr_blocks(A.rows * 4), 256, 0, st>>>(A.row_ptr, A.rows, rowidx);
-        count_launch();
-        ST_CUDA(cudaGetLastError());
+        ST_TRY(expand(rowidx));
         ST_CUDA(cudaFuncSetAttribute(tr_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)sizeof(TrSmem)));
         const int* ik = A.col;
@@ -266,13 +284,27 @@ int build_transpose(const DevCsr& A, DevCsr* T, cudaStream_t st) {
             ir = orw;
             iv = ov;
         }
-        tr_rowptr_kernel<<<tr_blocks(n), 256, 0, st>>>(keys, n, A.cols, out.row_ptr);
+        tr_rowptr_kernel<<<tr_blocks(n), 256, 0, st>>>(keys, out.col, n, A.cols, out.row_ptr, flag);
         count_launch();
         ST_CUDA(cudaGetLastError());
+        ST_CUDA(cudaMemcpyAsync(&irregular, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
         ST_CUDA(cudaStreamSynchronize(st));
         return ST_OK;
     };
-    const int rc = build();
+    auto build_sorted = [&]() -> int {
+        DeviceBuffers bufs;
+        auto* rowidx = static_cast<int*>(bufs.get((size_t)n * 4));
+        if (!rowidx) return bufs.fail();
+        ST_TRY(expand(rowidx));
+        ST_TRY((build_csr<int, float>(A.cols, A.rows, n, A.col, rowidx, A.val, false, &out, st)));
+        ST_CUDA(cudaStreamSynchronize(st));
+        return ST_OK;
+    };
+    int rc = build();
+    if (rc == ST_OK && irregular) {
+        out.release();
+        rc = build_sorted();
+    }
     if (rc < 0) {
         cudaStreamSynchronize(st);
         out.release();

@@ -691,7 +691,9 @@ int st_csr_build_sampled_ray_matrix(st_csr* m, st_ray_picks* p, int64_t* nnz);
 int st_csr_shape(st_csr* m, int64_t out[3]);
 /* row_ptr(), col_ind(), values() (csr_matrix.h:36-38) copied to the host (any may be NULL). */
 int st_csr_get(st_csr* m, int64_t* row_ptr, int64_t* col_ind, double* values);
-/* Device arrays of the matrix (borrowed; valid until the next build). */
+/* Device arrays of the matrix (borrowed; valid until the next build). Columns may
+ * be rewritten: a transpose made afterwards drops entries outside the columns and
+ * sums repeated ones; the products with the matrix itself need them in range. */
 int st_csr_device_arrays(st_csr* m, long long** row_ptr, int** col_ind, float** values);
 int st_csr_stream(st_csr* m, void** out);
 /* Replace spmv / spmv_transpose (csr_matrix.cpp:118-166; the transpose with
