@@ -28,7 +28,8 @@
 // are compared as integers, and the correctly rounded quotient is formed with
 // the axis's reciprocal. Rays that this form cannot take (end points that are
 // not finite, extreme ranges) walk with plain FP64 operations; a ray that
-// outruns its bound sends the call to the triplet builder. 500k rays on 50^3 cells
+// outruns its bound, or scratch that cannot be had, sends the call to the triplet
+// builder. 500k rays on 50^3 cells
 // (45M entries): build, transpose and two products 6.3 ms, 16.8 with two plain
 // walks and the sort of the triplets.
 #include "st_fp64.cuh"
@@ -349,7 +350,9 @@ unsigned grid_for(long long n) {
 }  // namespace
 
 // The walk-once builder; *done = false (and nothing built) where a ray outran its
-// bound or the rows do not fit in shared memory.
+// bound, the rows do not fit in shared memory, or an allocation fails: a tile's
+// scratch is 32 times its longest ray's bound, so rays of mixed lengths can ask for
+// many times what the triplets of their entries take.
 static int build_walk_once(long long nrays, const double* d_ends, const RayGrid& G, DevCsr* out, bool* done,
                            cudaStream_t st) {
     *done = false;
@@ -361,7 +364,14 @@ static int build_walk_once(long long nrays, const double* d_ends, const RayGrid&
     auto* down = static_cast<unsigned char*>(bufs.get((size_t)nrays));
     auto* info = static_cast<int*>(bufs.get(64));  // tallest, overrun
     void* stmp = bufs.get(scan_tmp_bytes(nrays));
-    if (!height || !off || !count || !down || !info || !stmp) return bufs.fail();
+    if (!height || !off || !count || !down || !info || !stmp) return ST_OK;
+    auto allocate = [&](auto** p, size_t n) {
+        if (cudaMalloc(p, n * sizeof(**p)) == cudaSuccess) return true;
+        cudaGetLastError();
+        *p = nullptr;
+        out->release();
+        return false;
+    };
     ST_CUDA(cudaMemsetAsync(info, 0, 2 * sizeof(int), st));
     ray_bound_kernel<<<grid_for(tiles * 32), 256, 0, st>>>(d_ends, nrays, G, height, info);
     count_launch();
@@ -379,12 +389,12 @@ static int build_walk_once(long long nrays, const double* d_ends, const RayGrid&
     if (smem > 200 * 1024) return ST_OK;
     auto* scol = static_cast<int*>(bufs.get((size_t)rows * 32 * 4));
     auto* sval = static_cast<float*>(bufs.get((size_t)rows * 32 * 4));
-    if (!scol || !sval) return bufs.fail();
+    if (!scol || !sval) return ST_OK;
     ray_walk_kernel<<<(unsigned)std::min<long long>((nrays + 127) / 128, 1 << 20), 128, 0, st>>>(
         d_ends, nrays, G, height, off, scol, sval, count, down, info + 1);
     count_launch();
     ST_CUDA(cudaGetLastError());
-    ST_CUDA(cudaMalloc(&out->row_ptr, (size_t)(nrays + 1) * sizeof(long long)));
+    if (!allocate(&out->row_ptr, (size_t)(nrays + 1))) return ST_OK;
     ST_TRY(exclusive_scan_i64(count, out->row_ptr, nrays, out->row_ptr + nrays, stmp, st));
     long long nnz = 0;
     ST_CUDA(cudaMemcpyAsync(&nnz, out->row_ptr + nrays, sizeof(nnz), cudaMemcpyDeviceToHost, st));
@@ -395,8 +405,8 @@ static int build_walk_once(long long nrays, const double* d_ends, const RayGrid&
         return ST_OK;
     }
     ST_CHECK(nnz < (1ll << 32), ST_ERR_ARG, "at most 2^32-1 triplets per build");
-    ST_CUDA(cudaMalloc(&out->col, (size_t)std::max<long long>(nnz, 1) * sizeof(int)));
-    ST_CUDA(cudaMalloc(&out->val, (size_t)std::max<long long>(nnz, 1) * sizeof(float)));
+    if (!allocate(&out->col, (size_t)std::max<long long>(nnz, 1))) return ST_OK;
+    if (!allocate(&out->val, (size_t)std::max<long long>(nnz, 1))) return ST_OK;
     out->rows = nrays;
     out->cols = (long long)G.nx * G.ny * G.nz;
     out->nnz = nnz;
