@@ -152,33 +152,6 @@ __global__ void pad_scatter_kernel(const long long* __restrict__ rp, const int* 
 
 __global__ void fill_last_kernel(long long* rp, long long R, const long long* total) { rp[R] = *total; }
 
-// A sum of a few products held as an unevaluated pair of FP32 values (Dot2 of
-// Ogita, Rump and Oishi, "Accurate sum and dot product", 2005): the products are
-// split exactly by FMA and the rounding error of every addition is kept, so eight
-// products lose at most (8 * 2^-24)^2 of their magnitude, typically 2^-49. The FP64
-// pipe takes a warp's operation in 16 cycles here (conversions too), the
-// FP32 one in a quarter of a cycle: a kernel adds up to eight products so and
-// then folds the pair into its FP64 sum. Only for factors that pair_safe admits:
-// zero or 2^-50 .. 2^60, so that no product or error term over- or underflows; the
-// callers take FP64 products otherwise (tiny gradients, infinities, NaN).
-__device__ __forceinline__ bool pair_safe(float a) {
-    const unsigned m = __float_as_uint(a) & 0x7fffffffu;
-    return (m - 0x26800000u <= 0x5d800000u - 0x26800000u) | (m == 0u);
-}
-struct PairSum {
-    float h = 0.0f, l = 0.0f;
-    __device__ __forceinline__ void add(float a, float b) {
-        const float p = __fmul_rn(a, b);
-        const float e = __fmaf_rn(a, b, -p);
-        const float t = __fadd_rn(h, p);
-        const float z = __fsub_rn(t, h);
-        const float err = __fadd_rn(__fsub_rn(h, __fsub_rn(t, z)), __fsub_rn(p, z));
-        h = t;
-        l = __fadd_rn(l, __fadd_rn(e, err));
-    }
-    __device__ __forceinline__ double value() const { return (double)h + (double)l; }
-};
-
 // A sum of products held as an unevaluated triple of FP32 values (the three-fold
 // sum of Ogita, Rump and Oishi, "Accurate sum and dot product", 2005): the products
 // are split exactly by FMA, the rounding errors of the leading sum and of the sum
@@ -495,8 +468,8 @@ inline bool quads_ok(std::initializer_list<const void*> ps) {
 // Bound by memory (8 words per unknown): read and written
 // four unknowns at a time where the caller's x allows it (quads), so that a
 // thread has five 16-byte loads in flight, with the inner products carried in
-// pairs of FP32 values within a quad. 16.8M unknowns: 85 us (a copy of the bytes
-// takes 79), 146 with FP64 products, 169 with single words as well.
+// triples of FP32 values over the thread's quads. 16.8M unknowns: 83 us (a copy of
+// the bytes takes 79), 146 with FP64 products, 169 with single words as well.
 // alpha = rz_old / pq; |pq| < 1e-30 stops the solve (sparse_ops.cpp:37,88).
 // The scalars are formed once per block (FP64 is a slow pipe on this GPU).
 // skip_rz: <r, z> comes from the stencil preconditioner's kernel instead.
@@ -527,6 +500,8 @@ __global__ void cg_update_kernel(long long n, float* __restrict__ x, float* __re
     if (s_stop) return;
     const float alpha = s_alpha;
     double a = 0.0, c = 0.0;
+    TripleSum rz, rr;
+    int held = 0;  // products in each triple
     const long long n4 = quads ? n >> 2 : 0;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
         const float4 p4 = reinterpret_cast<const float4*>(p)[i], q4 = reinterpret_cast<const float4*>(q)[i];
@@ -540,15 +515,14 @@ __global__ void cg_update_kernel(long long n, float* __restrict__ x, float* __re
         reinterpret_cast<float4*>(x)[i] = x4;
         reinterpret_cast<float4*>(r)[i] = r4;
         if (z) reinterpret_cast<float4*>(z)[i] = z4;
-        const bool safe = pair_safe(r4.x) & pair_safe(r4.y) & pair_safe(r4.z) & pair_safe(r4.w) & pair_safe(z4.x) &
-                          pair_safe(z4.y) & pair_safe(z4.z) & pair_safe(z4.w);
+        const bool safe = triple_safe(r4.x) & triple_safe(r4.y) & triple_safe(r4.z) & triple_safe(r4.w) &
+                          triple_safe(z4.x) & triple_safe(z4.y) & triple_safe(z4.z) & triple_safe(z4.w);
         if (!safe) {
             const double r0 = r4.x, r1 = r4.y, r2 = r4.z, r3 = r4.w;
             a += (r0 * (double)z4.x + r1 * (double)z4.y) + (r2 * (double)z4.z + r3 * (double)z4.w);
             c += (r0 * r0 + r1 * r1) + (r2 * r2 + r3 * r3);
             continue;
         }
-        PairSum rz, rr;
         rz.add(r4.x, z4.x);
         rz.add(r4.y, z4.y);
         rz.add(r4.z, z4.z);
@@ -557,9 +531,15 @@ __global__ void cg_update_kernel(long long n, float* __restrict__ x, float* __re
         rr.add(r4.y, r4.y);
         rr.add(r4.z, r4.z);
         rr.add(r4.w, r4.w);
-        a += rz.value();
-        c += rr.value();
+        if ((held += 4) == TRIPLE_MAX) {
+            a += rz.value();
+            c += rr.value();
+            rz = rr = TripleSum();
+            held = 0;
+        }
     }
+    a += rz.value();
+    c += rr.value();
     for (long long i = 4 * n4 + blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
          i += (long long)gridDim.x * blockDim.x) {
         x[i] = fmaf(alpha, p[i], x[i]);

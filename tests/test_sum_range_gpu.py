@@ -1,6 +1,7 @@
 """Sums of products at the edges of the FP32 triples that carry them: the
 normal-equation diagonal (both kernels) where the squares' sum leaves the FP32
-range and where it needs all of FP64's bits. Every expected value is exact."""
+range and where it needs all of FP64's bits, and the CG residual likewise. Every
+expected value is exact."""
 import numpy as np
 import pytest
 import torch
@@ -45,3 +46,15 @@ def test_diagonal_keeps_every_bit_of_fp64(fill):
     # squares 2^24 + 1 + 4 * 2^-28, 53 bits in any order of summation; lam leaves the last
     A, cols = _matrix([[2.0 ** 12, 1.0] + [2.0 ** -14] * 4], 100, fill)
     assert _diagonal(A, cols, -(2.0 ** 24 + 1.0))[0] == 2.0 ** 26
+
+
+def test_cg_residual_keeps_every_bit_of_fp64():
+    # r = b / 2 after one step with alpha = 1/2 (diagonal 1 and 3 in equal parts); the squares of a quad
+    # need 52 bits, and so do the sums of 32 equal quads
+    n = 128
+    diag = np.where(np.arange(n) < n // 2, 1.0, 3.0)
+    A = se.CSRMatrix().build_from_triplets(n, n, np.arange(n), np.arange(n), diag)
+    b = np.tile([2.0 ** 13, 2.0, 1.5 * 2.0 ** -12, 1.5 * 2.0 ** -12], n // 4)
+    se.SparseOps.conjugate_gradient(A, b, 1, 1e-30)
+    assert se.SparseOps.last_iterations == 1
+    assert se.SparseOps.last_relative_residual == 0.5
