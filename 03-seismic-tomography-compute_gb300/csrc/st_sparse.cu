@@ -299,6 +299,7 @@ __device__ __forceinline__ void copy16_async(void* dst, const void* src, int byt
 // turn at fewer warps per SM 28.0.
 constexpr int SR_ROWS = 128;
 constexpr int SR_CAP = 1408;  // entries of a tile (11 per row): 11 KB, sixteen CTAs per SM
+template <bool SPLIT>
 __global__ void __launch_bounds__(SR_ROWS, 16) spmv_rows_kernel(const long long* __restrict__ rp, const int* __restrict__ col,
                                                               const float* __restrict__ val,
                                                               const float* __restrict__ x, float* __restrict__ y,
@@ -330,26 +331,25 @@ __global__ void __launch_bounds__(SR_ROWS, 16) spmv_rows_kernel(const long long*
             }
             asm volatile("cp.async.wait_all;" ::: "memory");
             __syncthreads();
-            // four strided partial sums, as four lanes per row would hold
-            float t0 = 0.0f, t1 = 0.0f, t2 = 0.0f, t3 = 0.0f;
+            // four strided partial sums; SPLIT: each in two parts, its second and fourth
+            // entry in the other one (the shorter chains of four lanes per row)
+            float t[4] = {0.0f, 0.0f, 0.0f, 0.0f}, u[4] = {0.0f, 0.0f, 0.0f, 0.0f};
             const int kb = (int)(b - base);
-            int k = (int)(a - base);
-            for (; k + 4 <= kb; k += 4) {
-                const float x0 = __ldg(x + scol[k]), x1 = __ldg(x + scol[k + 1]), x2 = __ldg(x + scol[k + 2]),
-                            x3 = __ldg(x + scol[k + 3]);
-                t0 += __fmul_rn(sval[k], x0);
-                t1 += __fmul_rn(sval[k + 1], x1);
-                t2 += __fmul_rn(sval[k + 2], x2);
-                t3 += __fmul_rn(sval[k + 3], x3);
+            for (int k = (int)(a - base), j = 0; k < kb; k += 4, ++j) {
+                float xs[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) xs[i] = k + i < kb ? __ldg(x + scol[k + i]) : 0.0f;
+                if (SPLIT && (j == 1 || j == 3)) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        if (k + i < kb) u[i] = fmaf(sval[k + i], xs[i], u[i]);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        if (k + i < kb) t[i] = fmaf(sval[k + i], xs[i], t[i]);
+                }
             }
-            float x0 = 0.0f, x1 = 0.0f, x2 = 0.0f;
-            if (k < kb) x0 = __ldg(x + scol[k]);
-            if (k + 1 < kb) x1 = __ldg(x + scol[k + 1]);
-            if (k + 2 < kb) x2 = __ldg(x + scol[k + 2]);
-            if (k < kb) t0 += __fmul_rn(sval[k], x0);
-            if (k + 1 < kb) t1 += __fmul_rn(sval[k + 1], x1);
-            if (k + 2 < kb) t2 += __fmul_rn(sval[k + 2], x2);
-            sum = (t0 + t2) + (t1 + t3);
+            sum = ((t[0] + u[0]) + (t[2] + u[2])) + ((t[1] + u[1]) + (t[3] + u[3]));
             __syncthreads();
         } else {
             const int lane = tid & 31;
@@ -384,8 +384,8 @@ int launch_spmv_rows(const DevCsr& A, const float* x, float* y, const float* add
                      double* dot_acc, const int* done, cudaStream_t st) {
     const long long tiles = (A.rows + SR_ROWS - 1) / SR_ROWS;
     const unsigned blocks = (unsigned)std::max<long long>(1, std::min<long long>(tiles, grid_cap()));  // 16 per SM
-    spmv_rows_kernel<<<blocks, SR_ROWS, 0, st>>>(A.row_ptr, A.col, A.val, x, y, A.rows, add, add_scale, pdot, dot_acc,
-                                                 done);
+    const auto kernel = A.nnz >= 5 * A.rows ? spmv_rows_kernel<true> : spmv_rows_kernel<false>;
+    kernel<<<blocks, SR_ROWS, 0, st>>>(A.row_ptr, A.col, A.val, x, y, A.rows, add, add_scale, pdot, dot_acc, done);
     count_launch();
     ST_CUDA(cudaGetLastError());
     return ST_OK;

@@ -1,7 +1,7 @@
 """Sums of products at the edges of the FP32 triples that carry them: the
 normal-equation diagonal (both kernels) where the squares' sum leaves the FP32
-range and where it needs all of FP64's bits, and the CG residual likewise. Every
-expected value is exact."""
+range and where it needs all of FP64's bits, the CG residual likewise, and the
+short-row product where one rounding a term shows. Every expected value is exact."""
 import numpy as np
 import pytest
 import torch
@@ -58,3 +58,21 @@ def test_cg_residual_keeps_every_bit_of_fp64():
     se.SparseOps.conjugate_gradient(A, b, 1, 1e-30)
     assert se.SparseOps.last_iterations == 1
     assert se.SparseOps.last_relative_residual == 0.5
+
+
+@pytest.mark.parametrize("lengths", [[9] * 300, [9] * 7 + [3] * 290])
+def test_short_row_products_are_fused(lengths):
+    # the ninth entry cancels the first to 2^-46, which a product rounded before the addition loses
+    rows, cols = len(lengths), 200
+    r = np.repeat(np.arange(rows), lengths)
+    k = np.concatenate([np.arange(m) for m in lengths])
+    e = 2.0 ** -23
+    v = np.where(k == 0, 1.0, np.where(k == 8, -(1.0 - e), 0.0))
+    x = np.zeros(cols, np.float32)
+    x[0], x[8] = 1.0, 1.0 + e
+    A = se.CSRMatrix().build_from_triplets(rows, cols, r, k, v)
+    xd, y = torch.from_numpy(x).cuda(), torch.zeros(rows, device="cuda")
+    torch.cuda.synchronize()
+    A.spmv_device(xd, y)
+    torch.cuda.synchronize()
+    assert np.array_equal(y.cpu().numpy(), np.where(np.array(lengths) > 8, np.float32(e * e), np.float32(1.0)))
