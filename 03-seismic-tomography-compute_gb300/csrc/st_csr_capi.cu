@@ -31,7 +31,15 @@ int ensure_transpose(st_csr* m) {
     if (m->has_T) return ST_OK;
     ST_TRY(build_transpose(m->A, &m->AT, m->stream));
     m->has_T = true;
-    return ST_OK;
+    return find_uneven_rows(&m->AT, m->dacc, m->stream);
+}
+
+// The handle takes a matrix that has just been built.
+int take_matrix(st_csr* m, const DevCsr& built) {
+    m->A.release();
+    drop_transpose(m);
+    m->A = built;
+    return find_uneven_rows(&m->A, m->dacc, m->stream);
 }
 
 struct Scratch {
@@ -139,10 +147,7 @@ int st_csr_build_from_triplets(st_csr* m, int64_t rows, int64_t cols, int64_t n,
         return rc;
     }
     ST_CUDA(cudaStreamSynchronize(m->stream));
-    m->A.release();
-    drop_transpose(m);
-    m->A = out;
-    return ST_OK;
+    return take_matrix(m, out);
 }
 
 int st_csr_build_from_triplets_device(st_csr* m, int64_t rows, int64_t cols, int64_t n, const int32_t* r,
@@ -155,10 +160,7 @@ int st_csr_build_from_triplets_device(st_csr* m, int64_t rows, int64_t cols, int
         out.release();
         return rc;
     }
-    m->A.release();
-    drop_transpose(m);
-    m->A = out;
-    return ST_OK;
+    return take_matrix(m, out);
 }
 
 int st_csr_build_fd_stencil_7point(st_csr* m, int64_t nx, int64_t ny, int64_t nz, const double* velocity, double dx,
@@ -182,10 +184,7 @@ int st_csr_build_fd_stencil_7point(st_csr* m, int64_t nx, int64_t ny, int64_t nz
         out.release();
         return rc;
     }
-    m->A.release();
-    drop_transpose(m);
-    m->A = out;
-    return ST_OK;
+    return take_matrix(m, out);
 }
 
 int st_csr_build_ray_matrix(st_csr* m, int64_t n_rays, const double* endpoints, int on_device, int64_t nx,
@@ -210,9 +209,7 @@ int st_csr_build_ray_matrix(st_csr* m, int64_t n_rays, const double* endpoints, 
         out.release();
         return rc;
     }
-    m->A.release();
-    drop_transpose(m);
-    m->A = out;
+    ST_TRY(take_matrix(m, out));
     if (nnz) *nnz = total;
     return ST_OK;
 }
@@ -227,9 +224,7 @@ int st_csr_build_sampled_ray_matrix(st_csr* m, st_ray_picks* p, int64_t* nnz) {
         out.release();
         return rc;
     }
-    m->A.release();
-    drop_transpose(m);
-    m->A = out;
+    ST_TRY(take_matrix(m, out));
     if (nnz) *nnz = total;
     return ST_OK;
 }
@@ -351,6 +346,7 @@ int st_csr_clone(st_csr* m, st_csr** out) {
     ST_CHECK(m && out, ST_ERR_ARG, "null argument");
     ST_TRY(st_csr_create(m->A.rows, m->A.cols, m->A.nnz, m->device, out));
     st_csr* c = *out;
+    c->A.lanes = m->A.lanes;
     ST_CUDA(cudaMemcpy(c->A.row_ptr, m->A.row_ptr, (size_t)(m->A.rows + 1) * 8, cudaMemcpyDeviceToDevice));
     if (m->A.nnz) {
         ST_CUDA(cudaMemcpy(c->A.col, m->A.col, (size_t)m->A.nnz * 4, cudaMemcpyDeviceToDevice));

@@ -291,7 +291,9 @@ __device__ __forceinline__ void copy16_async(void* dst, const void* src, int byt
 // of a row, seven lines, and the L1 set the pace. A group of lanes per row spends
 // most of its instructions on predicates and waits for the row pointers, the
 // columns and the gathers one after another for 28 bytes of values. A tile with
-// more entries than fit in shared memory is summed a warp per row.
+// more entries than fit in shared memory is summed a warp per row; matrices with much
+// of their entries in such tiles, or in tiles with a long row that one thread works
+// through, go to a group of lanes per row (find_uneven_rows).
 // 7 entries per row on a 256^3 grid, 72 bytes per row: 199 us a product (a copy of
 // the bytes takes 178); products along the stream 244, four lanes per row 600. 40
 // CG iterations there with tiles of 256 / 128 / 64 rows 24.3 / 23.5 / 23.3 ms
@@ -299,6 +301,8 @@ __device__ __forceinline__ void copy16_async(void* dst, const void* src, int byt
 // turn at fewer warps per SM 28.0.
 constexpr int SR_ROWS = 128;
 constexpr int SR_CAP = 1408;  // entries of a tile (11 per row): 11 KB, sixteen CTAs per SM
+constexpr int SR_LONG = 32;   // a longer row makes its tile wait for the thread that has it
+constexpr long long SHORT_ROWS = 10;
 template <bool SPLIT>
 __global__ void __launch_bounds__(SR_ROWS, 16) spmv_rows_kernel(const long long* __restrict__ rp, const int* __restrict__ col,
                                                               const float* __restrict__ val,
@@ -907,10 +911,57 @@ template int build_csr<long long, double>(long long, long long, long long, const
 template int build_csr<int, float>(long long, long long, long long, const int*, const int*, const float*, bool,
                                    DevCsr*, cudaStream_t);
 
+// What spmv_rows_kernel is slow on, a warp per tile: out[0] the entries in tiles
+// beyond shared memory or with a long row, out[1] the longest row, out[2] the
+// entries of the heaviest tile.
+__global__ void uneven_tiles_kernel(const long long* __restrict__ rp, long long rows, unsigned long long* out) {
+    const int lane = threadIdx.x & 31;
+    unsigned long long entries = 0, longest = 0, heaviest = 0;
+    for (long long r0 = ((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5) * SR_ROWS; r0 < rows;
+         r0 += (((long long)gridDim.x * blockDim.x) >> 5) * SR_ROWS) {
+        const long long total = rp[min(r0 + SR_ROWS, rows)] - rp[r0];
+        long long most = 0;
+        for (long long r = r0 + lane; r < min(r0 + SR_ROWS, rows); r += 32) most = max(most, rp[r + 1] - rp[r]);
+        for (int o = 16; o > 0; o >>= 1) most = max(most, __shfl_xor_sync(FULL, most, o));
+        if (most > SR_LONG || total > SR_CAP - 3) entries += (unsigned long long)total;
+        longest = max(longest, (unsigned long long)most);
+        heaviest = max(heaviest, (unsigned long long)total);
+    }
+    if (lane == 0 && entries) {
+        atomicAdd(out, entries);
+        atomicMax(out + 1, longest);
+        atomicMax(out + 2, heaviest);
+    }
+}
+
+// Where an eighth of the entries or more lie in such tiles, the rows go to groups
+// of lanes: two lanes (fewer than five entries a row) or four, and eight where single
+// rows set the pace (beyond 1024 entries); those keep a warp to themselves in the row
+// tiles unless they share a tile or hardly a tile is without one. 1M rows, row tiles / lanes, us: a half of 18 entries
+// and a half of none 56 / 33; 1 row of 128 at 600, the others 3, 149 / 82; a power law
+// of mean 6.2 up to 2000 sorted by length 552 / 57, in random order 106 / 82; 1 row of
+// 1000 at 4000 101 / 120 (four lanes 149); 1000 rows, one of 5000, 61 / 53.
+int find_uneven_rows(DevCsr* A, void* scratch, cudaStream_t st) {
+    A->lanes = 0;
+    if (A->rows == 0 || A->nnz >= SHORT_ROWS * A->rows) return ST_OK;
+    auto* acc = static_cast<unsigned long long*>(scratch);
+    unsigned long long h[3] = {0, 0, 0};
+    ST_CUDA(cudaMemsetAsync(acc, 0, sizeof(h), st));
+    uneven_tiles_kernel<<<blocks_for((A->rows + SR_ROWS - 1) / SR_ROWS * 32), 256, 0, st>>>(A->row_ptr, A->rows, acc);
+    count_launch();
+    ST_CUDA(cudaGetLastError());
+    ST_CUDA(cudaMemcpyAsync(h, acc, sizeof(h), cudaMemcpyDeviceToHost, st));
+    ST_CUDA(cudaStreamSynchronize(st));
+    if (8 * h[0] <= (unsigned long long)A->nnz) return ST_OK;
+    if (h[1] <= 1024) A->lanes = A->nnz >= 5 * A->rows ? 4 : 2;
+    else if (h[2] > 8192 || 16 * h[0] > 15 * (unsigned long long)A->nnz) A->lanes = 8;
+    return ST_OK;
+}
+
 int launch_spmv(const DevCsr& A, const float* x, float* y, const float* add, float add_scale, const float* pdot,
                 double* dot_acc, const int* done, cudaStream_t st) {
     const double avg = A.rows > 0 ? (double)A.nnz / (double)A.rows : 0.0;
-    // tuning override: SEISMIC_GB300_SPMV_G=<1|8|16|32> threads per row
+    // tuning override: SEISMIC_GB300_SPMV_G=<1|2|4|8|16|32> threads per row
     static const int forced = [] {
         const char* e = std::getenv("SEISMIC_GB300_SPMV_G");
         return e ? std::atoi(e) : 0;
@@ -919,6 +970,8 @@ int launch_spmv(const DevCsr& A, const float* x, float* y, const float* add, flo
         case 32: return launch_spmv_g<32, 6, false, true>(A, x, y, add, add_scale, pdot, dot_acc, done, st);
         case 16: return launch_spmv_g<16, 10, true, false>(A, x, y, add, add_scale, pdot, dot_acc, done, st);
         case 8: return launch_spmv_g<8, 4, true, false>(A, x, y, add, add_scale, pdot, dot_acc, done, st);
+        case 4: return launch_spmv_g<4, 4, false, false>(A, x, y, add, add_scale, pdot, dot_acc, done, st);
+        case 2: return launch_spmv_g<2, 4, false, false>(A, x, y, add, add_scale, pdot, dot_acc, done, st);
         case 1: return launch_spmv_rows(A, x, y, add, add_scale, pdot, dot_acc, done, st);
         default: break;
     }
@@ -927,7 +980,10 @@ int launch_spmv(const DevCsr& A, const float* x, float* y, const float* add, flo
     // threads, 6 entries per lane, no prefetch and the rest in turns 0.570 ms (0.640 with the rest one by one)
     if (avg >= 256) return launch_spmv_g<32, 6, false, true>(A, x, y, add, add_scale, pdot, dot_acc, done, st);
     if (avg >= 24) return launch_spmv_g<16, 10, true, false>(A, x, y, add, add_scale, pdot, dot_acc, done, st);
-    if (avg >= 10) return launch_spmv_g<8, 4, true, false>(A, x, y, add, add_scale, pdot, dot_acc, done, st);
+    if (avg >= SHORT_ROWS) return launch_spmv_g<8, 4, true, false>(A, x, y, add, add_scale, pdot, dot_acc, done, st);
+    if (A.lanes == 8) return launch_spmv_g<8, 4, true, false>(A, x, y, add, add_scale, pdot, dot_acc, done, st);
+    if (A.lanes == 4) return launch_spmv_g<4, 4, false, false>(A, x, y, add, add_scale, pdot, dot_acc, done, st);
+    if (A.lanes == 2) return launch_spmv_g<2, 4, false, false>(A, x, y, add, add_scale, pdot, dot_acc, done, st);
     return launch_spmv_rows(A, x, y, add, add_scale, pdot, dot_acc, done, st);
 }
 

@@ -13,6 +13,7 @@ struct DevCsr {
     long long* row_ptr = nullptr;
     int* col = nullptr;
     float* val = nullptr;
+    int lanes = 0;  // lanes per row of products with uneven short rows, 0: even ones (find_uneven_rows)
     void release() {
         cudaFree(row_ptr);
         cudaFree(col);
@@ -109,6 +110,8 @@ template <class TI, class TV>
 int build_csr(long long rows, long long cols, long long n, const TI* r, const TI* c, const TV* v, bool pad,
               DevCsr* out, cudaStream_t st);
 int build_transpose(const DevCsr& A, DevCsr* T, cudaStream_t st);
+// Sets A->lanes from the row pointers; scratch: 24 bytes on the device. Waits for the stream.
+int find_uneven_rows(DevCsr* A, void* scratch, cudaStream_t st);
 // Straight-ray path-length matrix (st_rays.cu): d_ends = device [nrays][6]
 // endpoints in cell units; total_nnz (may be null) receives the entry count.
 int build_ray_csr(long long nrays, const double* d_ends, int nx, int ny, int nz, double h, DevCsr* out,
