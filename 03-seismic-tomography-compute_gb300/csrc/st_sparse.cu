@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "st_sparse.cuh"
+#include "st_update.cuh"
 
 #include <cstdlib>
 
@@ -186,6 +187,27 @@ struct TripleSum {
         l = __fadd_rn(__fadd_rn(l, t.l), __fadd_rn(f, g));
     }
     __device__ __forceinline__ double value() const { return (double)h + ((double)m + (double)l); }
+};
+// Two of them, an instruction for both.
+__device__ __forceinline__ F2 two_sum(F2 a, F2 b, F2& s) {
+    const F2 n1 = pack(-1.0f, -1.0f), t = add2(a, b), z = fma2(n1, a, t);
+    s = t;
+    return add2(fma2(n1, fma2(n1, z, t), a), fma2(n1, z, b));
+}
+struct TripleSum2 {
+    F2 h{0}, m{0}, l{0};
+    __device__ __forceinline__ void add_squares(F2 a) {
+        const F2 p = mul2(a, a), e = two_sum(h, p, h), f = two_sum(m, fma2(a, a, fma2(p, pack(-1.0f, -1.0f), F2{0})), m),
+                 g = two_sum(m, e, m);
+        l = add2(l, add2(f, g));
+    }
+    __device__ __forceinline__ TripleSum half(int k) const {
+        TripleSum a, b;
+        unpack(h, a.h, b.h);
+        unpack(m, a.m, b.m);
+        unpack(l, a.l, b.l);
+        return k ? b : a;
+    }
 };
 
 // ---------------------------------------------------------------- SpMV
@@ -642,62 +664,125 @@ __global__ void jacobi_kernel(const long long* __restrict__ rp, const int* __res
     }
 }
 
-// diag of A^T A + lam I from the rows of A^T: 1 / (sum_k AT[j,k]^2 + lam). A warp
-// per row, its lanes over the entries (coalesced). The rows of a warp lie a grid
-// apart (neighbouring cells are heavy together: where rays meet, a row holds
-// thousands of entries), and each group of 32 keeps row w's sum on lane w, so
-// that the FP64 division runs on full warps; triples of FP32 values carry the
-// squares until then, and rows they cannot hold are summed in FP64. 1M rows of 202
-// entries: 0.58 ms, bound by the FP32 instructions of the triples (1.21 with FP64
-// sums and a thread per row; pairs took 0.41 and lost what lies beyond 2^-48, and
-// the whole sum beyond 2^128). Short rows (less than 24 entries) are staged through
-// shared memory instead, a thread per row: 7.1M rows of 7 entries 0.18 ms (0.28
-// with FP64 sums).
-__global__ void normal_jacobi_kernel(const long long* __restrict__ rp, const float* __restrict__ val, long long rows,
-                                     double lam, float* __restrict__ dinv) {
-    const int lane = threadIdx.x & 31;
-    const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
-    const long long first = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-    for (long long r0 = first; r0 < rows; r0 += 32 * warps) {
+// diag of A^T A + lam I from the rows of A^T: 1 / (sum_k AT[j,k]^2 + lam). G lanes
+// per row, over its entries (coalesced); a group's rows lie a grid apart (neighbouring
+// cells are heavy together: where rays meet, a row holds thousands of entries), and
+// lane w keeps the sum of its w-th row, so that the FP64 division runs on full warps.
+// Triples of FP32 values carry the squares, two to an instruction, and rows with a
+// value they cannot hold are summed in FP64. Bound by the FP32 instructions. Eight
+// lanes join a row's sums in three steps for four rows at once; rows beyond NJ_FAR go
+// to the whole warp. 8 / 32 lanes, us: 262,144 rows of 40 entries 31 / 87 (47 a thread
+// per row in FP64), of 202 80 / 128 (214), 131,072 rows of 361 67 / 90 (213); means of
+// 3000 from 2 to 20,000 45 / 21. Triples one at a time, 32 lanes: 117, 146, 101.
+// Short rows (less than 24 entries on average) are staged through shared memory
+// instead, a thread per row: 2M rows of 7 entries 58 us (85 in FP64).
+constexpr int NJ_FAR = 512;  // rows that groups of eight leave to the warp
+
+// This lane's squares among [a, b), G lanes over them; full triples go to far.
+// Two sums per instruction, joined at the end. Whether a value does not fit.
+template <int G>
+__device__ __forceinline__ unsigned add_squares(const float* __restrict__ val, long long a, long long b, int lane,
+                                                TripleSum& s, double& far) {
+    unsigned odd = 0;
+    int held = 0;
+    TripleSum2 t;
+    for (long long q = a + lane; q - lane < b; q += 8 * G) {
+        float v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = q + G * k < b ? __ldg(val + q + G * k) : 0.0f;
+#pragma unroll
+        for (int k = 0; k < 8; k += 2)
+            if (k == 0 || q + G * k < b) {
+                odd |= triple_safe(v[k]) & triple_safe(v[k + 1]) ? 0u : 1u;
+                t.add_squares(pack(v[k], v[k + 1]));
+            }
+        if ((held += 4) == TRIPLE_MAX) {
+            far += t.half(0).value() + t.half(1).value();
+            t = TripleSum2();
+            held = 0;
+        }
+    }
+    s = t.half(0);
+    s.merge(t.half(1));
+    return odd;
+}
+
+template <int G>
+__device__ __forceinline__ void merge_lanes(TripleSum& s, double& far) {
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) {
+        TripleSum t;
+        t.h = __shfl_xor_sync(FULL, s.h, o);
+        t.m = __shfl_xor_sync(FULL, s.m, o);
+        t.l = __shfl_xor_sync(FULL, s.l, o);
+        s.merge(t);
+    }
+    if (__any_sync(FULL, far != 0.0)) {
+#pragma unroll
+        for (int o = G / 2; o > 0; o >>= 1) far += __shfl_xor_sync(FULL, far, o);
+    }
+}
+
+// The same sum in FP64.
+template <int G>
+__device__ __noinline__ double squares64(const float* __restrict__ val, long long a, long long b, int lane) {
+    double t = 0.0;
+    for (long long e = a + lane; e < b; e += G) t += (double)val[e] * (double)val[e];
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) t += __shfl_xor_sync(FULL, t, o);
+    return t;
+}
+
+template <int G>
+__global__ void __launch_bounds__(256, 4) normal_jacobi_kernel(const long long* __restrict__ rp,
+                                                               const float* __restrict__ val, long long rows, double lam,
+                                                               float* __restrict__ dinv) {
+    const int lane = threadIdx.x % G, wl = threadIdx.x & 31;
+    const long long groups = (long long)gridDim.x * (blockDim.x / G);
+    const long long first = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / G;
+    const int ahead = (wl - lane) / G;  // groups of the warp before this one
+    for (long long r0 = first; r0 - ahead < rows; r0 += G * groups) {
         TripleSum mine;
-        double wide = -1.0;  // the sum where the triples cannot hold it
-        for (int w = 0; w < 32; ++w) {
-            const long long r = r0 + w * warps;
-            if (r >= rows) break;
-            const long long ra = rp[r], rb = rp[r + 1];
+        double mfar = 0.0;
+        for (int w = 0; w < G && r0 - ahead + w * groups < rows; ++w) {
+            const long long r = r0 + w * groups;
+            const long long a = r < rows ? rp[r] : 0, b = r < rows ? rp[r + 1] : 0;
+            const bool rest = G < 32 && b - a > NJ_FAR;
             TripleSum s;
-            unsigned odd = rb - ra > 32 * TRIPLE_MAX ? 1u : 0u;
-            for (long long q = ra + lane; !odd && q - lane < rb; q += 8 * 32) {
-                float v[8];
-#pragma unroll
-                for (int k = 0; k < 8; ++k) v[k] = q + 32 * k < rb ? __ldg(val + q + 32 * k) : 0.0f;
-#pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    odd |= triple_safe(v[k]) ? 0u : 1u;
-                    s.add(v[k], v[k]);
+            double far = 0.0;
+            unsigned odd = __ballot_sync(FULL, add_squares<G>(val, a, rest ? a : b, lane, s, far));
+            merge_lanes<G>(s, far);
+            if (odd) {
+                const double t = squares64<G>(val, a, rest ? a : b, lane);
+                if ((odd >> (wl - lane)) & (FULL >> (32 - G))) {
+                    s = TripleSum();
+                    far = t;
                 }
             }
-            if (!__any_sync(FULL, odd)) {
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    TripleSum t;
-                    t.h = __shfl_xor_sync(FULL, s.h, o);
-                    t.m = __shfl_xor_sync(FULL, s.m, o);
-                    t.l = __shfl_xor_sync(FULL, s.l, o);
-                    s.merge(t);
+            if (lane == w) {
+                mine = s;
+                mfar = far;
+            }
+            if constexpr (G < 32) {
+                for (unsigned m = __ballot_sync(FULL, rest && lane == 0); m; m &= m - 1) {
+                    const int src = __ffs((int)m) - 1;
+                    const long long fa = __shfl_sync(FULL, a, src), fb = __shfl_sync(FULL, b, src);
+                    far = 0.0;
+                    odd = __ballot_sync(FULL, add_squares<32>(val, fa, fb, wl, s, far));
+                    merge_lanes<32>(s, far);
+                    if (odd) {
+                        s = TripleSum();
+                        far = squares64<32>(val, fa, fb, wl);
+                    }
+                    if (wl == src + w) {
+                        mine = s;
+                        mfar = far;
+                    }
                 }
-                if (lane == w) mine = s;
-            } else {
-                double t = 0.0;
-                for (long long e = ra + lane; e < rb; e += 32) t += (double)val[e] * (double)val[e];
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(FULL, t, o);
-                if (lane == w) wide = t;
             }
         }
-        const double sum = wide >= 0.0 || wide != wide ? wide : mine.value();
-        const long long i = r0 + lane * warps;
-        if (i < rows) dinv[i] = (float)(1.0 / (sum + lam));
+        const long long i = r0 + lane * groups;
+        if (i < rows) dinv[i] = (float)(1.0 / (mfar + mine.value() + lam));
     }
 }
 
@@ -715,14 +800,26 @@ __global__ void __launch_bounds__(NJ_ROWS) normal_jacobi_rows_kernel(const long 
         if (staged)
             for (long long e = e0 + threadIdx.x; e < e1; e += NJ_ROWS) v[e - e0] = __ldg(val + e);
         __syncthreads();
-        TripleSum s;
-        bool safe = staged && b - a <= TRIPLE_MAX;
-        if (safe)
-            for (int k = (int)(a - e0); k < (int)(b - e0); ++k) {
-                safe = safe & triple_safe(v[k]);
-                s.add(v[k], v[k]);
+        TripleSum2 s;
+        double t = 0.0;
+        bool safe = staged;
+        if (staged) {
+            const int kb = (int)(b - e0);
+            int held = 0;
+            for (int k = (int)(a - e0); k < kb; k += 2) {
+                const float v0 = v[k], v1 = k + 1 < kb ? v[k + 1] : 0.0f;
+                safe = safe & triple_safe(v0) & triple_safe(v1);
+                s.add_squares(pack(v0, v1));
+                if (++held == TRIPLE_MAX) {
+                    t += s.half(0).value() + s.half(1).value();
+                    s = TripleSum2();
+                    held = 0;
+                }
             }
-        double t = s.value();
+            TripleSum both = s.half(0);
+            both.merge(s.half(1));
+            t += both.value();
+        }
         if (!safe) {
             t = 0.0;
             for (long long e = a; e < b; ++e) t += (double)val[e] * (double)val[e];
@@ -1006,8 +1103,10 @@ int launch_jacobi(const DevCsr& A, float* dinv, cudaStream_t st) {
     return ST_OK;
 }
 int launch_normal_jacobi(const DevCsr& AT, double lam, float* dinv, cudaStream_t st) {
-    if (AT.nnz >= 24 * AT.rows)
-        normal_jacobi_kernel<<<blocks_for(AT.rows * 32) / 2 + 1, 256, 0, st>>>(AT.row_ptr, AT.val, AT.rows, lam, dinv);
+    if (AT.nnz >= 480 * AT.rows)
+        normal_jacobi_kernel<32><<<cg_blocks(AT.rows * 32), 256, 0, st>>>(AT.row_ptr, AT.val, AT.rows, lam, dinv);
+    else if (AT.nnz >= 24 * AT.rows)
+        normal_jacobi_kernel<8><<<cg_blocks(AT.rows * 8), 256, 0, st>>>(AT.row_ptr, AT.val, AT.rows, lam, dinv);
     else
         normal_jacobi_rows_kernel<<<blocks_for(AT.rows), NJ_ROWS, 0, st>>>(AT.row_ptr, AT.val, AT.rows, lam, dinv);
     count_launch();
