@@ -480,6 +480,41 @@ __global__ void pc_combine_kernel(const float* __restrict__ y, const float* __re
         z[i] = fmaf(inv * sqrtf(dinv[i]), y[i], dinv[i] * r[i]);
 }
 
+// The same with a block of one tap: every row is unpacked 27 times, but 27 times the
+// blocks share a small volume. 8^3 4.1 us (6.2 by rows), 16^3 6.2 (10.2).
+__global__ void out_conv_wgrad_tap_kernel(const float* __restrict__ dz, const __nv_bfloat16* __restrict__ h, Vol v,
+                                      float* __restrict__ dw) {
+    const int tap = blockIdx.y;
+    const int W2 = v.nz + 2, P2 = (v.ny + 2) * W2;
+    const long long shift = (long long)(tap / 9 - 1) * P2 + ((tap / 3) % 3 - 1) * W2 + (tap % 3 - 1);
+    float acc[CH];
+#pragma unroll
+    for (int c = 0; c < CH; ++c) acc[c] = 0.0f;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < v.n(); i += (long long)gridDim.x * blockDim.x) {
+        int x, y, z;
+        decode(i, v, x, y, z);
+        const float g = dz[i];
+        float f[CH];
+        load_row32(h + (v.pad_row(x, y, z) + shift) * CH, f);
+#pragma unroll
+        for (int c = 0; c < CH; ++c) acc[c] = fmaf(g, f[c], acc[c]);
+    }
+    __shared__ float red[CH][8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int c = 0; c < CH; ++c) {
+        float t = acc[c];
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane == 0) red[c][warp] = t;
+    }
+    __syncthreads();
+    if (threadIdx.x < CH) {
+        float t = 0.0f;
+        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[threadIdx.x][w];
+        atomicAdd(&dw[threadIdx.x * NTAP + tap], t);
+    }
+}
+
 // CTAs of four warps, a warp per group of bx x by x 8 voxels, all at once up to 16 per SM.
 unsigned grid_groups(const Vol& v, int bx, int by) {
     const long long g = (long long)((v.nz + 7) / 8) * ((v.ny + by - 1) / by) * ((v.nx + bx - 1) / bx);
@@ -494,6 +529,16 @@ dim3 wgrad_grid(const Vol& v) {
 
 unsigned grid_for(long long n, int cap = 152 * 16) {
     return (unsigned)std::max<long long>(1, std::min<long long>((n + 255) / 256, cap));
+}
+
+int launch_out_wgrad(const float* dz, const void* h, const Vol& v, float* dw, cudaStream_t st) {
+    const auto* hb = static_cast<const __nv_bfloat16*>(h);
+    // 16^3 6.2 us by taps, 10.2 by rows; 18^3 8.2 both; 22^3 12.3, 10.2
+    if (v.n() <= 5000) out_conv_wgrad_tap_kernel<<<dim3(grid_for(v.n(), 64), NTAP), 256, 0, st>>>(dz, hb, v, dw);
+    else out_conv_wgrad_kernel<<<wgrad_grid(v), OW_WARPS * 32, 0, st>>>(dz, hb, v, dw);
+    count_launch();
+    ST_CUDA(cudaGetLastError());
+    return ST_OK;
 }
 
 }  // namespace
@@ -543,10 +588,8 @@ int st_pc_out_conv_bwd(const float* dzhat, const void* h, const float* w, void* 
     cudaStream_t st = (cudaStream_t)stream;
     out_conv_dgrad_kernel<<<grid_groups(v, OD_X, OD_Y), 128, 0, st>>>(dzhat, w, v, static_cast<__nv_bfloat16*>(dh));
     count_launch();
-    out_conv_wgrad_kernel<<<wgrad_grid(v), OW_WARPS * 32, 0, st>>>(dzhat, static_cast<const __nv_bfloat16*>(h), v, dw);
-    count_launch();
     ST_CUDA(cudaGetLastError());
-    return ST_OK;
+    return launch_out_wgrad(dzhat, h, v, dw, st);
 }
 
 int st_pc_relu_mask(const void* dh, const void* h, void* g, int64_t nx, int64_t ny, int64_t nz, void* stream) {
@@ -602,10 +645,7 @@ int st_pc_tconv1(const float* a, const float* w, void* h, int64_t nx, int64_t ny
 int st_pc_conv1_wgrad(const float* dz, const void* h, float* dw, int64_t nx, int64_t ny, int64_t nz, void* stream) {
     ST_CHECK(dz && h && dw, ST_ERR_ARG, "null argument");
     const Vol v{(int)nx, (int)ny, (int)nz};
-    out_conv_wgrad_kernel<<<wgrad_grid(v), OW_WARPS * 32, 0, (cudaStream_t)stream>>>(dz, static_cast<const __nv_bfloat16*>(h), v, dw);
-    count_launch();
-    ST_CUDA(cudaGetLastError());
-    return ST_OK;
+    return launch_out_wgrad(dz, h, v, dw, (cudaStream_t)stream);
 }
 
 }  // extern "C"
