@@ -553,10 +553,15 @@ __global__ void __launch_bounds__(RES_THREADS, 1) resident_shot_kernel(const __g
 // receives its halo rows. Measured per step, K = 1 / 2 / 4 / 8 (x: does not fit):
 // 24^3 1.43 / 1.53 / 2.11 / 3.45 us, 48 x 40 x 56 1.61 / 1.62 / 2.14 / 5.07,
 // 64^3 2.05 / 1.73 / 1.80 / 3.63, 100^3 x / x / 2.52 / 3.54, 112^3 x / x / x / 3.88
-// (5.97 by launches of two steps).
+// (5.97 by launches of two steps). Where even that K receives its halo rows in four
+// rounds or more, launches of two steps are the faster ones: us per step resident / by
+// launches, three rounds 40 x 40 x 500 3.9 / 4.2, 36 x 36 x 500 3.9 / 4.1; four 25 x 25 x
+// 700 4.2 / 3.5, 16 x 16 x 1500 4.2 / 3.4, 60 x 60 x 400 5.9 / 5.8, 70 x 70 x 250 5.3 / 5.5;
+// six 50 x 50 x 500 6.9 / 6.0; eight 20 x 20 x 1300 6.3 / 4.0.
 ResPlan plan_resident(const Layout& L, int nsm) {
     ResPlan best;
     double best_cost = 0.0;
+    long long best_rounds = 0;
     const long long nz4 = (L.nz + 3) / 4;
     for (int K : {1, 2, 4, 8}) {
         const long long px = (L.nx + K - 1) / K;
@@ -567,9 +572,11 @@ ResPlan plan_resident(const Layout& L, int nsm) {
         const long long T = (rows * nz4 + 31) / 32 * 32;
         const long long smem = (2 * K * (rows + 2) * nz4 + (res_c_reg(K) ? 2 : K + 2) * T) * 16 + K * 4;
         if (smem > RES_SMEM) continue;
-        const double cost = 0.8 * (double)(K * T) + 4.0 * (double)(T + K * nz4) + 600.0 * (double)((2 * K * nz4 - 1) / T);
+        const long long rounds = (2 * K * nz4 + T - 1) / T;
+        const double cost = 0.8 * (double)(K * T) + 4.0 * (double)(T + K * nz4) + 600.0 * (double)(rounds - 1);
         if (best.K && cost >= best_cost) continue;
         best_cost = cost;
+        best_rounds = rounds;
         best.K = K;
         best.px = (int)px;
         best.py = (int)py;
@@ -579,6 +586,7 @@ ResPlan plan_resident(const Layout& L, int nsm) {
         best.smem = (size_t)smem;
         best.bytes = RES_HEAD + (size_t)(px * py) * 2 * 64 * (size_t)(T + K * nz4);
     }
+    if (best_rounds > 3) best.K = 0;
     return best;
 }
 
