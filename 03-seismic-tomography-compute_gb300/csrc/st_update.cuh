@@ -14,10 +14,15 @@ __device__ __forceinline__ void f4_to(const float4& v, float a[4]) {
     a[3] = v.w;
 }
 
-// The update of one point: out = 2u - upd + c * L u, upd = D * prev.
+// The update of one point: out = 2u - upd + c * L u, upd = D * prev. Every operation is
+// written out, so that no context or compiler setting contracts it otherwise than update2:
+// points of one launch that two blocks form, and the launches of one step, two steps and
+// all steps, agree bit for bit.
 __device__ __forceinline__ float update_fast(float u, float upd, float xm, float xp, float ym, float yp, float zm,
                                              float zp, float c, float ax, float ay, float az) {
-    const float lap = fmaf(-2.0f, u, xp + xm) * ax + fmaf(-2.0f, u, yp + ym) * ay + fmaf(-2.0f, u, zp + zm) * az;
+    const float lx = fmaf(-2.0f, u, __fadd_rn(xp, xm)), ly = fmaf(-2.0f, u, __fadd_rn(yp, ym)),
+                lz = fmaf(-2.0f, u, __fadd_rn(zp, zm));
+    const float lap = fmaf(lz, az, fmaf(lx, ax, __fmul_rn(ly, ay)));
     return fmaf(c, lap, fmaf(2.0f, u, -upd));
 }
 
@@ -93,8 +98,7 @@ __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
     return r;
 }
-// update_fast of two points, with the contractions the compiler makes of it:
-// lap = fma(lz, az, fma(lx, ax, ly * ay)); nD = -D.
+// update_fast of two points; nD = -D.
 __device__ __forceinline__ F2 update2(F2 u, F2 nD, F2 pv, F2 xs, F2 ys, F2 zs, F2 c, float ax, float ay, float az) {
     const F2 m2 = pack(-2.0f, -2.0f), p2 = pack(2.0f, 2.0f);
     const F2 lx = fma2(m2, u, xs), ly = fma2(m2, u, ys), lz = fma2(m2, u, zs);
