@@ -33,6 +33,7 @@
 #include <algorithm>
 #include <cmath>
 #include <memory>
+#include <mutex>
 
 struct st_ray_picks {
     int device = 0;
@@ -48,6 +49,9 @@ struct st_ray_picks {
     int* t_pick = nullptr;        // [n_samples] pick of each sample, cell-major
     int* pick_order = nullptr;    // [n_picks] picks by descending sample count
     int* cell_order = nullptr;    // [n_cells] cells by descending sample count
+    // table to stage_out belong to the call that holds busy: its launches follow one
+    // another on the stream, so calls from several threads don't see each other's values
+    std::mutex busy;
     double2* table = nullptr;     // [n_cells] (velocity used, its reciprocal or 0) of the current call
     double* trial_times = nullptr;  // line-search trials: [n_picks], on first use
     double* partial = nullptr;      // and the misfit's partial sums
@@ -584,6 +588,7 @@ int st_ray_picks_stream(st_ray_picks* p, void** out) {
 int st_ray_picks_forward_model(st_ray_picks* p, const double* vp, int on_device, double* times) {
     ST_CHECK(p && vp && (times || p->n_picks == 0), ST_ERR_ARG, "null argument");
     ST_CUDA(cudaSetDevice(p->device));
+    std::lock_guard<std::mutex> lock(p->busy);
     cudaStream_t st = p->stream;
     const double* dvp = vp;
     double* dt = times;
@@ -612,6 +617,7 @@ int st_ray_picks_compute_gradient(st_ray_picks* p, const double* vp, const doubl
                                   double* gradient) {
     ST_CHECK(p && vp && gradient && (residuals || p->n_picks == 0), ST_ERR_ARG, "null argument");
     ST_CUDA(cudaSetDevice(p->device));
+    std::lock_guard<std::mutex> lock(p->busy);
     cudaStream_t st = p->stream;
     const double* dvp = vp;
     const double* dres = residuals;
@@ -661,6 +667,7 @@ int st_ray_picks_misfit(st_ray_picks* p, const double* times, const double* obs,
                         double* misfit) {
     ST_CHECK(p && misfit && (p->n_picks == 0 || (times && obs && weight)), ST_ERR_ARG, "null argument");
     ST_CUDA(cudaSetDevice(p->device));
+    std::lock_guard<std::mutex> lock(p->busy);
     ST_TRY(ensure_misfit(p, false));
     return misfit_of(p, times, obs, weight, l1, misfit);
 }
@@ -670,6 +677,7 @@ int st_ray_picks_trial_misfit(st_ray_picks* p, const double* vp, const double* g
                               const double* weight, int l1, double* misfit) {
     ST_CHECK(p && vp && gradient && misfit && (p->n_picks == 0 || (obs && weight)), ST_ERR_ARG, "null argument");
     ST_CUDA(cudaSetDevice(p->device));
+    std::lock_guard<std::mutex> lock(p->busy);
     ST_TRY(ensure_misfit(p, true));
     const TrialClamp C{vp_min, vp_max, policy_range ? policy_range[0] : 0.0, policy_range ? policy_range[1] : 0.0,
                        policy_range != nullptr};
