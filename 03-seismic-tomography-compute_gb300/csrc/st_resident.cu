@@ -111,13 +111,13 @@ struct Pending {
     }
     // Waits for the group of tag; false when the limit ran out or another block
     // gave up.
-    __device__ __forceinline__ bool wait(unsigned tag, const unsigned* abort_word) {
+    __device__ __forceinline__ bool wait(unsigned tag, const unsigned* abort_word, uint64_t limit) {
         uint64_t t0 = 0;
         for (int i = 0; !ready(tag); ++i) {
             if (i == 256) {
                 const uint64_t now = now_ns();
                 if (t0 == 0) t0 = now;
-                if (now - t0 > RES_WAIT_NS || load_relaxed(abort_word)) return false;
+                if (now - t0 > limit || load_relaxed(abort_word)) return false;
                 i = 0;
             }
             issue();
@@ -303,6 +303,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) resident_shot_kernel(const __g
 
     // all blocks run from here on
     bool ok = true;
+    const bool lost = a.withhold < 0 && blockIdx.x == 0;  // the wait test: this block leaves after u_0
     if (tid == 0) {
         atomicAdd(arrived, 1u);
         const uint64_t t0 = now_ns();
@@ -312,6 +313,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) resident_shot_kernel(const __g
                 break;
             }
         }
+        if (lost) ok = false;
     }
 
     // the faces of u_t, t the parity of the buffers
@@ -323,12 +325,12 @@ __global__ void __launch_bounds__(RES_THREADS, 1) resident_shot_kernel(const __g
         if (tid < nyg) g.issue();
         float v[4];
         if (send_xlo) {
-            ok = l.wait(tag, abort_word) && ok;
+            ok = l.wait(tag, abort_word, a.timeout_ns) && ok;
             l.get(v);
             st4(Xlo, v);
         }
         if (send_xhi) {
-            ok = h.wait(tag, abort_word) && ok;
+            ok = h.wait(tag, abort_word, a.timeout_ns) && ok;
             h.get(v);
             st4(Xhi, v);
         }
@@ -340,7 +342,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) resident_shot_kernel(const __g
                 g.p = in + src;
                 g.issue();
             }
-            ok = g.wait(tag, abort_word) && ok;
+            ok = g.wait(tag, abort_word, a.timeout_ns) && ok;
             g.get(v);
             st4(S + dst, v);
         }
@@ -525,7 +527,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) resident_shot_kernel(const __g
     }
     for (int t = 0; t < r.nt && !dead; ++t) dead = step(t, t & 1 ? S1 : S0, t & 1 ? S0 : S1);
     if (dead) {
-        if (tid == 0) {
+        if (tid == 0 && !lost) {
             atomicExch(abort_word, 1u);
             atomicOr(a.flags, FLAG_TIMEOUT);
         }
@@ -641,6 +643,7 @@ int resident_shot(st_solver* s, const StepArgs& a, const st_shot* shot, float* s
     r.a.nz = (int)L.nz;
     r.a.NZP = (int)L.NZP;
     r.a.plane = L.plane;
+    if (r.a.timeout_ns == 0) r.a.timeout_ns = RES_WAIT_NS;
     r.c = s->c;
     r.cur = s->f[s->ic];
     r.prev = s->f[s->ip];

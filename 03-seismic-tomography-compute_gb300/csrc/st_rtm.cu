@@ -116,9 +116,9 @@ int shot_forward_impl(st_solver* s, const st_shot* shot, float* seis, int snap_k
     if (snap_kind != SNAP_NONE) ST_CUDA(cudaMemsetAsync(amax, 0, sizeof(unsigned) * (size_t)(nt + 1), s->stream));
     // a small grid without snapshots: every step in one launch. The switches of
     // the chunked path (one step per launch, the wait limit and its test, a
-    // fixed chunking) select that path.
+    // fixed chunking) select that path, and the resident wait test this one.
     if (nt >= RES_MIN_STEPS && snap_kind == SNAP_NONE && s->fused_steps == 2 && !s->zlim && !(slices && s->slices) &&
-        !s->withhold && !s->wait_limit_ns && !std::getenv("SEISMIC_GB300_XCHUNKS")) {
+        (s->withhold < 0 || (!s->withhold && !s->wait_limit_ns)) && !std::getenv("SEISMIC_GB300_XCHUNKS")) {
         StepArgs a = base_args(s, nullptr);
         set_injection(a, shot->src_ix, shot->src_iy, shot->src_iz, 0.0f);
         if (nrec > 0 && seis) set_receivers(a, R);

@@ -843,9 +843,9 @@ int st_solver_set_stream(st_solver* s, void* stream) {
 }
 
 int st_solver_set_wait_test(st_solver* s, unsigned long long limit_ns, int withhold_plane) {
-    ST_CHECK(s && withhold_plane >= -1, ST_ERR_ARG, "bad argument");
+    ST_CHECK(s && withhold_plane >= -2, ST_ERR_ARG, "bad argument");
     s->wait_limit_ns = limit_ns;
-    s->withhold = withhold_plane + 1;
+    s->withhold = withhold_plane + 1;  // -1: the resident shot's test
     return ST_OK;
 }
 

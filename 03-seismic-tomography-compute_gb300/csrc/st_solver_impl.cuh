@@ -99,7 +99,7 @@ struct st_solver {
     unsigned res_tag = 1;           // first tag of the next resident launch
     int sponge_mode = ST_SPONGE_REFERENCE;  // ST_SPONGE_STABLE: damp the new field (Cerjan form)
     unsigned long long wait_limit_ns = 0;   // bounded-wait limit of the stencil kernels (0: 2 s)
-    int withhold = 0;                       // st_solver_set_wait_test: plane + 1 withheld at the next launch
+    int withhold = 0;                       // st_solver_set_wait_test: plane + 1 withheld at the next launch (-1: resident test)
     int* zlim = nullptr;                // terrain: per-column z limits (st_solver_set_terrain), or null
     st_slice_stream* slices = nullptr;  // RTM slice stream (configure_rtm), borrowed
     int slice_interval = 0;             // capture every slice_interval steps

@@ -180,7 +180,9 @@ enum st_fault_param { ST_FT_MAX_REPAIR_ATTEMPTS = 0, ST_FT_AMPLITUDE_LIMIT = 1, 
  * launch drains its other copies (always with the full 2 s limit) and exits,
  * and the call returns ST_ERR_TIMEOUT with the handle still usable (its field
  * values are then undefined until reset_field). The withheld plane applies to
- * one launch; the limit stays until changed. */
+ * one launch; the limit stays until changed. withhold_plane = -2: the same for
+ * the next shot that keeps its grid on the SMs; its first block leaves
+ * before the first step, so the waits of the other blocks run out. -1: no test. */
 int st_solver_set_wait_test(st_solver* s, unsigned long long limit_ns, int withhold_plane);
 int st_solver_reset_fault_stats(st_solver* s);
 int st_solver_set_fault_param(st_solver* s, int which, double value);
