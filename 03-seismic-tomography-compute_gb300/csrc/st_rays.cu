@@ -362,7 +362,7 @@ static int build_walk_once(long long nrays, const double* d_ends, const RayGrid&
     auto* off = static_cast<long long*>(bufs.get((size_t)(tiles + 1) * 8));
     auto* count = static_cast<long long*>(bufs.get((size_t)nrays * 8));
     auto* down = static_cast<unsigned char*>(bufs.get((size_t)nrays));
-    auto* info = static_cast<int*>(bufs.get(64));  // tallest, overrun
+    auto* info = static_cast<int*>(bufs.get(64));  // tallest, overrun; from 16 bytes on the rows' measure
     void* stmp = bufs.get(scan_tmp_bytes(nrays));
     if (!height || !off || !count || !down || !info || !stmp) return ST_OK;
     auto allocate = [&](auto** p, size_t n) {
@@ -415,7 +415,10 @@ static int build_walk_once(long long nrays, const double* d_ends, const RayGrid&
         nrays, G, tallest, off, scol, sval, down, out->row_ptr, out->col, out->val);
     count_launch();
     ST_CUDA(cudaGetLastError());
+    UnevenRows u;
+    ST_TRY(measure_rows(*out, info + 4, &u, st));
     ST_CUDA(cudaStreamSynchronize(st));
+    out->lanes = lanes_of(*out, u);
     *done = true;
     return ST_OK;
 }

@@ -315,7 +315,7 @@ __device__ __forceinline__ void copy16_async(void* dst, const void* src, int byt
 // columns and the gathers one after another for 28 bytes of values. A tile with
 // more entries than fit in shared memory is summed a warp per row; matrices with much
 // of their entries in such tiles, or in tiles with a long row that one thread works
-// through, go to a group of lanes per row (find_uneven_rows).
+// through, go to a group of lanes per row (lanes_of).
 // 7 entries per row on a 256^3 grid, 72 bytes per row: 199 us a product (a copy of
 // the bytes takes 178); products along the stream 244, four lanes per row 600. 40
 // CG iterations there with tiles of 256 / 128 / 64 rows 24.3 / 23.5 / 23.3 ms
@@ -1006,7 +1006,10 @@ int build_csr(long long rows, long long cols, long long n, const TI* r, const TI
             out->nnz = pn;
         }
     }
+    UnevenRows u;
+    ST_TRY(measure_rows(*out, total, &u, st));
     ST_CUDA(cudaStreamSynchronize(st));
+    out->lanes = lanes_of(*out, u);
     return ST_OK;
 }
 
@@ -1015,9 +1018,7 @@ template int build_csr<long long, double>(long long, long long, long long, const
 template int build_csr<int, float>(long long, long long, long long, const int*, const int*, const float*, bool,
                                    DevCsr*, cudaStream_t);
 
-// What spmv_rows_kernel is slow on, a warp per tile: out[0] the entries in tiles
-// beyond shared memory or with a long row, out[1] the longest row, out[2] the
-// entries of the heaviest tile.
+// What spmv_rows_kernel is slow on (UnevenRows), a warp per tile.
 __global__ void uneven_tiles_kernel(const long long* __restrict__ rp, long long rows, unsigned long long* out) {
     const int lane = threadIdx.x & 31;
     unsigned long long entries = 0, longest = 0, heaviest = 0;
@@ -1045,21 +1046,23 @@ __global__ void uneven_tiles_kernel(const long long* __restrict__ rp, long long 
 // and a half of none 56 / 33; 1 row of 128 at 600, the others 3, 149 / 82; a power law
 // of mean 6.2 up to 2000 sorted by length 552 / 57, in random order 106 / 82; 1 row of
 // 1000 at 4000 101 / 120 (four lanes 149); 1000 rows, one of 5000, 61 / 53.
-int find_uneven_rows(DevCsr* A, void* scratch, cudaStream_t st) {
-    A->lanes = 0;
-    if (A->rows == 0 || A->nnz >= SHORT_ROWS * A->rows) return ST_OK;
+int measure_rows(const DevCsr& A, void* scratch, UnevenRows* u, cudaStream_t st) {
+    if (u) *u = UnevenRows();
+    // a small matrix is built in less time than a few products save (the measure takes 16 us)
+    if (A.nnz < 4096 || A.nnz >= SHORT_ROWS * A.rows) return ST_OK;
     auto* acc = static_cast<unsigned long long*>(scratch);
-    unsigned long long h[3] = {0, 0, 0};
-    ST_CUDA(cudaMemsetAsync(acc, 0, sizeof(h), st));
-    uneven_tiles_kernel<<<blocks_for((A->rows + SR_ROWS - 1) / SR_ROWS * 32), 256, 0, st>>>(A->row_ptr, A->rows, acc);
+    if (u) ST_CUDA(cudaMemsetAsync(acc, 0, sizeof(UnevenRows), st));
+    uneven_tiles_kernel<<<blocks_for((A.rows + SR_ROWS - 1) / SR_ROWS * 32), 256, 0, st>>>(A.row_ptr, A.rows, acc);
     count_launch();
     ST_CUDA(cudaGetLastError());
-    ST_CUDA(cudaMemcpyAsync(h, acc, sizeof(h), cudaMemcpyDeviceToHost, st));
-    ST_CUDA(cudaStreamSynchronize(st));
-    if (8 * h[0] <= (unsigned long long)A->nnz) return ST_OK;
-    if (h[1] <= 1024) A->lanes = A->nnz >= 5 * A->rows ? 4 : 2;
-    else if (h[2] > 8192 || 16 * h[0] > 15 * (unsigned long long)A->nnz) A->lanes = 8;
+    if (u) ST_CUDA(cudaMemcpyAsync(u, acc, sizeof(UnevenRows), cudaMemcpyDeviceToHost, st));
     return ST_OK;
+}
+
+int lanes_of(const DevCsr& A, const UnevenRows& u) {
+    if (8 * u.entries <= (unsigned long long)A.nnz) return 0;
+    if (u.longest <= 1024) return A.nnz >= 5 * A.rows ? 4 : 2;
+    return u.heaviest > 8192 || 16 * u.entries > 15 * (unsigned long long)A.nnz ? 8 : 0;
 }
 
 int launch_spmv(const DevCsr& A, const float* x, float* y, const float* add, float add_scale, const float* pdot,

@@ -13,7 +13,7 @@ struct DevCsr {
     long long* row_ptr = nullptr;
     int* col = nullptr;
     float* val = nullptr;
-    int lanes = 0;  // lanes per row of products with uneven short rows, 0: even ones (find_uneven_rows)
+    int lanes = 0;  // lanes per row of products with uneven short rows, 0: even ones (lanes_of)
     void release() {
         cudaFree(row_ptr);
         cudaFree(col);
@@ -110,8 +110,16 @@ template <class TI, class TV>
 int build_csr(long long rows, long long cols, long long n, const TI* r, const TI* c, const TV* v, bool pad,
               DevCsr* out, cudaStream_t st);
 int build_transpose(const DevCsr& A, DevCsr* T, cudaStream_t st);
-// Sets A->lanes from the row pointers; scratch: 24 bytes on the device. Waits for the stream.
-int find_uneven_rows(DevCsr* A, void* scratch, cudaStream_t st);
+// Entries of a short-row matrix in 128-row tiles beyond shared memory or with a long
+// row, the longest row, and the entries of the heaviest tile (0 where the rows are not
+// short). The builders read it with their last copies (scratch: its size on the device,
+// zero already where u is null; *u, or scratch, holds it once the stream has been
+// waited for) and set DevCsr::lanes.
+struct UnevenRows {
+    unsigned long long entries = 0, longest = 0, heaviest = 0;
+};
+int measure_rows(const DevCsr& A, void* scratch, UnevenRows* u, cudaStream_t st);
+int lanes_of(const DevCsr& A, const UnevenRows& u);
 // Straight-ray path-length matrix (st_rays.cu): d_ends = device [nrays][6]
 // endpoints in cell units; total_nnz (may be null) receives the entry count.
 int build_ray_csr(long long nrays, const double* d_ends, int nx, int ny, int nz, double h, DevCsr* out,

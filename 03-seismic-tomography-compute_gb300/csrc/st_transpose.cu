@@ -212,6 +212,10 @@ int build_transpose(const DevCsr& A, DevCsr* T, cudaStream_t st) {
     out.rows = A.cols;
     out.cols = A.rows;
     out.nnz = n;
+    struct Checks {
+        int irregular = 0;
+        UnevenRows rows;
+    };
     int irregular = 0;
     auto expand = [&](int* rowidx) -> int {
         if (n >= 12 * A.rows) tr_rows_kernel<32><<<tr_blocks(A.rows * 32), 256, 0, st>>>(A.row_ptr, A.rows, rowidx);
@@ -243,12 +247,12 @@ int build_transpose(const DevCsr& A, DevCsr* T, cudaStream_t st) {
         const long long hn = (long long)bins * grid;
         DeviceBuffers bufs;
         auto* rowidx = static_cast<int*>(bufs.get((size_t)n * 4));  // the rows, then the last pass's keys
-        auto* hist = static_cast<long long*>(bufs.get((size_t)hn * 8 + sizeof(int)));  // the irregular word behind it
+        auto* hist = static_cast<long long*>(bufs.get((size_t)hn * 8 + sizeof(Checks)));  // the checks behind it
         auto* offs = static_cast<long long*>(bufs.get((size_t)hn * 8));
         void* stmp = bufs.get(scan_tmp_bytes(hn));
         if (!rowidx || !hist || !offs || !stmp) return bufs.fail();
-        int* flag = reinterpret_cast<int*>(hist + hn);
-        ST_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), st));
+        auto* found = reinterpret_cast<Checks*>(hist + hn);
+        ST_CUDA(cudaMemsetAsync(found, 0, sizeof(Checks), st));
         int* bk[2] = {nullptr, nullptr};
         int* br[2] = {nullptr, nullptr};
         float* bv[2] = {nullptr, nullptr};
@@ -284,11 +288,15 @@ int build_transpose(const DevCsr& A, DevCsr* T, cudaStream_t st) {
             ir = orw;
             iv = ov;
         }
-        tr_rowptr_kernel<<<tr_blocks(n), 256, 0, st>>>(keys, out.col, n, A.cols, out.row_ptr, flag);
+        tr_rowptr_kernel<<<tr_blocks(n), 256, 0, st>>>(keys, out.col, n, A.cols, out.row_ptr, &found->irregular);
         count_launch();
         ST_CUDA(cudaGetLastError());
-        ST_CUDA(cudaMemcpyAsync(&irregular, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
+        ST_TRY(measure_rows(out, &found->rows, nullptr, st));
+        Checks h;
+        ST_CUDA(cudaMemcpyAsync(&h, found, sizeof(h), cudaMemcpyDeviceToHost, st));
         ST_CUDA(cudaStreamSynchronize(st));
+        irregular = h.irregular;
+        out.lanes = lanes_of(out, h.rows);
         return ST_OK;
     };
     auto build_sorted = [&]() -> int {

@@ -19,8 +19,9 @@ def _lengths(kind):
         "half": np.where(i < ROWS // 2, 0, 18),                  # four lanes
         "half thin": np.where(i < ROWS // 4, 13, 1),             # two lanes
         "one of 128": np.where(i % 128 == 7, 600, 3),            # four lanes
-        "last row": np.where(i == ROWS - 1, 1024, 2),            # two lanes, the longest they take
-        "a long row": np.where(i == 3, 1025, 2),                 # row tiles
+        "last row": np.where(i == ROWS - 1, 1024, 3),            # two lanes, the longest they take
+        "a long row": np.where(i == 3, 1025, 3),                 # row tiles
+        "few": np.where(i == 5, 1000, 2),                        # row tiles: fewer than 4,096 entries
         "long rows": np.where(i < 8, 1100, 3),                   # eight lanes: one tile of 9,160 entries
         "sorted": np.sort(np.random.default_rng(2).zipf(1.7, ROWS).clip(0, 3000))[::-1],
     }[kind].astype(np.int64)
@@ -34,7 +35,7 @@ def _product(A, x, rows, transpose=False):
     return y.cpu().numpy()
 
 
-@pytest.mark.parametrize("kind", ["half", "half thin", "one of 128", "last row", "a long row", "long rows", "sorted"])
+@pytest.mark.parametrize("kind", ["half", "half thin", "one of 128", "last row", "a long row", "few", "long rows", "sorted"])
 def test_uneven_rows(kind):
     rng = np.random.default_rng(1)
     m = _lengths(kind)
