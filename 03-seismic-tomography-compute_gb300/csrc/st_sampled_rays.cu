@@ -19,9 +19,10 @@
 // rounded division per sample); threads take picks and cells in order of
 // their sample counts, so the lanes of a warp run loops of similar length
 // and the FP64 pipe is not spent on masked-off lanes. The divisor belongs to
-// the cell (v, or v * v), so its reciprocal is formed once per cell and call and
-// the sample's quotient takes five operations (quotient_of, correctly rounded)
-// where the division takes about ten; values out of its range are divided. All
+// the cell (v, or v * v), so where there are samples enough its reciprocal is
+// formed once per cell and call, and the sample's quotient takes five operations
+// (quotient_of, correctly rounded) where the division takes about ten; values
+// out of its range are divided. All
 // FP64 arithmetic is written with explicitly rounded intrinsics (no contraction
 // into FMA), so each value is the reference's expression evaluated in IEEE
 // double: the results match it bit for bit given the same source-station
@@ -240,24 +241,31 @@ __device__ __forceinline__ double sample_time(double d, double2 e, bool fast) {
 // _forward_model (inversion.py:329-381), one thread per pick, the samples
 // added in order. The loads and quotients of four samples are issued
 // together (they are independent); only the additions keep the reference's
-// order.
+// order. TABLE: velocities and reciprocals from the table, else from vp by division
+// (the same bits).
+template <bool TABLE>
 __global__ void ray_forward_kernel(long long np, const int* __restrict__ order, const long long* __restrict__ off,
                                    const int* __restrict__ cell, const double* __restrict__ ds,
                                    const double* __restrict__ dist, const double2* __restrict__ table,
-                                   double* __restrict__ times) {
+                                   const double* __restrict__ vp, double* __restrict__ times) {
+    auto entry = [&](int c) {
+        if (TABLE) return __ldg(table + c);
+        const double v = __ldg(vp + c);
+        return make_double2(valid_velocity(v) ? v : 1500.0, 0.0);
+    };
     for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < np;
          j += (long long)gridDim.x * blockDim.x) {
         const long long i = order[j];
         const long long b = off[i], e = off[i + 1];
         const double d = ds[i];
-        const bool fast = moderate(d) || d == 0.0;
+        const bool fast = TABLE && (moderate(d) || d == 0.0);
         double t = 0.0;
         long long k = b;
         for (; k + 4 <= e; k += 4) {
             double2 v[4];
             double term[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) v[j] = __ldg(table + __ldg(cell + k + j));
+            for (int j = 0; j < 4; ++j) v[j] = entry(__ldg(cell + k + j));
 #pragma unroll
             for (int j = 0; j < 4; ++j) term[j] = sample_time(d, v[j], fast);
 #pragma unroll
@@ -265,7 +273,7 @@ __global__ void ray_forward_kernel(long long np, const int* __restrict__ order, 
                 if (finite_bits(term[j])) t = __dadd_rn(t, term[j]);
         }
         for (; k < e; ++k) {
-            const double term = sample_time(d, __ldg(table + __ldg(cell + k)), fast);
+            const double term = sample_time(d, entry(__ldg(cell + k)), fast);
             if (finite_bits(term)) t = __dadd_rn(t, term);
         }
         if (b < e && (!finite_bits(t) || t < 0.0)) t = __ddiv_rn(dist[i], 6000.0);
@@ -598,10 +606,18 @@ int st_ray_picks_forward_model(st_ray_picks* p, const double* vp, int on_device,
         dt = p->stage_out;
     }
     if (p->n_picks > 0) {
-        table_kernel<<<blocks_for(p->n_cells, 256), 256, 0, st>>>(dvp, p->n_cells, p->table);
-        count_launch();
-        ray_forward_kernel<<<blocks_for(p->n_picks, 128), 128, 0, st>>>(p->n_picks, p->pick_order, p->off, p->cell,
-                                                                        p->ds, p->dist, p->table, dt);
+        // The table takes a launch and 11 us per 10^6 cells, and saves 5 us per 10^6 samples.
+        // By table / by division, us: 125,000 cells, 31,000 samples 15.4 / 12.3, 610,000 22.5 /
+        // 22.5, 1.2M 27.7 / 32.8; 10^6 cells, 130,000 32 / 20, 2.0M 55 / 55, 6.4M 102 / 122;
+        // 4.1M cells, 6.2M 141 / 121.
+        const bool table = p->n_samples > 400000 + 9 * p->n_cells / 4;
+        if (table) {
+            table_kernel<<<blocks_for(p->n_cells, 256), 256, 0, st>>>(dvp, p->n_cells, p->table);
+            count_launch();
+        }
+        auto kernel = table ? ray_forward_kernel<true> : ray_forward_kernel<false>;
+        kernel<<<blocks_for(p->n_picks, 128), 128, 0, st>>>(p->n_picks, p->pick_order, p->off, p->cell, p->ds, p->dist,
+                                                            p->table, dvp, dt);
         count_launch();
         ST_CUDA(cudaGetLastError());
     }
@@ -684,8 +700,8 @@ int st_ray_picks_trial_misfit(st_ray_picks* p, const double* vp, const double* g
     trial_table_kernel<<<blocks_for(p->n_cells, 256), 256, 0, p->stream>>>(vp, gradient, step, C, p->n_cells, p->table);
     count_launch();
     if (p->n_picks > 0) {
-        ray_forward_kernel<<<blocks_for(p->n_picks, 128), 128, 0, p->stream>>>(
-            p->n_picks, p->pick_order, p->off, p->cell, p->ds, p->dist, p->table, p->trial_times);
+        ray_forward_kernel<true><<<blocks_for(p->n_picks, 128), 128, 0, p->stream>>>(
+            p->n_picks, p->pick_order, p->off, p->cell, p->ds, p->dist, p->table, nullptr, p->trial_times);
         count_launch();
     }
     ST_CUDA(cudaGetLastError());
