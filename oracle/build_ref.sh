@@ -23,8 +23,8 @@
 #   3. csr_matrix.cpp:233-234: pad_to_alignment allocates nnz + 8 * rows
 #      entries (an upper bound of the padded total) instead of a size that is
 #      too small whenever padding fires (heap overflow).
-# x86-64 only (the reference includes <x86intrin.h>/<immintrin.h>); the GPU
-# box has no reference sources, so this runs only where they are present.
+# x86-64 only (the reference includes <x86intrin.h>/<immintrin.h>), and only
+# where the reference's sources are present.
 set -euo pipefail
 HERE="$(cd "$(dirname "${BASH_SOURCE[0]}")" && pwd)"
 REF="${SEISMIC_REFERENCE_DIR:-/root/reference}"

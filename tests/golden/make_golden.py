@@ -4,7 +4,7 @@ place by oracle/build_ref.sh into oracle/_ref/libseismic_ref.so) on small
 seeded inputs. The reference sources exist only where this script is run;
 the fixtures it writes are what the tests (and the GPU machine) use.
 
-    python tests/golden/make_golden.py
+    SEISMIC_REFERENCE_DIR=<reference checkout> python tests/golden/make_golden.py
 
 Fixtures (all FP64 reference outputs):
   prop_small.npz     inject_source + step_forward stepping with a source and
@@ -33,7 +33,7 @@ sys.path.insert(0, os.path.join(REPO, "03-seismic-tomography-compute_gb300"))
 from oracle import Reference, build_ref  # noqa: E402
 from seismic_engine import workloads as wl  # noqa: E402
 
-REFERENCE = os.environ.get("SEISMIC_REFERENCE_DIR", "/root/reference")
+REFERENCE = os.environ.get("SEISMIC_REFERENCE_DIR") or sys.exit("set SEISMIC_REFERENCE_DIR to a reference checkout")
 
 
 def prop_case():

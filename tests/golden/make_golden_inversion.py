@@ -6,7 +6,7 @@ model, with the reference's own synthetic OBS data
 gradient model's velocities (VelocityModel.initialize_gradient_model,
 model.py:46-64).
 
-    python tests/golden/make_golden_inversion.py
+    SEISMIC_REFERENCE_DIR=<reference checkout> python tests/golden/make_golden_inversion.py
 
 The driver's compiled-engine calls (check_field_health, repair_field_nan,
 SparseOps.smooth_gradient; inversion.py:10-18, gradient.py:5-9) are served
@@ -27,7 +27,7 @@ import numpy as np
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 REPO = os.path.dirname(os.path.dirname(HERE))
-REFERENCE = os.environ.get("SEISMIC_REFERENCE_DIR", "/root/reference")
+REFERENCE = os.environ.get("SEISMIC_REFERENCE_DIR") or sys.exit("set SEISMIC_REFERENCE_DIR to a reference checkout")
 PKG = os.path.join(REFERENCE, "src", "python", "seismic_tomography")
 sys.path.insert(0, os.path.join(REPO, "oracle"))
 

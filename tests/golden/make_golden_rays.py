@@ -4,7 +4,7 @@ inversion driver (src/python/seismic_tomography of
 straight-ray traveltime forward model and its gradient
 (seismic_tomography/inversion.py:329-433) on a small seeded model.
 
-    python tests/golden/make_golden_rays.py
+    SEISMIC_REFERENCE_DIR=<reference checkout> python tests/golden/make_golden_rays.py
 
 Fixtures: rays_small.npz (the guard case below) and rays_medium.npz (300
 picks between 12 sources and 25 stations over a 40 x 32 x 24 model).
@@ -33,7 +33,7 @@ import types
 import numpy as np
 
 HERE = os.path.dirname(os.path.abspath(__file__))
-REFERENCE = os.environ.get("SEISMIC_REFERENCE_DIR", "/root/reference")
+REFERENCE = os.environ.get("SEISMIC_REFERENCE_DIR") or sys.exit("set SEISMIC_REFERENCE_DIR to a reference checkout")
 PKG = os.path.join(REFERENCE, "src", "python", "seismic_tomography")
 
 
