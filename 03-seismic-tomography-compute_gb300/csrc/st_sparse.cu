@@ -675,43 +675,52 @@ __global__ void jacobi_kernel(const long long* __restrict__ rp, const int* __res
 // per row, over its entries (coalesced); a group's rows lie a grid apart (neighbouring
 // cells are heavy together: where rays meet, a row holds thousands of entries), and
 // lane w keeps the sum of its w-th row, so that the FP64 division runs on full warps.
-// Triples of FP32 values carry the squares, two to an instruction, and rows with a
-// value they cannot hold are summed in FP64. Bound by the FP32 instructions. Eight
+// Triples of FP32 values carry the squares, two to an instruction, and rows whose sum
+// they cannot hold are summed again in FP64. Bound by the FP32 instructions. Eight
 // lanes join a row's sums in three steps for four rows at once; rows beyond NJ_FAR go
-// to the whole warp. 8 / 32 lanes, us: 262,144 rows of 40 entries 31 / 87 (47 a thread
-// per row in FP64), of 202 80 / 128 (214), 131,072 rows of 361 67 / 90 (213); means of
-// 3000 from 2 to 20,000 45 / 21. Triples one at a time, 32 lanes: 117, 146, 101.
+// to the whole warp. 8 / 32 lanes, us: 262,144 rows of 40 entries 33 / 87 (47 a thread
+// per row in FP64), of 202 68 / 128 (214), 131,072 rows of 361 56 / 90 (213); means of
+// 3000 from 2 to 20,000 45 / 17. The cells of 2M rays on 100^3 (361M entries) 0.49 ms,
+// 0.58 with the range tested per entry and every load against the row's end.
 // Short rows (less than 24 entries on average) are staged through shared memory
 // instead, a thread per row: 2M rows of 7 entries 58 us (85 in FP64).
-constexpr int NJ_FAR = 512;  // rows that groups of eight leave to the warp
+constexpr int NJ_FAR = 1024;  // rows that groups of eight leave to the warp
 
-// This lane's squares among [a, b), G lanes over them; full triples go to far.
-// Two sums per instruction, joined at the end. Whether a value does not fit.
+// This lane's squares among p[0 .. n), G lanes over them; full triples go to far. Two
+// sums per instruction, joined at the end.
 template <int G>
-__device__ __forceinline__ unsigned add_squares(const float* __restrict__ val, long long a, long long b, int lane,
-                                                TripleSum& s, double& far) {
-    unsigned odd = 0;
+__device__ __forceinline__ void add_squares(const float* __restrict__ p, long long n, int lane, TripleSum& s,
+                                            double& far) {
     int held = 0;
     TripleSum2 t;
-    for (long long q = a + lane; q - lane < b; q += 8 * G) {
+    p += lane;
+    for (; n - lane > 7 * G; n -= 8 * G, p += 8 * G) {
         float v[8];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) v[k] = q + G * k < b ? __ldg(val + q + G * k) : 0.0f;
+        for (int k = 0; k < 8; ++k) v[k] = __ldg(p + G * k);
 #pragma unroll
-        for (int k = 0; k < 8; k += 2)
-            if (k == 0 || q + G * k < b) {
-                odd |= triple_safe(v[k]) & triple_safe(v[k + 1]) ? 0u : 1u;
-                t.add_squares(pack(v[k], v[k + 1]));
-            }
+        for (int k = 0; k < 8; k += 2) t.add_squares(pack(v[k], v[k + 1]));
         if ((held += 4) == TRIPLE_MAX) {
             far += t.half(0).value() + t.half(1).value();
             t = TripleSum2();
             held = 0;
         }
     }
+    const int m = (int)n - lane;
+    float v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = G * k < m ? __ldg(p + G * k) : 0.0f;
+#pragma unroll
+    for (int k = 0; k < 8; k += 2)
+        if (G * k < m) t.add_squares(pack(v[k], v[k + 1]));
     s = t.half(0);
     s.merge(t.half(1));
-    return odd;
+}
+
+// Whether a sum of squares needs FP64: out of range on the way (infinite or NaN then),
+// or so small that what the triples lose to underflow, 2^-149 a product, may count.
+__device__ __forceinline__ bool squares_odd(float h, double far) {
+    return !(h <= 0x1p120f) || (far == 0.0 ? !(h >= 0x1p-40f) : !(far >= 0x1p-40 && far <= 0x1p200));
 }
 
 template <int G>
@@ -757,8 +766,9 @@ __global__ void __launch_bounds__(256, 4) normal_jacobi_kernel(const long long* 
             const bool rest = G < 32 && b - a > NJ_FAR;
             TripleSum s;
             double far = 0.0;
-            unsigned odd = __ballot_sync(FULL, add_squares<G>(val, a, rest ? a : b, lane, s, far));
+            add_squares<G>(val + a, rest ? 0 : b - a, lane, s, far);
             merge_lanes<G>(s, far);
+            unsigned odd = __ballot_sync(FULL, b > a && !rest && squares_odd(s.h, far));
             if (odd) {
                 const double t = squares64<G>(val, a, rest ? a : b, lane);
                 if ((odd >> (wl - lane)) & (FULL >> (32 - G))) {
@@ -775,8 +785,9 @@ __global__ void __launch_bounds__(256, 4) normal_jacobi_kernel(const long long* 
                     const int src = __ffs((int)m) - 1;
                     const long long fa = __shfl_sync(FULL, a, src), fb = __shfl_sync(FULL, b, src);
                     far = 0.0;
-                    odd = __ballot_sync(FULL, add_squares<32>(val, fa, fb, wl, s, far));
+                    add_squares<32>(val + fa, fb - fa, wl, s, far);
                     merge_lanes<32>(s, far);
+                    odd = __ballot_sync(FULL, squares_odd(s.h, far));
                     if (odd) {
                         s = TripleSum();
                         far = squares64<32>(val, fa, fb, wl);
