@@ -676,15 +676,17 @@ __global__ void jacobi_kernel(const long long* __restrict__ rp, const int* __res
 // cells are heavy together: where rays meet, a row holds thousands of entries), and
 // lane w keeps the sum of its w-th row, so that the FP64 division runs on full warps.
 // Triples of FP32 values carry the squares, two to an instruction, and rows whose sum
-// they cannot hold are summed again in FP64. Bound by the FP32 instructions. Eight
-// lanes join a row's sums in three steps for four rows at once; rows beyond NJ_FAR go
-// to the whole warp. 8 / 32 lanes, us: 262,144 rows of 40 entries 33 / 87 (47 a thread
-// per row in FP64), of 202 68 / 128 (214), 131,072 rows of 361 56 / 90 (213); means of
-// 3000 from 2 to 20,000 45 / 17. The cells of 2M rays on 100^3 (361M entries) 0.49 ms,
-// 0.58 with the range tested per entry and every load against the row's end.
+// they cannot hold are summed again in FP64. Bound by the FP32 instructions and, where
+// lengths differ, by the rows that take longest: groups of 8 and 16 join a row's sums in
+// few steps for four or two rows at once, and four times the blocks that fit even the
+// lengths out. 8 / 16 / 32 lanes, us: 262,144 rows of 40 entries 33 / 56 / 87 (47 a
+// thread per row in FP64), of 202 68 / 88 / 128 (214); the cells of rays, mean 211 on
+// 54^3 84 / 72 / 80, mean 361 on 100^3 482 / 465 / 511, with as many blocks as fit 108 /
+// 84 / 80 and 487 / 466 / 565; means of 3000 from 2 to 20,000 45 / - / 17.
 // Short rows (less than 24 entries on average) are staged through shared memory
 // instead, a thread per row: 2M rows of 7 entries 58 us (85 in FP64).
-constexpr int NJ_FAR = 1024;  // rows that groups of eight leave to the warp
+// Rows beyond this many entries go to the whole warp.
+__host__ __device__ constexpr int nj_far(int G) { return G == 8 ? 1024 : 4096; }
 
 // This lane's squares among p[0 .. n), G lanes over them; full triples go to far. Two
 // sums per instruction, joined at the end.
@@ -763,7 +765,7 @@ __global__ void __launch_bounds__(256, 4) normal_jacobi_kernel(const long long* 
         for (int w = 0; w < G && r0 - ahead + w * groups < rows; ++w) {
             const long long r = r0 + w * groups;
             const long long a = r < rows ? rp[r] : 0, b = r < rows ? rp[r + 1] : 0;
-            const bool rest = G < 32 && b - a > NJ_FAR;
+            const bool rest = G < 32 && b - a > nj_far(G);
             TripleSum s;
             double far = 0.0;
             add_squares<G>(val + a, rest ? 0 : b - a, lane, s, far);
@@ -1125,9 +1127,11 @@ int launch_jacobi(const DevCsr& A, float* dinv, cudaStream_t st) {
 }
 int launch_normal_jacobi(const DevCsr& AT, double lam, float* dinv, cudaStream_t st) {
     if (AT.nnz >= 480 * AT.rows)
-        normal_jacobi_kernel<32><<<cg_blocks(AT.rows * 32), 256, 0, st>>>(AT.row_ptr, AT.val, AT.rows, lam, dinv);
+        normal_jacobi_kernel<32><<<blocks_for(AT.rows * 32), 256, 0, st>>>(AT.row_ptr, AT.val, AT.rows, lam, dinv);
+    else if (AT.nnz >= 160 * AT.rows)
+        normal_jacobi_kernel<16><<<blocks_for(AT.rows * 16), 256, 0, st>>>(AT.row_ptr, AT.val, AT.rows, lam, dinv);
     else if (AT.nnz >= 24 * AT.rows)
-        normal_jacobi_kernel<8><<<cg_blocks(AT.rows * 8), 256, 0, st>>>(AT.row_ptr, AT.val, AT.rows, lam, dinv);
+        normal_jacobi_kernel<8><<<blocks_for(AT.rows * 8), 256, 0, st>>>(AT.row_ptr, AT.val, AT.rows, lam, dinv);
     else
         normal_jacobi_rows_kernel<<<blocks_for(AT.rows), NJ_ROWS, 0, st>>>(AT.row_ptr, AT.val, AT.rows, lam, dinv);
     count_launch();
