@@ -4,8 +4,9 @@
 // add_diagonal, Frobenius norm (:168-193), and the Krylov solvers of
 // SparseOps (sparse/sparse_ops.cpp:8-113) -- plain CG, Jacobi-PCG and the
 // damped normal-equation solve of the tomography system -- with FP32
-// vectors and matrix values, int32 column indices, int64 row pointers and
-// every inner product, residual norm and step scalar in FP64 on the device.
+// vectors and matrix values, int32 column indices, int64 row pointers, and
+// every inner product, residual norm and step scalar on the device in FP64 or,
+// with no fewer bits, in triples of FP32 values folded into FP64 (TripleSum).
 #include "st_sort.cuh"
 
 #include <algorithm>
@@ -316,7 +317,7 @@ __device__ __forceinline__ void copy16_async(void* dst, const void* src, int byt
 // more entries than fit in shared memory is summed a warp per row; matrices with much
 // of their entries in such tiles, or in tiles with a long row that one thread works
 // through, go to a group of lanes per row (lanes_of).
-// 7 entries per row on a 256^3 grid, 72 bytes per row: 199 us a product (a copy of
+// 7 entries per row on a 256^3 grid, 72 bytes per row: 192 us a product (a copy of
 // the bytes takes 178); products along the stream 244, four lanes per row 600. 40
 // CG iterations there with tiles of 256 / 128 / 64 rows 24.3 / 23.5 / 23.3 ms
 // (smaller tiles overflow more easily), a tile per warp 25.9 (spills), two tiles in

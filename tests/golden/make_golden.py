@@ -2,7 +2,7 @@
 own C++ (src/cpp of 13262233692/03-seismic-tomography-compute, compiled in
 place by oracle/build_ref.sh into oracle/_ref/libseismic_ref.so) on small
 seeded inputs. The reference sources exist only where this script is run;
-the fixtures it writes are what the tests (and the GPU machine) use.
+the fixtures it writes are what the tests use everywhere.
 
     SEISMIC_REFERENCE_DIR=<reference checkout> python tests/golden/make_golden.py
 
